@@ -14,7 +14,7 @@ enter.
 from __future__ import annotations
 
 import ctypes
-from typing import Optional, Tuple
+from typing import Optional, Sequence, Tuple
 
 import torch
 
@@ -1210,6 +1210,9 @@ _STATUS_ROLES = {
     22: "paged_attention_prefill (tcgen05 form): the MMA issuer",
     23: "paged_attention_prefill (tcgen05 form): a softmax warp",
     24: "paged_attention_prefill (tcgen05 form): shared memory not on a 1024-byte mark;",
+    31: "widened_attention: the copying warp", 32: "widened_attention: the MMA issuer",
+    33: "widened_attention: a softmax warp",
+    34: "widened_attention: shared memory not on a 1024-byte mark;",
 }
 
 
@@ -1617,6 +1620,148 @@ def latent_attention(q_lat: torch.Tensor, q_rot: torch.Tensor, cache: torch.Tens
         _ptr(step.positions), _ptr(out), ctypes.c_longlong(T * rank), ctypes.c_longlong(rank),
         _dtype_code(q_lat), T, H, rank, dr, page, window, ctypes.c_float(scale), _stream()),
         "latent_attention")
+    _count()
+    return out
+
+
+USE_WIDENED_LATENT = True
+
+
+def widened_latent_applies(dtype, dim: int, rot_dim: int, vdim: int, rank: int,
+                           offsets: Sequence[int] = ()) -> bool:
+    """Whether the widened form of latent attention takes these sizes: bf16, heads of the
+    kernel's widths, and records, products and column offsets in 16-byte chunks."""
+    return bool(USE_WIDENED_LATENT and dtype == torch.bfloat16 and rot_dim % 2 == 0
+                and rank % 8 == 0 and rot_dim % 8 == 0 and all(o % 8 == 0 for o in offsets)
+                and _lib().ix_widened_attention_applies(dim + rot_dim, vdim))
+
+
+# The widened rows of a step live in one buffer; beyond this the folded form runs.
+WIDENED_MAX_BYTES = 1 << 30
+# What either form takes, in microseconds, for the choice between them: operations a
+# microsecond of the folded kernel; microseconds that the folded form's two more products take
+# at least; microseconds a 64-key tile of the widened kernel's walk; operations a microsecond of
+# the widening product.  Fitted to whole mixers at a latent of 512 + 64 (folded / widened, us):
+# 16 heads, n new tokens behind b: (33, 0) 37 / 28, (33, 512) 50 / 42, (33, 2048) 63 / 77,
+# (64, 8192) 157 / 236, (128, 2048) 114 / 83, (128, 8192) 250 / 237, (3000, 0) 1064 / 200,
+# (3000, 8192) 5916 / 703; 32 heads: (33, 2048) 103 / 113, (64, 2048) 132 / 114, (3000, 0)
+# 2010 / 398; 8 heads, latent 256 + 32: (128, 512) 42 / 36, (256, 2048) 75 / 88, (700, 2048)
+# 154 / 100.
+WIDENED_RATES = (165e6, 12.0, 1.2, 800e6)
+
+
+def widened_latent_rows(q_lens: Sequence[int], max_kv_len: int, window: int, heads: int,
+                        rank: int, rot_dim: int, width: int, mixed: bool = False) -> int:
+    """Rows a sequence's collected records take when these portions (``q_lens`` new tokens
+    each, at most ``max_kv_len`` with what the cache holds) should attend over widened keys
+    and values, 0 when the folded form is the cheaper one.  Depends on the step's shape
+    only.  ``width``: key and value entries of a head together.  ``mixed``: ``max_kv_len``
+    covers other sequences too, so that half of it is taken for the portions' own."""
+    if not q_lens:
+        return 0
+    rows = int(max_kv_len)
+    if window > 0:
+        rows = min(rows, window + max(q_lens) + 63)
+    rows = -(-rows // 64) * 64
+    S, tokens = len(q_lens), sum(q_lens)
+    if S * rows * heads * width * 2 > WIDENED_MAX_BYTES:
+        return 0
+    folded_rate, products_us, walk_us, widen_rate = WIDENED_RATES
+    own = 0.5 * rows if mixed else float(rows)
+    pairs = tokens * max(own - 0.5 * tokens / S, 0.5 * own)
+    folded = products_us + pairs * heads * 2.0 * (2 * rank + rot_dim) / folded_rate
+    items = heads * sum(-(-n // 256) for n in q_lens)     # blocks of the walk, one an SM
+    walk = max(1.0, 0.75 * items / 148.0) * (own / 64.0) * walk_us
+    widen = S * rows * heads * width * 2.0 * (rank + rot_dim) / widen_rate
+    return rows if walk + widen < folded else 0
+
+
+def latent_front_inplace(q: Optional[torch.Tensor], q_ld: int, kv: Optional[torch.Tensor],
+                         kv_ld: int, positions: torch.Tensor, freq: torch.Tensor, mag: float,
+                         gain: Optional[torch.Tensor], eps: float, heads: int, dim: int,
+                         rot_dim: int, rot_dims: int, rank: int, cache: Optional[torch.Tensor],
+                         slots: Optional[torch.Tensor]):
+    """The rotated query parts of ``q`` (rows of pitch ``q_ld``, head by head ``dim`` plain
+    and ``rot_dim`` rotated entries) turned where they lie, and the records of the
+    down-projections ``kv`` (rows of pitch ``kv_ld``) into ``cache`` at ``slots`` (no cache:
+    none).  ``q`` and ``kv`` are one-dimensional views that start at the first entry."""
+    T = positions.numel()
+    for name, t, ld, width in (("q", q, q_ld, heads * (dim + rot_dim)),
+                               ("kv", kv, kv_ld, rank + rot_dim)):
+        _chk(name, t, torch.bfloat16, optional=True)
+        if t is not None and (t.dim() != 1 or ld < width or t.numel() < (T - 1) * ld + width):
+            raise KernelError(f"latent_front_inplace: {name} does not hold {T} rows")
+    _chk("positions", positions, torch.int32)
+    _chk("freq", freq, torch.float32)
+    _chk("gain", gain, torch.float32, optional=True)
+    _chk("cache", cache, torch.bfloat16, optional=True)
+    _chk("slots", slots, torch.int32, optional=True)
+    if freq.numel() * 2 != rot_dims:
+        raise KernelError("latent_front_inplace: one frequency per rotated pair")
+    if cache is not None and (cache.shape[1] != 1 or cache.shape[3] != rank + rot_dim
+                              or gain is None or gain.numel() != rank or kv is None
+                              or slots is None or slots.numel() != T):
+        raise KernelError("latent_front_inplace: cache records must be [1, page, rank + "
+                          "rot_dim], with one gain per latent entry and one slot per row")
+    _check(_lib().ix_latent_front_inplace(
+        _ptr(q), ctypes.c_longlong(q_ld), _ptr(kv), ctypes.c_longlong(kv_ld), _ptr(positions),
+        _ptr(freq), ctypes.c_float(mag), _ptr(gain), ctypes.c_float(eps), _ptr(slots),
+        _ptr(cache), T, heads, dim, rot_dim, rot_dims, rank, _stream()), "latent_front_inplace")
+    _count()
+
+
+def latent_collect(cache: torch.Tensor, block_table: torch.Tensor, q_pos0: torch.Tensor,
+                   kv_len: torch.Tensor, rows: int, window: int):
+    """The records that a step's queries can see, [S * rows, rank + rot_dim]: row r of
+    sequence s is the record of position base(s) + r, where base is 0, or with a window the
+    first visible position rounded down to 64; zeros where there is none."""
+    _chk("cache", cache)
+    for name, t in (("block_table", block_table), ("q_pos0", q_pos0), ("kv_len", kv_len)):
+        _chk(name, t, torch.int32)
+    S, width = block_table.shape[0], cache.shape[3]
+    if q_pos0.numel() != S or kv_len.numel() != S or cache.shape[1] != 1:
+        raise KernelError("latent_collect: one position and one length per sequence")
+    out = torch.empty((S * rows, width), dtype=cache.dtype, device=cache.device)
+    _check(_lib().ix_latent_collect(
+        _ptr(cache), _ptr(block_table), block_table.shape[1], _ptr(q_pos0), _ptr(kv_len),
+        _ptr(out), S, rows, cache.shape[2], window, width * cache.element_size(), _stream()),
+        "latent_collect")
+    _count()
+    return out
+
+
+def widened_attention(q: torch.Tensor, q_ld: int, kv: torch.Tensor, cu_q: torch.Tensor,
+                      q_pos0: torch.Tensor, tokens: int, heads: int, dk: int, dv: int, rows: int,
+                      window: int, scale: float, gate: Optional[torch.Tensor] = None, gate_ld: int = 0,
+                      out: Optional[torch.Tensor] = None):
+    """Causal attention of prompt portions over the step's own widened keys and values.
+
+    ``q``: a one-dimensional view that starts at the first row's first query, rows of pitch
+    ``q_ld``, heads of ``dk`` beside each other; softmax weights keep 16 bits in their product
+    with the values; ``kv`` [S * rows, heads * (dk + dv)], the keys
+    of every head then the values, rows as ``latent_collect`` lays them out.  ``gate``: a
+    one-dimensional view likewise, whose sigmoid multiplies the result entry by entry.
+    Returns [tokens, heads * dv]."""
+    _chk("q", q, torch.bfloat16)
+    _chk("kv", kv, torch.bfloat16)
+    _chk("cu_q", cu_q, torch.int32)
+    _chk("q_pos0", q_pos0, torch.int32)
+    _chk("gate", gate, torch.bfloat16, optional=True)
+    _chk("out", out, torch.bfloat16, optional=True)
+    S = q_pos0.numel()
+    if cu_q.numel() != S + 1 or tuple(kv.shape) != (S * rows, heads * (dk + dv)):
+        raise KernelError("widened_attention: keys and values do not fit the sequences")
+    for name, t, ld, width in (("q", q, q_ld, heads * dk), ("gate", gate, gate_ld, heads * dv)):
+        if t is not None and (t.dim() != 1 or t.numel() < (tokens - 1) * ld + width):
+            raise KernelError(f"widened_attention: {name} does not hold {tokens} rows")
+    if out is None:
+        out = torch.empty((tokens, heads * dv), dtype=q.dtype, device=q.device)
+    elif tuple(out.shape) != (tokens, heads * dv):
+        raise KernelError("widened_attention: out must be [tokens, heads * dv]")
+    _check(_lib().ix_widened_attention(
+        _ptr(q), ctypes.c_longlong(q_ld), _ptr(kv), _ptr(cu_q), _ptr(q_pos0), _ptr(out), tokens,
+        S, heads, dk, dv, rows, window, ctypes.c_float(scale), _ptr(gate), ctypes.c_longlong(gate_ld), _ptr(_tc_status(q.device)), _stream()),
+        "widened_attention")
     _count()
     return out
 

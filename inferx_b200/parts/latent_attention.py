@@ -11,9 +11,10 @@ the query instead of widening cached latents:
 
 so attention runs with one shared key head of ``kv_rank + rot_dim`` entries whose values
 are the latents themselves, and the head's output ``sum_j p_j c_j`` is widened by
-``W_uv[h]`` afterwards.  Every step - a whole prompt, a portion, a decoded token - takes
-this one path through the cache, so a position's result does not depend on how its
-sequence was cut.  Queries carry ``dim`` plain and ``rot_dim`` rotated entries per head;
+``W_uv[h]`` afterwards.  That is the form for a few queries per sequence: a pair costs the
+latent's size instead of a head's.  Prompt portions of enough tokens (decided by the shape
+of the step) widen the records they can see once, with one product, and attend over keys
+and values of the head's own size.  Queries carry ``dim`` plain and ``rot_dim`` rotated entries per head;
 an optional sigmoid gate computed from the mixer's input multiplies the heads' outputs
 before the output projection.
 
@@ -27,6 +28,8 @@ and a second product widens c_q to the queries.  A layer without records of its 
 cache, which holds that layer's records of this step too by the time it runs.
 """
 from __future__ import annotations
+
+from types import SimpleNamespace
 
 import torch
 
@@ -105,6 +108,20 @@ class LatentAttentionMixer:
         self.uk_t = w[self._n("uk")].view(s.heads, s.dim, s.kv_rank).transpose(1, 2).contiguous()
         self.uv = w[self._n("uv")].view(s.heads, s.vdim, s.kv_rank).contiguous()
         self.o_w = w[self._n("o")]
+        applies = getattr(self.ctx.ops, "widened_latent_applies", None)
+        self.kv_w = None
+        if applies is not None and self.in_w.is_cuda and applies(
+                self.in_w.dtype, s.dim, s.rot_dim, s.vdim, s.kv_rank,
+                (self.kv_off, self.gate_off, self.in_w.shape[0])):
+            # one matrix from records to the keys of every head, then the values: the record's
+            # rotated part passes through identity columns
+            kv = torch.zeros((s.heads * (s.dim + s.rot_dim + s.vdim), s.kv_rank + s.rot_dim),
+                             dtype=self.in_w.dtype, device=self.in_w.device)
+            keys = kv[:s.heads * (s.dim + s.rot_dim)].view(s.heads, s.dim + s.rot_dim, -1)
+            keys[:, :s.dim, :s.kv_rank] = w[self._n("uk")].view(s.heads, s.dim, s.kv_rank)
+            keys[:, s.dim:, s.kv_rank:] = torch.eye(s.rot_dim, dtype=kv.dtype, device=kv.device)
+            kv[s.heads * (s.dim + s.rot_dim):, :s.kv_rank] = w[self._n("uv")]
+            self.kv_w = kv
 
     def cache_needs(self):
         s = self.spec
@@ -112,14 +129,16 @@ class LatentAttentionMixer:
             return []
         return [PagedKvNeed(1, s.kv_rank + s.rot_dim, s.window, entries=(ENTRY,))]
 
+    def _pair_table(self, x):
+        if self.position is not None:
+            return self.position.pair_table()
+        return torch.empty(0, dtype=torch.float32, device=x.device), 1.0, 0
+
     def _queries(self, x, proj, step, cache, group, records):
         """(rotated query parts, plain ones heads outermost); the step's records are in the
         cache when this returns."""
         s, ops = self.spec, self.ctx.ops
-        if self.position is not None:
-            freq, mag, rot_dims = self.position.pair_table()
-        else:
-            freq, mag, rot_dims = torch.empty(0, dtype=torch.float32, device=x.device), 1.0, 0
+        freq, mag, rot_dims = self._pair_table(x)
         writes = s.own_records and cache.writes
         if not s.q_rank and s.own_records:
             return ops.latent_prepare(
@@ -140,8 +159,36 @@ class LatentAttentionMixer:
         s, ops = self.spec, self.ctx.ops
         T = x.shape[0]
         group = step.groups[cache.group]
-        records = cache.pages[ENTRY]
         proj = ops.linear(x, self.in_w)
+        # single tokens come first in a batch; what follows them may attend over widened keys
+        alone, rows = T, 0
+        if self.kv_w is not None and not step.all_decode:
+            nd = step.num_decode_seqs
+            rows = ops.widened_latent_rows(step.q_lens[nd:], step.max_kv_len, s.window, s.heads,
+                                           s.kv_rank, s.rot_dim, s.dim + s.rot_dim + s.vdim,
+                                           mixed=nd > 0)
+            if rows:
+                alone = nd
+        if alone == T:
+            o = self._folded(x, proj, step, cache, group)
+        else:
+            o = torch.empty((T, s.heads * s.vdim), dtype=x.dtype, device=x.device)
+            if alone:
+                group_alone = SimpleNamespace(block_table=group.block_table[:alone],
+                                              slots=group.slots[:alone])
+                first = SimpleNamespace(
+                    positions=step.positions[:alone], seq_of_token=step.seq_of_token[:alone],
+                    cu_q=step.cu_q[:alone + 1], q_pos0=step.q_pos0[:alone],
+                    q_lens=step.q_lens[:alone], max_kv_len=step.max_kv_len)
+                self._folded(x[:alone], proj[:alone], first, cache, group_alone, o[:alone])
+            self._widened(x, proj, step, cache, group, alone, rows, o[alone:])
+        return ops.linear(o, self.o_w, out_dtype=torch.float32 if s.out_float32 else None)
+
+    def _folded(self, x, proj, step, cache, group, out=None):
+        """The heads' gated outputs [T, heads * vdim], keys folded into the queries."""
+        s, ops = self.spec, self.ctx.ops
+        T = x.shape[0]
+        records = cache.pages[ENTRY]
         q_rot, q_plain = self._queries(x, proj, step, cache, group, records)
         q_lat = ops.batched_linear(q_plain, self.uk_t)                       # [heads, T, rank]
         mixed = ops.latent_attention(q_lat, q_rot, records, group.block_table, step, s.window,
@@ -149,12 +196,42 @@ class LatentAttentionMixer:
                                                  else {}))                   # [heads, T, rank]
         if s.output_gate:
             o = ops.gate_heads(ops.batched_linear(mixed, self.uv), proj, self.gate_off)
-        else:
-            # the heads' values land beside each other, ready for the output projection
-            o = torch.empty((T, s.heads, s.vdim), dtype=x.dtype, device=x.device)
-            ops.batched_linear(mixed, self.uv, out=o.transpose(0, 1))        # [heads, T, vdim]
-            o = o.view(T, s.heads * s.vdim)
-        return ops.linear(o, self.o_w, out_dtype=torch.float32 if s.out_float32 else None)
+            return o if out is None else out.copy_(o)
+        # the heads' values land beside each other, ready for the output projection
+        o = out if out is not None else torch.empty((T, s.heads * s.vdim), dtype=x.dtype,
+                                                    device=x.device)
+        ops.batched_linear(mixed, self.uv, out=o.view(T, s.heads, s.vdim).transpose(0, 1))
+        return o
+
+    def _widened(self, x, proj, step, cache, group, first, rows, out):
+        """The same for the tokens from ``first`` on (the first ``first`` sequences bring one
+        token each), over widened keys and values, into ``out``."""
+        s, ops = self.spec, self.ctx.ops
+        records = cache.pages[ENTRY]
+        ld = proj.shape[1]
+        flat = proj[first:].view(-1)
+        positions = step.positions[first:]
+        freq, mag, rot_dims = self._pair_table(x)
+        writes = s.own_records and cache.writes
+        kept = records if writes else None
+        slots = group.slots[first:] if writes else None
+        q, q_ld = flat, ld
+        if s.q_rank:
+            c_q = ops.latent_front(
+                proj[first:], self.q_rank, self.q_gain, s.latent_eps, self.kv_off, positions,
+                freq, mag, self.latent_gain, s.kv_rank, s.rot_dim, rot_dims, kept, slots)
+            q, q_ld = ops.linear(c_q, self.uq_w).view(-1), self.q_width
+            kept = slots = None
+        ops.latent_front_inplace(q, q_ld, flat[self.kv_off:] if kept is not None else None, ld,
+                                 positions, freq, mag, self.latent_gain, s.latent_eps, s.heads,
+                                 s.dim, s.rot_dim, rot_dims, s.kv_rank, kept, slots)
+        rec = ops.latent_collect(records, group.block_table[first:], step.q_pos0[first:],
+                                 step.kv_len[first:], rows, s.window)
+        kv = ops.linear(rec, self.kv_w)
+        ops.widened_attention(
+            q, q_ld, kv, step.cu_q_prompt if first else step.cu_q, step.q_pos0[first:],
+            x.shape[0] - first, s.heads, s.dim + s.rot_dim, s.vdim, rows, s.window, s.scale,
+            gate=flat[self.gate_off:] if s.output_gate else None, gate_ld=ld, out=out)
 
 
 register_part("mixer", "latent_attention", LatentAttentionMixer)

@@ -1,0 +1,186 @@
+"""Latent attention over widened keys and values: the kernels alone against plain statements,
+and the mixer's widened form against its folded one and against 32-bit arithmetic."""
+import math
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+import host_ops
+from test_gpu_dominex import _cuda, _step
+
+pytestmark = pytest.mark.gpu
+BF = torch.bfloat16
+
+
+def _ops():
+    from inferx_b200.kernels import ops
+    return ops
+
+
+def _pages(lens, page, g):
+    maxb = max(-(-n // page) for n in lens)
+    bt = torch.full((len(lens), maxb), -1, dtype=torch.int32)
+    perm, k = torch.randperm(sum(-(-n // page) for n in lens) + 2, generator=g), 0
+    for s, n in enumerate(lens):
+        for b in range(-(-n // page)):
+            bt[s, b] = perm[k]
+            k += 1
+    return bt, perm.numel()
+
+
+@pytest.mark.parametrize("page,window,width", [(4, 0, 72), (16, 100, 576), (8, 64, 40)])
+def test_collect(page, window, width):
+    g = torch.Generator().manual_seed(width)
+    q_lens, starts = [3, 70, 200], [0, 130, 5]
+    st = _step(q_lens, starts)
+    bt, P = _pages([a + n for a, n in zip(starts, q_lens)], page, g)
+    cache = torch.randn(P, 1, page, width, generator=g).to(BF)
+    rows = 320
+    base = [max(0, a - window + 1) // 64 * 64 if window else 0 for a in starts]
+    for s, b in enumerate(base):               # pages the window has passed may be gone
+        bt[s, :b // page] = -1
+    got = _ops().latent_collect(cache.cuda(), bt.cuda(), st.q_pos0.cuda(), st.kv_len.cuda(), rows,
+                                window).cpu().view(len(q_lens), rows, width)
+    want = torch.zeros_like(got)
+    for s in range(len(q_lens)):
+        for r in range(rows):
+            p = base[s] + r
+            if p < int(st.kv_len[s]):
+                want[s, r] = cache[bt[s, p // page], 0, p % page]
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("H,dn,dr,rot_dims,rank", [(3, 24, 16, 16, 40), (16, 128, 64, 64, 512),
+                                                  (2, 64, 0, 0, 24), (5, 8, 24, 8, 64)])
+def test_front_in_place(H, dn, dr, rot_dims, rank):
+    g = torch.Generator().manual_seed(rank)
+    T, page, P = 9, 4, 30
+    pos = torch.tensor([0, 1, 2, 3, 900, 61, 62, 63, 7], dtype=torch.int32)
+    kv_off = H * (dn + dr)
+    proj = torch.randn(T, kv_off + rank + dr + 8, generator=g).to(BF)
+    freq, gain = torch.rand(rot_dims // 2, generator=g), 1.0 + 0.2 * torch.randn(rank, generator=g)
+    slots = torch.randperm(P * page, generator=g)[:T].to(torch.int32)
+    cache = torch.zeros(P, 1, page, rank + dr, dtype=BF)
+    want = cache.clone()
+    rot, plain = host_ops.latent_prepare(proj, 0, kv_off, pos, freq, 1.3, gain, 1e-5, H, dn, dr,
+                                         rot_dims, rank, want, slots)
+    p, c = proj.cuda(), cache.cuda()
+    _ops().latent_front_inplace(p.view(-1), p.shape[1], p.view(-1)[kv_off:], p.shape[1], pos.cuda(),
+                                freq.cuda(), 1.3, gain.cuda(), 1e-5, H, dn, dr, rot_dims, rank, c,
+                                slots.cuda())
+    q = p.cpu()[:, :kv_off].view(T, H, dn + dr)
+    tol = dict(rtol=1.6e-2, atol=1.6e-2)
+    assert torch.equal(q[..., :dn].transpose(0, 1), plain)
+    torch.testing.assert_close(q[..., dn:].float(), rot.float(), **tol)
+    assert torch.equal(p.cpu()[:, kv_off:], proj[:, kv_off:])
+    torch.testing.assert_close(c.cpu().float(), want.float(), **tol)
+
+
+# edges: of the 64-key tile, of the 128-query tile, of the 256 queries a block owns; windows
+# that cut a tile; several sequences behind contexts; more key tiles than ring stages
+@pytest.mark.parametrize("dk,dv", [(64, 64), (64, 128), (128, 64), (128, 128), (192, 64),
+                                   (192, 128)])
+@pytest.mark.parametrize("q_lens,starts,window", [
+    ([2], [0], 0), ([64], [0], 0), ([65, 127], [63, 0], 0), ([128, 129], [0, 200], 0),
+    ([256, 257], [1, 511], 0), ([300, 33], [100, 700], 90), ([513], [0], 64), ([70], [640], 1)])
+def test_attention(dk, dv, q_lens, starts, window):
+    g = torch.Generator().manual_seed(dk + dv + sum(q_lens))
+    H, T, S = 3, sum(q_lens), len(q_lens)
+    st = _step(q_lens, starts)
+    need = max(a + n for a, n in zip(starts, q_lens))
+    if window:
+        need = min(need, window + max(q_lens) + 63)
+    rows = -(-need // 64) * 64
+    q = torch.randn(T, H * dk + 8, generator=g).to(BF)
+    kv = torch.randn(S * rows, H * (dk + dv), generator=g).to(BF)
+    gate = torch.randn(T, H * dv, generator=g).to(BF)
+    scale = 2.0 / math.sqrt(dk)
+    want = torch.zeros(T, H, dv)
+    t0 = 0
+    for s, (n, a) in enumerate(zip(q_lens, starts)):
+        base = max(0, a - window + 1) // 64 * 64 if window else 0
+        m = a + n - base
+        k = kv[s * rows:s * rows + m, :H * dk].float().view(m, H, dk)
+        v = kv[s * rows:s * rows + m, H * dk:].float().view(m, H, dv)
+        sc = torch.einsum("thd,mhd->htm", q[t0:t0 + n, :H * dk].float().view(n, H, dk), k) * scale
+        i, j = torch.arange(a, a + n)[:, None], torch.arange(base, a + n)[None]
+        seen = (j <= i) & ((i - j < window) if window else torch.ones_like(j <= i))
+        want[t0:t0 + n] = torch.einsum("htm,mhd->thd", sc.masked_fill(~seen, -math.inf).softmax(-1),
+                                       v)
+        t0 += n
+    most = float(kv.float().abs().max())
+    for gt in (None, gate):
+        out = _ops().widened_attention(
+            q.cuda().view(-1), q.shape[1], kv.cuda(), st.cu_q.cuda(), st.q_pos0.cuda(), T, H, dk, dv,
+            rows, window, scale, None if gt is None else gt.cuda().view(-1), H * dv)
+        _ops().check_async_errors()
+        ref = want if gt is None else want * torch.sigmoid(gt.float().view(T, H, dv))
+        # weights of 16 bits move a mean of values by at most 2^-17 of the largest one, the
+        # result's own rounding by 2^-9; scores of some tens of units are fp32 sums, exp2 is
+        # good to 2^-22 of them
+        bound = most * (2.0 ** -9 + 2.0 ** -17 + 2.0 ** -15)
+        assert float((out.cpu().float().view(T, H, dv) - ref).abs().max()) <= bound
+
+
+@pytest.mark.parametrize("dim,rot,vdim,rank,heads", [(96, 32, 128, 64, 4), (128, 64, 128, 128, 3)])
+@pytest.mark.parametrize("q_rank,own,gated,exact", [(0, True, True, False), (40, True, False, True),
+                                                    (48, False, False, False)])
+@pytest.mark.parametrize("window", [0, 150])
+def test_mixer_forms_agree(dim, rot, vdim, rank, heads, q_rank, own, gated, exact, window):
+    """The same mixed batch (single tokens far into their sequences, portions behind contexts)
+    through the folded and the widened form, both against 32-bit arithmetic."""
+    from inferx_b200.parts.latent_attention import LatentAttentionMixer
+    from inferx_b200.parts.specs import LatentAttentionSpec
+    ops = _ops()
+    g = torch.Generator().manual_seed(rank + window + q_rank)
+    hidden, page = 64, 16
+    spec = LatentAttentionSpec(hidden=hidden, heads=heads, dim=dim, rot_dim=rot, vdim=vdim,
+                               kv_rank=rank, scale=1.0 / math.sqrt(dim + rot), window=window,
+                               position=None, latent_eps=1e-6, output_gate=gated, q_rank=q_rank,
+                               own_records=own, fp32_weights=exact)
+    q_lens, starts = [1, 1, 90, 300], [500, 3, 250, 0]
+    st = _step(q_lens, starts)
+    lens = [a + n for a, n in zip(starts, q_lens)]
+    bt, P = _pages(lens, page, g)
+    slots = torch.tensor([int(bt[s, p // page]) * page + p % page
+                          for s, (n, a) in enumerate(zip(q_lens, starts)) for p in range(a, a + n)],
+                         dtype=torch.int32)
+    x = torch.randn(st.num_tokens, hidden, generator=g)
+    cache = torch.randn(P, 1, page, rank + rot, generator=g)
+
+    def run(dtype, widened):
+        mixer = LatentAttentionMixer(spec, SimpleNamespace(ops=ops, dtype=dtype), "m")
+        gw = torch.Generator().manual_seed(5)
+        w = {d.name: (torch.randn(d.shape, generator=gw) * d.shape[-1] ** -0.5 if len(d.shape) == 2
+                      else 1 + 0.1 * torch.randn(d.shape, generator=gw)) for d in mixer.tensors()}
+        w = {k: (v.to(BF).to(dtype) if v.dim() == 2 else v).cuda() for k, v in w.items()}
+        mixer.bind(w)
+        if not widened:
+            mixer.kv_w = None
+        elif mixer.kv_w is None:
+            pytest.fail("the widened form does not take these sizes")
+        records = cache.to(BF).to(dtype).cuda()
+        step = _cuda(st)
+        step.groups = [SimpleNamespace(block_table=bt.cuda(), slots=slots.cuda())]
+        before = ops.widened_latent_rows
+        if widened:
+            need = max(lens) if not window else min(max(lens), window + max(q_lens) + 63)
+            ops.widened_latent_rows = lambda *a, **k: -(-need // 64) * 64
+        try:
+            out = mixer.forward(x.to(BF).to(dtype).cuda(), step,
+                                SimpleNamespace(group=0, pages={"latent": records}, writes=True))
+        finally:
+            ops.widened_latent_rows = before
+        ops.check_async_errors()
+        return out.float().cpu(), records.float().cpu()
+
+    exact32, rec32 = run(torch.float32, False)
+    folded, rec_f = run(BF, False)
+    widened, rec_w = run(BF, True)
+    scale = float(exact32.norm())
+    off_f, off_w = float((folded - exact32).norm()) / scale, float((widened - exact32).norm()) / scale
+    # either form rounds every stored value once to 8 bits; the widened one is held to what
+    # the folded one shows here (two roundings of a quarter more each would still pass)
+    assert off_w <= 1.25 * off_f and off_f < 0.02, (off_f, off_w)
+    assert torch.equal(rec_f, rec_w)
