@@ -8,8 +8,7 @@ falls back to a library implementation.
 Matrix products without a fused epilogue go to cuBLAS through ``torch`` in the
 bfloat16 mode, where the reference engine also calls a library
 (src/backends/cuda/ops/gemm_cublaslt.cc:391-396); the 32-bit mode runs the
-library's own fp32 FFMA kernel so that no reduced-precision matrix mode can
-enter.
+library's own fp32 kernels so that no reduced-precision matrix mode can enter.
 """
 from __future__ import annotations
 
@@ -279,13 +278,15 @@ def linear_act(x: torch.Tensor, w: torch.Tensor, activation: str):
         return gemm_small_m(x, w.unsqueeze(0), None, None, False, M, rows_per_pass=M,
                             activation=activation)
     if x.dtype == torch.float32:
+        if _splits_fp32(x, w):
+            return gemm_fp32_tc(x, w, activation)
         return gemm_generic(x, w.unsqueeze(0), None, None, dual=False, activation=activation)
     y = linear(x, w)
     return activate(y, activation, out=y)
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None):
-    """x[M,K] . w[N,K]^T.  bfloat16: cuBLAS, fp32 accumulation.  float32: own FFMA kernel."""
+    """x[M,K] . w[N,K]^T.  bfloat16: cuBLAS, fp32 accumulation.  float32: own kernels."""
     _chk("x", x)
     _chk("w", w)
     if x.dtype != w.dtype:
@@ -303,7 +304,46 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = 
         if out_dtype == torch.bfloat16:
             return torch.mm(x, w.t())
         return torch.mm(x, w.t(), out_dtype=out_dtype)
+    if out_dtype == torch.float32 and _splits_fp32(x, w):
+        return gemm_fp32_tc(x, w)
     return gemm_generic(x, w.unsqueeze(0), None, None, dual=False, out_dtype=out_dtype)
+
+
+USE_FP32_TC = True
+# Fewer rows stream the weights past the CUDA cores (gemm_generic's rows kernel, bound by
+# reading them).  Above, that kernel's tiles are bound by the FFMA rate (us, tiles / this form):
+# 17 rows of 2048 x 2048 161 / 28, 600 rows of 11264 x 2048 794 / 175, 17 rows of 5632 x 1024
+# 85 / 29, 64 x 64 x 64 13 / 16.5.
+FP32_TC_MIN_ROWS = 17
+
+
+def _splits_fp32(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether an fp32 product goes to the tensor cores in three bfloat16 terms a number:
+    enough rows, K in 32-byte chunks."""
+    return bool(USE_FP32_TC and x.dtype == torch.float32 and w.dtype == torch.float32
+                and x.shape[0] >= FP32_TC_MIN_ROWS and x.shape[1] % 8 == 0
+                and (x.data_ptr() | w.data_ptr()) % 32 == 0)
+
+
+def gemm_fp32_tc(x: torch.Tensor, w: torch.Tensor, activation: Optional[str] = None,
+                 splits: Optional[int] = None):
+    """x[M,K] . w[N,K]^T in fp32 by six bfloat16 products of three terms a number; closer to
+    64 bits than a chain of fp32 multiply-adds.  ``splits``: runs that k is cut into."""
+    _chk("x", x, torch.float32)
+    _chk("w", w, torch.float32)
+    M, K = x.shape
+    N = w.shape[0]
+    if w.shape[1] != K:
+        raise KernelError(f"gemm_fp32_tc: inner sizes differ ({K} vs {w.shape[1]})")
+    if splits is None:
+        splits = _lib().ix_gemm_fp32_tc_splits(M, N, K)
+    out = torch.empty((M, N), dtype=torch.float32, device=x.device)
+    part = torch.empty((splits, M, N), dtype=torch.float32, device=x.device) if splits > 1 else None
+    _check(_lib().ix_gemm_fp32_tc(_ptr(x), _ptr(w), _ptr(out), _ptr(part), M, N, K, splits,
+                                  _ACTIVATIONS[activation], _ptr(_tc_status(x.device)),
+                                  _stream()), "gemm_fp32_tc")
+    _count(2 if splits > 1 else 1)
+    return out
 
 
 def gemm_generic(x: torch.Tensor, w: torch.Tensor, rows: Optional[torch.Tensor],
@@ -1213,6 +1253,7 @@ _STATUS_ROLES = {
     31: "widened_attention: the copying warp", 32: "widened_attention: the MMA issuer",
     33: "widened_attention: a softmax warp",
     34: "widened_attention: shared memory not on a 1024-byte mark;",
+    41: "gemm_fp32_tc: a splitting warp", 42: "gemm_fp32_tc: the MMA issuer",
 }
 
 
