@@ -2209,8 +2209,25 @@ def ssd_recurrence(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tenso
             not (dt_bias.numel() == a_log.numel() == d_skip.numel() == heads):
         raise KernelError("ssd_recurrence: inputs and state do not fit together")
     out = torch.empty((T, heads * vdim), dtype=torch.float32, device=xbc.device)
-    seg_len, nseg = recurrence_segments(int(getattr(step, "max_q_len", 0) or T), step.num_seqs,
-                                        heads, vdim)
+    walked, longest = step.num_seqs, int(getattr(step, "max_q_len", 0) or T)
+    if _ssd_in_chunks(xbc, ld, state, longest, nstate, vdim):
+        # single tokens come first in a batch: they are walked, the sequences after them chunked
+        walked = int(getattr(step, "num_decode_seqs", 0) or 0)
+        tokens, S = T - walked, step.num_seqs
+        size = _lib().ix_ssd_chunks_scratch_floats
+        size.restype = ctypes.c_longlong
+        scratch = torch.empty((size(tokens, S - walked, heads, nstate, vdim),),
+                              dtype=torch.float32, device=xbc.device)
+        _check(_lib().ix_ssd_chunks(
+            _ptr(xbc), ctypes.c_longlong(ld), _ptr(dt_raw), ctypes.c_longlong(ld_dt),
+            _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), _ptr(step.cu_q),
+            _ptr(step.state_slot), _ptr(out), tokens, S, walked, longest, heads, vdim, nstate,
+            groups, _ptr(scratch), _stream()), "ssd_chunks")
+        _count(3)
+        if not walked:
+            return out
+        longest = 1
+    seg_len, nseg = recurrence_segments(longest, walked, heads, vdim)
     scratch = None
     if nseg > 1:
         scratch = torch.empty((_lib().ix_ssd_recurrence_scratch_floats(
@@ -2218,10 +2235,23 @@ def ssd_recurrence(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tenso
     _check(_lib().ix_ssd_recurrence(
         _ptr(xbc), ctypes.c_longlong(ld), _ptr(dt_raw), ctypes.c_longlong(ld_dt),
         _dtype_code(xbc), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), _ptr(step.cu_q),
-        _ptr(step.state_slot), _ptr(out), step.num_seqs, heads, vdim, nstate, groups, seg_len,
+        _ptr(step.state_slot), _ptr(out), walked, heads, vdim, nstate, groups, seg_len,
         nseg, _ptr(scratch), _stream()), "ssd_recurrence")
     _count(2 if nseg > 1 else 1)
     return out
+
+
+USE_SSD_CHUNKS = True
+# bfloat16 portions from this many tokens on run in chunks on the tensor cores (walk / chunks at
+# 32 heads of 128 x 64, us: 33 tokens 19 / 23, 64 31 / 25, 256 67 / 27, 2,048 441 / 92).
+SSD_CHUNK_MIN_TOKENS = 64
+
+
+def _ssd_in_chunks(xbc, ld: int, state, longest: int, nstate: int, vdim: int) -> bool:
+    return bool(USE_SSD_CHUNKS and longest >= SSD_CHUNK_MIN_TOKENS
+                and xbc.dtype == torch.bfloat16 and ld % 8 == 0
+                and (xbc.data_ptr() | state.data_ptr()) % 16 == 0
+                and _lib().ix_ssd_chunks_applies(nstate, vdim))
 
 
 def delta_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta_raw: torch.Tensor,

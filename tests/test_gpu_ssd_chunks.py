@@ -1,0 +1,89 @@
+"""The state-space recurrence in chunks: against 64 bits beside the walk, at the edges of a
+chunk, of the padding and of the batch."""
+import pytest
+import torch
+
+from test_gpu_dominex import _cuda, _step
+
+pytestmark = pytest.mark.gpu
+
+
+def _ops():
+    from inferx_b200.kernels import ops
+    return ops
+
+
+def _plain64(xbc, dt_raw, dt_bias, a_log, d_skip, state, q_lens, slots, H, V, N, G):
+    x, dt_raw, st = xbc.double(), dt_raw.double(), state.double().clone()
+    dt = torch.nn.functional.softplus(dt_raw + dt_bias.double(), threshold=1000.0)
+    a = torch.exp(-torch.exp(a_log.double()) * dt)
+    out, t = torch.zeros(x.shape[0], H, V, dtype=torch.float64, device=x.device), 0
+    for n, slot in zip(q_lens, slots):
+        S = st[slot]
+        for _ in range(n):
+            xv = x[t, :H * V].view(H, V)
+            B = x[t, H * V:H * V + G * N].view(G, N).repeat_interleave(H // G, 0)
+            C = x[t, H * V + G * N:].view(G, N).repeat_interleave(H // G, 0)
+            S = a[t][:, None, None] * S + (dt[t][:, None] * B)[:, :, None] * xv[:, None]
+            out[t] = torch.einsum("hnv,hn->hv", S, C) + d_skip.double()[:, None] * xv
+            t += 1
+        st[slot] = S
+    return out.view(x.shape[0], H * V), st
+
+
+def _off(a, ref):
+    return float((a.double() - ref).norm() / ref.norm())
+
+
+@pytest.mark.parametrize("H,V,N,G", [(4, 64, 128, 2), (2, 40, 24, 1), (6, 8, 8, 3), (1, 136, 256, 1)])
+@pytest.mark.parametrize("q_lens", [[64], [65, 128], [1, 1, 63, 200], [129, 2, 15]])
+@pytest.mark.parametrize("spread", [0.5, 3.0])     # of the decays' exponents: near 1, and some at 0
+def test_against_64_bits(H, V, N, G, q_lens, spread):
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(H + V + sum(q_lens))
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    q_lens = sorted(q_lens, key=lambda n: n != 1)
+    S, T = len(q_lens), sum(q_lens)
+    step = _cuda(_step(q_lens, [5] * S, slots=list(range(S))[::-1]))
+    slots = step.state_slot.tolist()
+    xbc, dt = rnd(T, H * V + 2 * G * N).bfloat16(), rnd(T, H).bfloat16()
+    bias, a_log, d = rnd(H) - 2.0, spread * rnd(H), rnd(H)
+    state = rnd(S + 1, H, N, V)
+    ref, st_ref = _plain64(xbc, dt, bias, a_log, d, state, q_lens, slots, H, V, N, G)
+    res = {}
+    for form in ("chunks", "walk"):
+        ops.USE_SSD_CHUNKS = form == "chunks"
+        try:
+            st = state.clone()
+            assert ops._ssd_in_chunks(xbc, xbc.shape[1], st, max(q_lens), N, V) == (
+                form == "chunks" and max(q_lens) >= ops.SSD_CHUNK_MIN_TOKENS)
+            out = ops.ssd_recurrence(xbc, dt, bias, a_log, d, st, step, H, V, N, G)
+        finally:
+            ops.USE_SSD_CHUNKS = True
+        res[form] = _off(out, ref), _off(st, st_ref)
+        assert torch.equal(st[S], state[S])          # a slot of no sequence is untouched
+    # 24-bit terms into fp32 sums: no further off than 32-bit arithmetic token by token, or a
+    # few units in the last place of a sum of a hundred products
+    for c, w in zip(res["chunks"], res["walk"]):
+        assert c <= max(w, 4e-7), res
+
+
+def test_decays_of_zero_and_infinite_rates():
+    ops = _ops()
+    H, V, N, T = 2, 16, 16, 100
+    g = torch.Generator(device="cuda").manual_seed(3)
+    xbc = torch.randn(T, H * V + 2 * N, generator=g, device="cuda").bfloat16()
+    dt = torch.randn(T, H, generator=g, device="cuda").bfloat16()
+    step = _cuda(_step([T], [0]))
+    par = (torch.zeros(H, device="cuda"), torch.tensor([20.0, 95.0], device="cuda"),
+           torch.ones(H, device="cuda"))
+    a, b = (torch.randn(1, H, N, V, generator=torch.Generator(device="cuda").manual_seed(5),
+                        device="cuda") for _ in range(2))
+    got = ops.ssd_recurrence(xbc, dt, *par, a, step, H, V, N, 1)
+    ops.USE_SSD_CHUNKS = False
+    try:
+        ref = ops.ssd_recurrence(xbc, dt, *par, b, step, H, V, N, 1)
+    finally:
+        ops.USE_SSD_CHUNKS = True
+    torch.testing.assert_close(got, ref, rtol=1e-5, atol=1e-5)
+    torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-5)
