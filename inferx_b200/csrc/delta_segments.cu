@@ -1,0 +1,446 @@
+// The gated delta rule of delta_parts.cu over prompts long enough to be cut into segments that
+// are walked side by side.  Per head, with D_t = diag(g_t) S_(t-1):
+//
+//   u_t = beta_t (v_t - D_t^T k_t),   S_t = D_t + k_t u_t^T,   o_t = D_t^T q_t + (k_t . q_t) u_t
+//
+// which is linear in the state, S_t = A_t S_(t-1) + beta_t k_t v_t^T with
+// A_t = (I - beta_t k_t k_t^T) diag(g_t).  Four passes:
+//   prepare  unit vectors q (times q_scale) and k in fp32, k . q and beta of every token
+//   local    every segment but a sequence's last, from a zero state without outputs: its own state,
+//            and, as the same walk over the identity's columns with values of zero, the product
+//            of its A_t
+//   join     the segments' start states, S <- A_e S + S_e in ascending e, from the slot's state on
+//   walk     every segment from its start state, with outputs; the last one leaves the slot's state
+// All of it is fp32, as in the walk from end to end, and differs from it by rounding only.
+//
+// In local and walk LANES neighbouring lanes share a column of the state, KQ float4 of it each, in
+// registers: a token's two sums over the key's entries are met by shuffles inside the warp, warps
+// meet once per 16 tokens, and a float4 of k, q and g from shared memory serves 32 / LANES columns.
+// Multiplies and adds are packed, two to an instruction; the chunks arrive by cp.async, two
+// buffers.  What bounds it is the issue of those instructions.  Measured (B200, 16 heads of 64 x
+// 128, 2,048 tokens): walks whose eight warps were slices of the key that met at a barrier for
+// every token, and that made the unit vectors once per column tile, took 595 us for both passes,
+// these four 330 us (32 heads 1,104 and 542, 8 heads 477 and 274, 701 tokens 277 and 175).
+#include "common.cuh"
+
+#define DS_CHUNK 16
+#define DS_THREADS 128
+#define DS_WARPS (DS_THREADS / 32)
+
+typedef unsigned long long ds_pair;       // two fp32 numbers
+
+__device__ __forceinline__ ds_pair ds_pack(float a, float b) {
+  ds_pair r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 ds_unpack(ds_pair p) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ ds_pair ds_mul2(ds_pair a, ds_pair b) {
+  ds_pair r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ ds_pair ds_fma2(ds_pair a, ds_pair b, ds_pair c) {
+  ds_pair r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ void ds_async(void* dst, const void* src, int bytes) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  if (bytes == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
+}
+
+// ---------------------------------------------------------------------------
+// prepare: a warp per (token, key head); rows of KP entries, zero from K on
+// ---------------------------------------------------------------------------
+template <typename TA>
+__global__ void __launch_bounds__(128)
+delta_prepare_kernel(const TA* __restrict__ q, long long ldq, const TA* __restrict__ k,
+                     long long ldk, const TA* __restrict__ beta_raw, long long ldb,
+                     float* __restrict__ qn, float* __restrict__ kn, float* __restrict__ kq,
+                     float* __restrict__ beta, int T, int H, int HK, int K, int KP,
+                     float unit_eps, float q_scale) {
+  IX_PDL_WAIT();
+  const int t = blockIdx.x, lane = threadIdx.x & 31;
+  for (int h = threadIdx.x; h < H && blockIdx.y == 0; h += 128)
+    beta[(size_t)t * H + h] = 1.0f / (1.0f + expf(-to_f32(beta_raw[(size_t)t * ldb + h])));
+  const int j = blockIdx.y * 4 + (threadIdx.x >> 5);
+  if (j >= HK) return;
+  const TA* qr = q + (size_t)t * ldq + (size_t)j * K;
+  const TA* kr = k + (size_t)t * ldk + (size_t)j * K;
+  float sq = 0.f, sk = 0.f;
+  for (int c = lane; c < K; c += 32) {
+    const float a = to_f32(qr[c]), b = to_f32(kr[c]);
+    sq = fmaf(a, a, sq);
+    sk = fmaf(b, b, sk);
+  }
+  const float iq = q_scale / sqrtf(warp_sum(sq) + unit_eps);
+  const float ik = 1.0f / sqrtf(warp_sum(sk) + unit_eps);
+  const size_t at = ((size_t)t * HK + j) * KP;
+  float dot = 0.f;
+  for (int c = lane; c < KP; c += 32) {
+    const float a = c < K ? to_f32(qr[c]) * iq : 0.f, b = c < K ? to_f32(kr[c]) * ik : 0.f;
+    qn[at + c] = a;
+    kn[at + c] = b;
+    dot = fmaf(a, b, dot);
+  }
+  dot = warp_sum(dot);
+  if (lane == 0) kq[(size_t)t * HK + j] = dot;
+}
+
+// ---------------------------------------------------------------------------
+// local and walk: grid (column tiles * segments, heads, sequences)
+// ---------------------------------------------------------------------------
+struct DsIn {
+  const float *qn, *kn, *kq, *beta, *decay;
+  const int *cu_q, *state_slot;
+  int H, HK, K, V, seg_len, nseg, vec_g;
+};
+
+template <typename TA, int LANES, int KQ, bool LOCAL>
+__global__ void __launch_bounds__(DS_THREADS, KQ <= 4 ? 5 : 3)
+delta_segment_kernel(DsIn in, const TA* __restrict__ v, long long ldv, float* __restrict__ state,
+                     float* __restrict__ out, float* __restrict__ scr_s,
+                     float* __restrict__ scr_a) {
+  constexpr int CW = 32 / LANES, COLS = DS_WARPS * CW;    // columns of a warp, of a block
+  constexpr int KP = LANES * KQ * 4;
+  constexpr int ROWS = DS_CHUNK * KP;                     // floats of one operand's chunk
+  constexpr int PV = DS_CHUNK * COLS / DS_THREADS;        // values a thread stages
+  extern __shared__ __align__(16) float sm[];
+  float* q_s = sm;                          // [2][DS_CHUNK][KP]
+  float* k_s = q_s + 2 * ROWS;
+  float* g_s = k_s + 2 * ROWS;
+  float* v_s = g_s + 2 * ROWS;              // [2][DS_CHUNK][COLS]
+  float* b_s = v_s + 2 * DS_CHUNK * COLS;   // [2][DS_CHUNK] beta
+  float* kq_s = b_s + 2 * DS_CHUNK;         // [2][DS_CHUNK]
+  IX_PDL_WAIT();
+  const int K = in.K, V = in.V, H = in.H;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int l = lane % LANES;               // entries 4 (l + LANES i) + {0..3}, i < KQ
+  const int my_col = warp * CW + lane / LANES;
+  const int vtiles = (V + COLS - 1) / COLS;
+  const int tiles = vtiles + (LOCAL ? (K + COLS - 1) / COLS : 0);
+  const int seg = blockIdx.x / tiles, tile = blockIdx.x % tiles;
+  const bool a_tile = tile >= vtiles;       // columns of the segment's transition matrix
+  const int v0 = (a_tile ? tile - vtiles : tile) * COLS, h = blockIdx.y, s = blockIdx.z;
+  const int col = v0 + my_col, width = a_tile ? K : V;
+  const int j = h / (H / in.HK);
+  const int seq_begin = in.cu_q[s], seq_end = in.cu_q[s + 1];
+  const int nseg_s = (seq_end - seq_begin + in.seg_len - 1) / in.seg_len;
+  if (seg >= nseg_s || (LOCAL && seg == nseg_s - 1)) return;
+  const int t_begin = seq_begin + seg * in.seg_len, t_end = min(seq_end, t_begin + in.seg_len);
+  const size_t cell = ((size_t)s * H + h) * in.nseg + seg;
+  float* my_s = scr_s + cell * K * V;       // local: the segment's own state; walk: its start
+  float* my_a = scr_a + cell * K * K;
+  auto entry = [&](int i) { return 4 * (l + LANES * (i >> 2)) + (i & 3); };
+
+  ds_pair S[KQ * 2];
+#pragma unroll
+  for (int i = 0; i < KQ * 2; ++i) {
+    float f[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int kk = entry(2 * i + e);
+      const bool ok = kk < K && col < width;
+      f[e] = LOCAL ? (a_tile && ok && kk == col ? 1.f : 0.f)
+                   : (ok ? my_s[(size_t)kk * V + col] : 0.f);
+    }
+    S[i] = ds_pack(f[0], f[1]);
+  }
+
+  float pv[PV];
+  auto fetch_v = [&](int t0) {
+#pragma unroll
+    for (int e = 0; e < PV; ++e) {
+      const int i = tid + e * DS_THREADS, c = i / COLS, x = v0 + i % COLS;
+      pv[e] = (!a_tile && t0 + c < t_end && x < V)
+                  ? to_f32(v[(size_t)(t0 + c) * ldv + (size_t)h * V + x]) : 0.f;
+    }
+  };
+  auto fetch = [&](int t0, int buf) {
+    const int n = min(DS_CHUNK, t_end - t0);
+    for (int i = tid; i < n * (KP / 4); i += DS_THREADS) {
+      const int c = i / (KP / 4), x = (i % (KP / 4)) * 4;
+      const size_t row = ((size_t)(t0 + c) * in.HK + j) * KP + x;
+      const int at = buf * ROWS + c * KP + x;
+      if (!LOCAL) ds_async(q_s + at, in.qn + row, 16);
+      ds_async(k_s + at, in.kn + row, 16);
+      const float* g = in.decay + ((size_t)(t0 + c) * H + h) * K + x;
+      if (in.vec_g) {
+        if (x < K) ds_async(g_s + at, g, 16);
+        else *reinterpret_cast<float4*>(g_s + at) = make_float4(0.f, 0.f, 0.f, 0.f);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) g_s[at + e] = x + e < K ? g[e] : 0.f;
+      }
+    }
+    if (tid < n) ds_async(b_s + buf * DS_CHUNK + tid, in.beta + (size_t)(t0 + tid) * H + h, 4);
+    else if (!LOCAL && tid >= 32 && tid - 32 < n)
+      ds_async(kq_s + buf * DS_CHUNK + tid - 32, in.kq + (size_t)(t0 + tid - 32) * in.HK + j, 4);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(t_begin, 0);
+  fetch_v(t_begin);
+  int buf = 0;
+  for (int t0 = t_begin; t0 < t_end; t0 += DS_CHUNK, buf ^= 1) {
+    const int n = min(DS_CHUNK, t_end - t0);
+#pragma unroll
+    for (int e = 0; e < PV; ++e) v_s[buf * DS_CHUNK * COLS + tid + e * DS_THREADS] = pv[e];
+    if (t0 + DS_CHUNK < t_end) {
+      fetch(t0 + DS_CHUNK, buf ^ 1);
+      fetch_v(t0 + DS_CHUNK);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    const ulonglong2* g4 = reinterpret_cast<const ulonglong2*>(g_s + buf * ROWS) + l;
+    const ulonglong2* k4 = reinterpret_cast<const ulonglong2*>(k_s + buf * ROWS) + l;
+    const ulonglong2* q4 = reinterpret_cast<const ulonglong2*>(q_s + buf * ROWS) + l;
+    const float* vc = v_s + buf * DS_CHUNK * COLS + my_col;
+    const float* bc = b_s + buf * DS_CHUNK;
+    const float* dc = kq_s + buf * DS_CHUNK;
+    float* dst = LOCAL ? nullptr : out + ((size_t)t0 * H + h) * V + col;
+#pragma unroll 2
+    for (int c = 0; c < n; ++c) {
+      ds_pair ka = 0, kb = 0, qa = 0, qb = 0;
+      ulonglong2 kv[KQ];
+#pragma unroll
+      for (int i = 0; i < KQ; ++i) {
+        const ulonglong2 gv = g4[i * LANES];
+        kv[i] = k4[i * LANES];
+        S[2 * i] = ds_mul2(gv.x, S[2 * i]);
+        S[2 * i + 1] = ds_mul2(gv.y, S[2 * i + 1]);
+        ka = ds_fma2(S[2 * i], kv[i].x, ka);
+        kb = ds_fma2(S[2 * i + 1], kv[i].y, kb);
+        if (!LOCAL) {
+          const ulonglong2 qv = q4[i * LANES];
+          qa = ds_fma2(S[2 * i], qv.x, qa);
+          qb = ds_fma2(S[2 * i + 1], qv.y, qb);
+        }
+      }
+      const float2 k0 = ds_unpack(ka), k1 = ds_unpack(kb);
+      float kd = (k0.x + k0.y) + (k1.x + k1.y);
+#pragma unroll
+      for (int o = 1; o < LANES; o <<= 1) kd += __shfl_xor_sync(0xffffffffu, kd, o);
+      const float u = __fmul_rn(bc[c], vc[c * COLS] - kd);
+      const ds_pair uu = ds_pack(u, u);
+#pragma unroll
+      for (int i = 0; i < KQ; ++i) {
+        S[2 * i] = ds_fma2(kv[i].x, uu, S[2 * i]);
+        S[2 * i + 1] = ds_fma2(kv[i].y, uu, S[2 * i + 1]);
+      }
+      if (!LOCAL) {
+        const float2 q0 = ds_unpack(qa), q1 = ds_unpack(qb);
+        float qd = (q0.x + q0.y) + (q1.x + q1.y);
+#pragma unroll
+        for (int o = 1; o < LANES; o <<= 1) qd += __shfl_xor_sync(0xffffffffu, qd, o);
+        if (l == 0 && col < V) *dst = __fmaf_rn(dc[c], u, qd);
+        dst += (size_t)H * V;
+      }
+      g4 += KP / 4;
+      k4 += KP / 4;
+      q4 += KP / 4;
+    }
+    __syncthreads();
+  }
+  if (!LOCAL && seg != nseg_s - 1) return;
+  float* st = state + ((size_t)in.state_slot[s] * H + h) * K * V;
+#pragma unroll
+  for (int i = 0; i < KQ * 2; ++i) {
+    const float2 f = ds_unpack(S[i]);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int kk = entry(2 * i + e);
+      const float x = e ? f.y : f.x;
+      if (kk >= K || col >= width) continue;
+      if (!LOCAL) st[(size_t)kk * V + col] = x;
+      else if (a_tile) my_a[(size_t)kk * K + col] = x;
+      else my_s[(size_t)kk * V + col] = x;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// join: grid (tiles of 32 value columns, heads, sequences); eight warps share the rows.  A
+// segment's own state in scratch gives way to its start state.
+// ---------------------------------------------------------------------------
+#define DJ_ROWS 8             // warps; each takes rows warp, warp + 8, ...
+
+__global__ void __launch_bounds__(DJ_ROWS * 32)
+delta_join_kernel(float* __restrict__ scr_s, const float* __restrict__ scr_a,
+                  const float* __restrict__ state, const int* __restrict__ cu_q,
+                  const int* __restrict__ state_slot, int H, int K, int V, int seg_len, int nseg) {
+  extern __shared__ __align__(16) float sm[];   // [2][K][32]: the state's columns
+  IX_PDL_WAIT();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int h = blockIdx.y, s = blockIdx.z, col = blockIdx.x * 32 + lane;
+  const int nseg_s = (cu_q[s + 1] - cu_q[s] + seg_len - 1) / seg_len;
+  if (nseg_s <= 0) return;
+  const bool ok = col < V;
+  const float* st = state + ((size_t)state_slot[s] * H + h) * K * V;
+  const size_t cell = ((size_t)s * H + h) * nseg;
+  float *x = sm, *y = sm + K * 32;
+  for (int kk = warp; kk < K; kk += DJ_ROWS) x[kk * 32 + lane] = ok ? st[(size_t)kk * V + col] : 0.f;
+  __syncthreads();
+  for (int e = 0; e < nseg_s; ++e) {
+    float* own = scr_s + (cell + e) * K * V;
+    const float* A = scr_a + (cell + e) * K * K;
+    const bool more = e + 1 < nseg_s;
+    // four rows at a time share the reads of x; a row's entries of A reach every lane at once
+    for (int k0 = warp; k0 < K; k0 += 4 * DJ_ROWS) {
+      float acc[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int kk = k0 + r * DJ_ROWS;
+        acc[r] = 0.f;
+        if (kk < K && ok) {
+          if (more) acc[r] = own[(size_t)kk * V + col];
+          own[(size_t)kk * V + col] = x[kk * 32 + lane];
+        }
+      }
+      if (!more) continue;
+      if ((K & 3) == 0) {
+#pragma unroll 2
+        for (int i = 0; i < K; i += 4) {
+          const float x0 = x[i * 32 + lane], x1 = x[(i + 1) * 32 + lane];
+          const float x2 = x[(i + 2) * 32 + lane], x3 = x[(i + 3) * 32 + lane];
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            const int kk = k0 + r * DJ_ROWS;
+            if (kk < K) {
+              const float4 a = *reinterpret_cast<const float4*>(A + (size_t)kk * K + i);
+              acc[r] = fmaf(a.w, x3, fmaf(a.z, x2, fmaf(a.y, x1, fmaf(a.x, x0, acc[r]))));
+            }
+          }
+        }
+      } else {
+        for (int i = 0; i < K; ++i) {
+          const float x0 = x[i * 32 + lane];
+#pragma unroll
+          for (int r = 0; r < 4; ++r)
+            if (k0 + r * DJ_ROWS < K)
+              acc[r] = fmaf(A[(size_t)(k0 + r * DJ_ROWS) * K + i], x0, acc[r]);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        if (k0 + r * DJ_ROWS < K) y[(k0 + r * DJ_ROWS) * 32 + lane] = acc[r];
+    }
+    __syncthreads();
+    float* z = x;
+    x = y;
+    y = z;
+  }
+}
+
+// Lanes a column, float4 of it a lane, by the key's size.
+#define DS_BY_K(K, GO)          \
+  do {                          \
+    if ((K) <= 16) GO(4, 1);    \
+    else if ((K) <= 32) GO(4, 2);  \
+    else if ((K) <= 64) GO(4, 4);  \
+    else if ((K) <= 128) GO(4, 8); \
+    else if ((K) <= 256) GO(16, 4);  \
+    else GO(16, 8);             \
+  } while (0)
+
+static inline int ds_cols(int K) { return DS_WARPS * (K <= 128 ? 8 : 2); }
+static inline int ds_pitch(int K) {
+  return K <= 16 ? 16 : K <= 32 ? 32 : K <= 64 ? 64 : K <= 128 ? 128 : K <= 256 ? 256 : 512;
+}
+static inline size_t ds_smem(int K) {
+  return 2 * ((size_t)3 * DS_CHUNK * ds_pitch(K) + DS_CHUNK * ds_cols(K) + 2 * DS_CHUNK) *
+         sizeof(float);
+}
+
+// Segments for a step whose longest sequence brings max_q_len tokens: as many as keep the local
+// pass within the blocks the device holds at once (five an SM up to keys of 64, three beyond), none
+// shorter than 64 tokens.  Returns the number of segments and sets *seg_len; 1 and 0 when the
+// sequences are walked from end to end.
+IX_API int ix_delta_recurrence_segments(int S, int H, int K, int V, int max_q_len, int min_tokens,
+                                        int max_segments, int* seg_len) {
+  *seg_len = 0;
+  if (S <= 0 || H <= 0 || K <= 0 || V <= 0 || K > 8 * 64 || max_q_len < min_tokens) return 1;
+  const int cols = ds_cols(K);
+  const long long per = (long long)S * H * ((V + cols - 1) / cols + (K + cols - 1) / cols);
+  const int resident = K <= 64 ? 5 : K <= 256 ? 3 : 1;
+  long long want = (long long)resident * 148 / per + 1;    // (the last segment has no local pass)
+  if (want > max_segments) want = max_segments;
+  if (want < 2) return 1;
+  int len = (int)((max_q_len + want - 1) / want);
+  len = (len + DS_CHUNK - 1) / DS_CHUNK * DS_CHUNK;
+  if (len < 64) len = 64;
+  const int nseg = (max_q_len + len - 1) / len;
+  if (nseg <= 1) return 1;
+  *seg_len = len;
+  return nseg;
+}
+
+// Floats of scratch: the segments' states and transitions, unit vectors, k . q and beta.
+IX_API long long ix_delta_segments_scratch_floats(int T, int S, int H, int HK, int K, int V,
+                                                  int nseg) {
+  const long long cells = (long long)S * H * nseg;
+  return ((cells * K * V + 3) & ~3LL) + ((cells * K * K + 3) & ~3LL) +
+         2LL * T * HK * ds_pitch(K) + (long long)T * (HK + H) + 8;
+}
+
+// Sequences are cut into segments of seg_len tokens (nseg covers the longest).
+IX_API int ix_delta_segments(const void* q, long long ldq, const void* k, long long ldk,
+                             const void* v, long long ldv, const void* beta_raw, long long ldb,
+                             int dtype, const float* decay, float* state, const int* cu_q,
+                             const int* state_slot, float* out, int T, int S, int H, int HK, int K,
+                             int V, float unit_eps, float q_scale, int seg_len, int nseg,
+                             float* scratch, cudaStream_t stream) {
+  if (S <= 0 || T <= 0) return IX_OK;
+  if (H <= 0 || HK <= 0 || H % HK || K <= 0 || V <= 0 || K > 8 * 64 || H > 65535 || S > 65535)
+    return IX_ERR_SIZE;
+  if (ldq < (long long)HK * K || ldk < (long long)HK * K || ldv < (long long)H * V || ldb < H)
+    return IX_ERR_SIZE;
+  if (nseg < 2 || seg_len <= 0 || seg_len % DS_CHUNK || !scratch) return IX_ERR_SIZE;
+  if ((uintptr_t)scratch & 15) return IX_ERR_ALIGN;
+  const int KP = ds_pitch(K), cols = ds_cols(K);
+  const long long cells = (long long)S * H * nseg;
+  float* scr_s = scratch;
+  float* scr_a = scr_s + ((cells * K * V + 3) & ~3LL);
+  float* qn = scr_a + ((cells * K * K + 3) & ~3LL);
+  float* kn = qn + (size_t)T * HK * KP;
+  float* kq = kn + (size_t)T * HK * KP;
+  float* beta = kq + (size_t)T * HK;
+  const int vtiles = (V + cols - 1) / cols, atiles = (K + cols - 1) / cols;
+  const DsIn in = {qn, kn, kq, beta, decay, cu_q, state_slot, H, HK, K, V, seg_len, nseg,
+                   K % 4 == 0 && ((uintptr_t)decay & 15) == 0 ? 1 : 0};
+  const size_t smem = ds_smem(K), join = (size_t)2 * K * 32 * sizeof(float);
+  if (join > 48 * 1024)
+    cudaFuncSetAttribute(delta_join_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)join);
+#define DS_ONE(L, Q, LOCAL, TILES)                                                              \
+  do {                                                                                          \
+    auto kern = delta_segment_kernel<TA, L, Q, LOCAL>;                                          \
+    if (smem > 48 * 1024)                                                                       \
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);       \
+    ix_launch(kern, dim3((TILES) * nseg, H, S), dim3(DS_THREADS), smem, stream, in, (const TA*)v, \
+              ldv, state, out, scr_s, scr_a);                                                   \
+  } while (0)
+#define DS_LOCAL(L, Q) DS_ONE(L, Q, true, vtiles + atiles)
+#define DS_WALK(L, Q) DS_ONE(L, Q, false, vtiles)
+  IX_DISPATCH_DTYPE(dtype, TA, {
+    ix_launch(delta_prepare_kernel<TA>, dim3(T, (HK + 3) / 4), dim3(128), 0, stream, (const TA*)q,
+              ldq, (const TA*)k, ldk, (const TA*)beta_raw, ldb, qn, kn, kq, beta, T, H, HK, K, KP,
+              unit_eps, q_scale);
+    DS_BY_K(K, DS_LOCAL);
+    ix_launch(delta_join_kernel, dim3((V + 31) / 32, H, S), dim3(DJ_ROWS * 32), join, stream, scr_s,
+              (const float*)scr_a, (const float*)state, cu_q, state_slot, H, K, V, seg_len, nseg);
+    DS_BY_K(K, DS_WALK);
+  });
+#undef DS_WALK
+#undef DS_LOCAL
+#undef DS_ONE
+  return ix_launch_status();
+}

@@ -2274,26 +2274,28 @@ def delta_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta_raw
             decay.shape != (T, heads * dim) or tuple(state.shape[1:]) != (heads, dim, vdim):
         raise KernelError("delta_recurrence: inputs and state do not fit together")
     out = torch.empty((T, heads, vdim), dtype=torch.float32, device=q.device)
-    # the kernel's side knows how many of its blocks the device holds at once
+    views = (_ptr(q), ctypes.c_longlong(ldq), _ptr(k), ctypes.c_longlong(ldk), _ptr(v),
+             ctypes.c_longlong(ldv), _ptr(beta_raw), ctypes.c_longlong(ldb), _dtype_code(q),
+             _ptr(decay), _ptr(state), _ptr(step.cu_q), _ptr(step.state_slot), _ptr(out))
+    # the kernels' side knows how many of their blocks the device holds at once
     seg = ctypes.c_int(0)
     nseg = _lib().ix_delta_recurrence_segments(
-        _dtype_code(q), step.num_seqs, heads, dim, vdim,
-        int(getattr(step, "max_q_len", 0) or T), RECURRENCE_SEGMENT_MIN, RECURRENCE_MAX_SEGMENTS,
-        ctypes.byref(seg))
-    if nseg < 1:
-        _check(nseg, "delta_recurrence_segments")
-    seg_len = seg.value
-    scratch = None
-    if nseg > 1:
-        scratch = torch.empty((_lib().ix_delta_recurrence_scratch_floats(
-            step.num_seqs, heads, dim, vdim, nseg),), dtype=torch.float32, device=q.device)
-    _check(_lib().ix_delta_recurrence(
-        _ptr(q), ctypes.c_longlong(ldq), _ptr(k), ctypes.c_longlong(ldk), _ptr(v),
-        ctypes.c_longlong(ldv), _ptr(beta_raw), ctypes.c_longlong(ldb), _dtype_code(q),
-        _ptr(decay), _ptr(state), _ptr(step.cu_q), _ptr(step.state_slot), _ptr(out),
-        step.num_seqs, heads, kv_heads, dim, vdim, ctypes.c_float(unit_eps),
-        ctypes.c_float(q_scale), seg_len, nseg, _ptr(scratch), _stream()), "delta_recurrence")
-    _count(2 if nseg > 1 else 1)
+        step.num_seqs, heads, dim, vdim, int(getattr(step, "max_q_len", 0) or T),
+        RECURRENCE_SEGMENT_MIN, RECURRENCE_MAX_SEGMENTS, ctypes.byref(seg))
+    if nseg <= 1:
+        _check(_lib().ix_delta_recurrence(
+            *views, step.num_seqs, heads, kv_heads, dim, vdim, ctypes.c_float(unit_eps),
+            ctypes.c_float(q_scale), _stream()), "delta_recurrence")
+        _count()
+        return out
+    size = _lib().ix_delta_segments_scratch_floats
+    size.restype = ctypes.c_longlong
+    scratch = torch.empty((size(T, step.num_seqs, heads, kv_heads, dim, vdim, nseg),),
+                          dtype=torch.float32, device=q.device)
+    _check(_lib().ix_delta_segments(
+        *views, T, step.num_seqs, heads, kv_heads, dim, vdim, ctypes.c_float(unit_eps),
+        ctypes.c_float(q_scale), seg.value, nseg, _ptr(scratch), _stream()), "delta_segments")
+    _count(4)
     return out
 
 
