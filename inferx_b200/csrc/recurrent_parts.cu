@@ -194,34 +194,24 @@ IX_API int ix_lowrank_decay(const void* x, int x_dtype, long long ldx, const flo
 }
 
 // ---------------------------------------------------------------------------
-// linear recurrence.  grid (ceil(V / 32) * segments, heads, sequences); a block is 32
+// linear recurrence.  grid (ceil(V / 32), heads, sequences); a block is 32
 // value columns times KS slices of the key channels (one warp per slice).  A thread keeps
 // its KPT entries of one state column in registers while it walks its tokens; key channels
 // do not interact, so the slices walk a chunk of tokens without meeting, leave their
 // partial outputs in shared memory, and the partials are added in ascending slice order.
 //
-// Three forms of the walk:
-//   whole (segments = 1)  a block walks all of its sequence's tokens of the step, from the
-//                         state in the slot to the state it leaves there.  The order of
-//                         every sum is fixed by (K, KS): a position's output does not
-//                         depend on how its sequence was cut into steps or chunks.
-//   local                 long prompts are cut into segments of seg_len tokens that are
-//                         walked side by side.  The first pass walks every segment but a
-//                         sequence's last from a zero state and leaves in scratch the
-//                         state it ends with and the product of its decays (entry seg + 1);
-//                         entry 0 takes the state from the slot.
-//   joined                the second pass rebuilds a segment's start state from the
-//                         entries before it, S <- P_i S + S_i in ascending i, then walks
-//                         the segment with outputs; the last segment leaves the state.
+// A block walks all of its sequence's tokens of the step, from the state in the slot to the
+// state it leaves there.  The order of every sum is fixed by (K, KS): a position's output
+// does not depend on how its sequence was cut into steps or chunks.  Long prompts are walked
+// in segments side by side: linear_segments.cu.
 // ---------------------------------------------------------------------------
 #define LR_COLS 32
 #define LR_CHUNK 16
 #define LR_PF 4
-enum { LR_WHOLE = 0, LR_LOCAL = 1, LR_JOINED = 2 };
 
 // One state entry, one token.  The roundings are spelled out (one product, two fused
 // multiply-adds; three in the bonus form), so that every path through the kernel - staged
-// chunks, vector reads, the single-token form, the pass without outputs - rounds alike.
+// chunks, vector reads, the single-token form - rounds alike.
 template <bool BONUS>
 __device__ __forceinline__ void lr_step(float& S, float u, float kk, float w, float q, float vj,
                                         float& acc) {
@@ -234,20 +224,14 @@ __device__ __forceinline__ void lr_step(float& S, float u, float kk, float w, fl
     acc = __fmaf_rn(S, q, acc);
   }
 }
-__device__ __forceinline__ void lr_step_local(float& S, float kk, float w, float vj) {
-  S = __fmaf_rn(w, S, __fmul_rn(kk, vj));
-}
-
-template <typename TA, int KPT, bool BONUS, int MODE>
+template <typename TA, int KPT, bool BONUS>
 __global__ void __launch_bounds__(LR_COLS * 8, KPT <= 8 ? 4 : (KPT <= 16 ? 3 : 1))
 linear_recurrence_kernel(const TA* __restrict__ q, long long ldq, const TA* __restrict__ k,
                          long long ldk, const TA* __restrict__ v, long long ldv,
                          const float* __restrict__ decay, const float* __restrict__ bonus,
                          float* __restrict__ state, const int* __restrict__ cu_q,
                          const int* __restrict__ state_slot, float* __restrict__ out, int H,
-                         int K, int V, int KS, float q_scale, int seg_len, int nseg,
-                         float* __restrict__ scr_s, float* __restrict__ scr_p) {
-  constexpr int mode = MODE;
+                         int K, int V, int KS, float q_scale) {
   extern __shared__ __align__(16) float sm[];
   float* q_s = sm;                       // [LR_CHUNK][K]
   float* k_s = q_s + LR_CHUNK * K;       // [LR_CHUNK][K]
@@ -256,56 +240,28 @@ linear_recurrence_kernel(const TA* __restrict__ q, long long ldq, const TA* __re
   float* part = v_s + LR_CHUNK * LR_COLS;  // [KS][LR_CHUNK][LR_COLS]
   IX_PDL_WAIT();
   const int lane = threadIdx.x & 31, ks = threadIdx.x >> 5;
-  const int vtiles = (V + LR_COLS - 1) / LR_COLS;
-  const int seg = blockIdx.x / vtiles;
-  const int v0 = (blockIdx.x % vtiles) * LR_COLS, h = blockIdx.y, s = blockIdx.z;
+  const int v0 = blockIdx.x * LR_COLS, h = blockIdx.y, s = blockIdx.z;
   const int col = v0 + lane;
   const bool col_ok = col < V;
-  const int seq_begin = cu_q[s], seq_end = cu_q[s + 1];
-  const int nseg_s = mode == LR_WHOLE ? 1 : (seq_end - seq_begin + seg_len - 1) / seg_len;
-  if (seg >= nseg_s) return;
-  const int t_begin = mode == LR_WHOLE ? seq_begin : seq_begin + seg * seg_len;
-  const int t_end = mode == LR_WHOLE ? seq_end : min(seq_end, t_begin + seg_len);
+  const int t_begin = cu_q[s], t_end = cu_q[s + 1];
+  if (t_end <= t_begin) return;
   float* st = state + ((size_t)state_slot[s] * H + h) * K * V;
-  float* my_s = scr_s + ((size_t)s * H + h) * nseg * K * V;    // entries of this (sequence, head)
-  float* my_p = scr_p + ((size_t)s * H + h) * nseg * K;
   const int kk0 = ks * KPT;
   const bool vec4 = (K & 3) == 0;      // then kk0 and every row of q_s, k_s, w_s are 16-byte marks
-  const bool walks = mode != LR_LOCAL || seg < nseg_s - 1;
 
-  float S[KPT], u[KPT], P[KPT];
+  float S[KPT], u[KPT];
 #pragma unroll
   for (int i = 0; i < KPT; ++i) {
     const int kk = kk0 + i;
-    const bool ok = kk < K && col_ok;
-    P[i] = 1.f;
     u[i] = (BONUS && kk < K) ? bonus[(size_t)h * K + kk] : 0.f;
-    if (mode == LR_WHOLE) {
-      S[i] = ok ? st[(size_t)kk * V + col] : 0.f;
-    } else if (mode == LR_LOCAL) {
-      if (seg == 0 && ok) my_s[(size_t)kk * V + col] = st[(size_t)kk * V + col];
-      S[i] = 0.f;
-    } else {
-      S[i] = ok ? my_s[(size_t)kk * V + col] : 0.f;
-    }
+    S[i] = kk < K && col_ok ? st[(size_t)kk * V + col] : 0.f;
   }
-  if (mode == LR_JOINED) {
-    for (int e = 1; e <= seg; ++e) {
-#pragma unroll
-      for (int i = 0; i < KPT; ++i) {
-        const int kk = kk0 + i;
-        if (kk < K && col_ok)
-          S[i] = my_p[(size_t)e * K + kk] * S[i] + my_s[((size_t)e * K + kk) * V + col];
-      }
-    }
-  }
-  if (!walks) return;
 
   // A sequence that brings one token (a decode step): nothing is staged.  Every thread reads
   // its slice of q, k and the decay straight from global memory (the lanes of a warp read
   // the same addresses), the slices' partial outputs meet in shared memory once.  The same
   // operations in the same order as the walk below, so the same bits.
-  if (mode == LR_WHOLE && t_end - t_begin == 1) {
+  if (t_end - t_begin == 1) {
     const size_t t = (size_t)t_begin;
     const float vj = col_ok ? to_f32(v[t * ldv + (size_t)h * V + col]) : 0.f;
     float acc = 0.f;
@@ -346,7 +302,7 @@ linear_recurrence_kernel(const TA* __restrict__ q, long long ldq, const TA* __re
       if (i < n * K) {
         const int c = i / K, kk = i % K;
         const size_t t = (size_t)(t0 + c);
-        if (mode != LR_LOCAL) pq[e] = __fmul_rn(to_f32(q[t * ldq + (size_t)h * K + kk]), q_scale);
+        pq[e] = __fmul_rn(to_f32(q[t * ldq + (size_t)h * K + kk]), q_scale);
         pk[e] = to_f32(k[t * ldk + (size_t)h * K + kk]);
         pw[e] = decay[(t * H + h) * K + kk];
       }
@@ -365,7 +321,7 @@ linear_recurrence_kernel(const TA* __restrict__ q, long long ldq, const TA* __re
       for (int e = 0; e < LR_PF; ++e) {
         const int i = threadIdx.x + e * blockDim.x;
         if (i < n * K) {
-          if (mode != LR_LOCAL) q_s[i] = pq[e];
+          q_s[i] = pq[e];
           k_s[i] = pk[e];
           w_s[i] = pw[e];
         }
@@ -375,7 +331,7 @@ linear_recurrence_kernel(const TA* __restrict__ q, long long ldq, const TA* __re
       for (int i = threadIdx.x; i < n * K; i += blockDim.x) {
         const int c = i / K, kk = i % K;
         const size_t t = (size_t)(t0 + c);
-        if (mode != LR_LOCAL) q_s[i] = __fmul_rn(to_f32(q[t * ldq + (size_t)h * K + kk]), q_scale);
+        q_s[i] = __fmul_rn(to_f32(q[t * ldq + (size_t)h * K + kk]), q_scale);
         k_s[i] = to_f32(k[t * ldk + (size_t)h * K + kk]);
         w_s[i] = decay[(t * H + h) * K + kk];
       }
@@ -387,38 +343,6 @@ linear_recurrence_kernel(const TA* __restrict__ q, long long ldq, const TA* __re
     __syncthreads();
     if (prefetch && t0 + LR_CHUNK < t_end)
       fetch(t0 + LR_CHUNK, min(LR_CHUNK, t_end - t0 - LR_CHUNK));
-    if (mode == LR_LOCAL) {
-#pragma unroll 4
-      for (int c = 0; c < n; ++c) {
-        const float vj = v_s[c * LR_COLS + lane];
-        const float* kc = k_s + c * K + kk0;
-        const float* wc = w_s + c * K + kk0;
-        if (vec4) {      // K a multiple of 4: four channels a shared-memory read
-#pragma unroll
-          for (int i = 0; i < KPT; i += 4) {
-            if (kk0 + i < K) {
-              const float4 k4 = *reinterpret_cast<const float4*>(kc + i);
-              const float4 w4 = *reinterpret_cast<const float4*>(wc + i);
-              lr_step_local(S[i], k4.x, w4.x, vj);
-              lr_step_local(S[i + 1], k4.y, w4.y, vj);
-              lr_step_local(S[i + 2], k4.z, w4.z, vj);
-              lr_step_local(S[i + 3], k4.w, w4.w, vj);
-              P[i] *= w4.x; P[i + 1] *= w4.y; P[i + 2] *= w4.z; P[i + 3] *= w4.w;
-            }
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < KPT; ++i) {
-            if (kk0 + i < K) {
-              lr_step_local(S[i], kc[i], wc[i], vj);
-              P[i] *= wc[i];
-            }
-          }
-        }
-      }
-      __syncthreads();
-      continue;
-    }
 #pragma unroll 4
     for (int c = 0; c < n; ++c) {
       const float vj = v_s[c * LR_COLS + lane];
@@ -460,16 +384,6 @@ linear_recurrence_kernel(const TA* __restrict__ q, long long ldq, const TA* __re
     }
     __syncthreads();
   }
-  if (mode == LR_LOCAL) {
-#pragma unroll
-    for (int i = 0; i < KPT; ++i) {
-      const int kk = kk0 + i;
-      if (kk < K && col_ok) my_s[((size_t)(seg + 1) * K + kk) * V + col] = S[i];
-      if (kk < K && v0 == 0 && lane == 0) my_p[(size_t)(seg + 1) * K + kk] = P[i];
-    }
-    return;
-  }
-  if (mode == LR_JOINED && seg != nseg_s - 1) return;
 #pragma unroll
   for (int i = 0; i < KPT; ++i) {
     const int kk = kk0 + i;
@@ -479,52 +393,32 @@ linear_recurrence_kernel(const TA* __restrict__ q, long long ldq, const TA* __re
 
 IX_API int ix_linear_recurrence_max_dim() { return 8 * 64; }
 
-// Floats of scratch the segmented walk needs for `S` sequences cut into `nseg` segments.
-IX_API long long ix_linear_recurrence_scratch_floats(int S, int H, int K, int V, int nseg) {
-  return nseg <= 1 ? 0 : (long long)S * H * nseg * ((long long)K * V + K);
-}
-
 template <typename TA, int KPT>
 static void launch_recurrence(const void* q, long long ldq, const void* k, long long ldk,
                               const void* v, long long ldv, const float* decay,
                               const float* bonus, float* state, const int* cu_q,
                               const int* state_slot, float* out, int S, int H, int K, int V,
-                              int KS, float q_scale, int bonus_form, size_t smem, int seg_len,
-                              int nseg, float* scratch, cudaStream_t stream) {
-  const int vtiles = (V + LR_COLS - 1) / LR_COLS;
-  dim3 grid(vtiles * nseg, H, S), block(LR_COLS * KS);
-  float* scr_s = scratch;
-  float* scr_p = scratch ? scratch + (size_t)S * H * nseg * K * V : nullptr;
-  auto go = [&](auto kern, int seg_len_, int nseg_) {
+                              int KS, float q_scale, int bonus_form, size_t smem,
+                              cudaStream_t stream) {
+  dim3 grid((V + LR_COLS - 1) / LR_COLS, H, S), block(LR_COLS * KS);
+  auto go = [&](auto kern) {
     if (smem > 48 * 1024)
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     ix_launch(kern, grid, block, smem, stream, (const TA*)q, ldq, (const TA*)k, ldk, (const TA*)v,
-              ldv, decay, bonus, state, cu_q, state_slot, out, H, K, V, KS, q_scale, seg_len_,
-              nseg_, scr_s, scr_p);
+              ldv, decay, bonus, state, cu_q, state_slot, out, H, K, V, KS, q_scale);
   };
-  if (nseg <= 1) {
-    if (bonus_form) go(linear_recurrence_kernel<TA, KPT, true, LR_WHOLE>, 0, 1);
-    else go(linear_recurrence_kernel<TA, KPT, false, LR_WHOLE>, 0, 1);
-    return;
-  }
-  go(linear_recurrence_kernel<TA, KPT, false, LR_LOCAL>, seg_len, nseg);
-  if (bonus_form) go(linear_recurrence_kernel<TA, KPT, true, LR_JOINED>, seg_len, nseg);
-  else go(linear_recurrence_kernel<TA, KPT, false, LR_JOINED>, seg_len, nseg);
+  if (bonus_form) go(linear_recurrence_kernel<TA, KPT, true>);
+  else go(linear_recurrence_kernel<TA, KPT, false>);
 }
 
-// seg_len, nseg: 0, 1 for the walk from end to end; otherwise every sequence is cut into
-// segments of seg_len tokens (nseg covers the longest) and `scratch` holds
-// ix_linear_recurrence_scratch_floats(...) floats.
 IX_API int ix_linear_recurrence(const void* q, long long ldq, const void* k, long long ldk,
                                 const void* v, long long ldv, int dtype, const float* decay,
                                 const float* bonus, float* state, const int* cu_q,
                                 const int* state_slot, float* out, int S, int H, int K, int V,
-                                float q_scale, int bonus_form, int seg_len, int nseg,
-                                float* scratch, cudaStream_t stream) {
+                                float q_scale, int bonus_form, cudaStream_t stream) {
   if (S <= 0) return IX_OK;
   if (H <= 0 || K <= 0 || V <= 0 || K > 8 * 64 || H > 65535 || S > 65535) return IX_ERR_SIZE;
   if (bonus_form && !bonus) return IX_ERR_SIZE;
-  if (nseg < 1 || (nseg > 1 && (seg_len <= 0 || !scratch))) return IX_ERR_SIZE;
   const int KS = K > 32 ? 8 : (K > 8 ? 4 : 1);
   const int kpt = (K + KS - 1) / KS;
   const size_t smem =
@@ -535,8 +429,7 @@ IX_API int ix_linear_recurrence(const void* q, long long ldq, const void* k, lon
   IX_DISPATCH_DTYPE(dtype, TA,                                                                  \
                     (launch_recurrence<TA, KPT>(q, ldq, k, ldk, v, ldv, decay, bonus, state,    \
                                                 cu_q, state_slot, out, S, H, K, V, KS, q_scale, \
-                                                bonus_form, smem, seg_len, nseg, scratch,       \
-                                                stream)))
+                                                bonus_form, smem, stream)))
   if (kpt <= 8) LR_GO(8);
   else if (kpt <= 16) LR_GO(16);
   else if (kpt <= 32) LR_GO(32);

@@ -2018,19 +2018,28 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: 
     if bonus_form and (bonus is None or bonus.numel() != heads * dim):
         raise KernelError("linear_recurrence: the bonus form needs u [heads, dim]")
     out = torch.empty((T, heads, vdim), dtype=torch.float32, device=q.device)
-    seg_len, nseg = recurrence_segments(int(getattr(step, "max_q_len", 0) or T), step.num_seqs,
-                                        heads, vdim)
-    scratch = None
-    if nseg > 1:
-        scratch = torch.empty((_lib().ix_linear_recurrence_scratch_floats(
-            step.num_seqs, heads, dim, vdim, nseg),), dtype=torch.float32, device=q.device)
-    _check(_lib().ix_linear_recurrence(
-        _ptr(q), ctypes.c_longlong(ldq), _ptr(k), ctypes.c_longlong(ldk), _ptr(v),
-        ctypes.c_longlong(ldv), _dtype_code(q), _ptr(decay), _ptr(bonus), _ptr(state),
-        _ptr(step.cu_q), _ptr(step.state_slot), _ptr(out), step.num_seqs, heads, dim, vdim,
-        ctypes.c_float(q_scale), 1 if bonus_form else 0, seg_len, nseg, _ptr(scratch),
-        _stream()), "linear_recurrence")
-    _count(2 if nseg > 1 else 1)
+    views = (_ptr(q), ctypes.c_longlong(ldq), _ptr(k), ctypes.c_longlong(ldk), _ptr(v),
+             ctypes.c_longlong(ldv), _dtype_code(q), _ptr(decay), _ptr(bonus), _ptr(state),
+             _ptr(step.cu_q), _ptr(step.state_slot), _ptr(out))
+    # the kernels' side knows how many of their blocks the device holds at once
+    seg = ctypes.c_int(0)
+    nseg = _lib().ix_linear_recurrence_segments(
+        step.num_seqs, heads, dim, vdim, int(getattr(step, "max_q_len", 0) or T),
+        RECURRENCE_SEGMENT_MIN, RECURRENCE_MAX_SEGMENTS, ctypes.byref(seg))
+    if nseg <= 1:
+        _check(_lib().ix_linear_recurrence(
+            *views, step.num_seqs, heads, dim, vdim, ctypes.c_float(q_scale),
+            1 if bonus_form else 0, _stream()), "linear_recurrence")
+        _count()
+        return out
+    size = _lib().ix_linear_segments_scratch_floats
+    size.restype = ctypes.c_longlong
+    scratch = torch.empty((size(T, step.num_seqs, heads, dim, vdim, nseg),), dtype=torch.float32,
+                          device=q.device)
+    _check(_lib().ix_linear_segments(
+        *views, T, step.num_seqs, heads, dim, vdim, ctypes.c_float(q_scale),
+        1 if bonus_form else 0, seg.value, nseg, _ptr(scratch), _stream()), "linear_segments")
+    _count(4)
     return out
 
 

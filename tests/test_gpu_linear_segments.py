@@ -1,0 +1,38 @@
+"""The linear recurrence in segments at every width of key that has a form of its own, at the edges
+of a segment and of the batch, against the plain statement."""
+import pytest
+import torch
+
+import host_ops
+from test_gpu_dominex import _cuda, _step
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,K,V", [(2, 16, 40), (2, 20, 33), (2, 64, 128), (2, 66, 8), (1, 128, 64),
+                                   (1, 130, 9), (1, 260, 17)])
+@pytest.mark.parametrize("q_lens", [[128], [129, 64], [1, 1, 300, 2]])
+@pytest.mark.parametrize("bonus", [False, True])
+def test_segments(dtype, H, K, V, q_lens, bonus):
+    from inferx_b200.kernels import ops
+    g = torch.Generator().manual_seed(K + V + sum(q_lens))
+    q_lens = sorted(q_lens, key=lambda n: n != 1)
+    S, T = len(q_lens), sum(q_lens)
+    st = _step(q_lens, [3] * S, slots=list(range(S))[::-1])
+    q, k = (torch.randn(T, H * K, generator=g).to(dtype) for _ in range(2))
+    v = torch.randn(T, H * V, generator=g).to(dtype)
+    decay = torch.rand(T, H * K, generator=g) * 0.3 + 0.7
+    u = torch.randn(H, K, generator=g) if bonus else None
+    state = torch.randn(S + 1, H, K, V, generator=g)
+    st_ref = state.clone()
+    ref = host_ops.linear_recurrence(q, k, v, decay, u, st_ref, st, H, K, V, 0.37, bonus)
+    before = ops.LAUNCHES[0]
+    got = state.cuda()
+    out = ops.linear_recurrence(q.cuda(), k.cuda(), v.cuda(), decay.cuda(),
+                                None if u is None else u.cuda(), got, _cuda(st), H, K, V, 0.37,
+                                bonus)
+    assert ops.LAUNCHES[0] == before + 4                  # the four passes
+    off = lambda a, b: float((a.cpu() - b.view(a.shape)).norm() / b.norm())
+    assert off(out, ref) <= 2e-5 and off(got, st_ref) <= 2e-5
+    assert torch.equal(got[S].cpu(), state[S])
