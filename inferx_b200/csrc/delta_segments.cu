@@ -13,14 +13,14 @@
 //   walk     every segment from its start state, with outputs; the last one leaves the slot's state
 // All of it is fp32, as in the walk from end to end, and differs from it by rounding only.
 //
-// In local and walk LANES neighbouring lanes share a column of the state, KQ float4 of it each, in
-// registers: a token's two sums over the key's entries are met by shuffles inside the warp, warps
-// meet once per 16 tokens, and a float4 of k, q and g from shared memory serves 32 / LANES columns.
-// Multiplies and adds are packed, two to an instruction; the chunks arrive by cp.async, two
-// buffers.  What bounds it is the issue of those instructions.  Measured (B200, 16 heads of 64 x
-// 128, 2,048 tokens): walks whose eight warps were slices of the key that met at a barrier for
+// In local and walk lanes share columns of the state, in registers (segments.cuh): a token's two
+// sums over the key's entries are met by shuffles inside the warp, and warps meet once per 16
+// tokens.  Multiplies and adds are packed, two to an instruction; the chunks arrive by cp.async,
+// two buffers.  What bounds it is the arithmetic (four multiply-adds an entry and token, 1.5 times
+// in local for the transitions) and shared-memory reads, about equally.  Measured (B200, 16 heads of
+// 64 x 128, 2,048 tokens): walks whose eight warps were slices of the key that met at a barrier for
 // every token, and that made the unit vectors once per column tile, took 595 us for both passes,
-// these four 330 us (32 heads 1,104 and 542, 8 heads 477 and 274, 701 tokens 277 and 175).
+// these four 216 us (32 heads 1,104 and 384, 8 heads 477 and 158, 256 tokens 144 and 59).
 #include "segments.cuh"
 
 // ---------------------------------------------------------------------------
@@ -70,13 +70,13 @@ struct DsIn {
   int H, HK, K, V, seg_len, nseg, vec_g;
 };
 
-template <typename TA, int LANES, int KQ, bool LOCAL>
-__global__ void __launch_bounds__(DS_THREADS, KQ <= 4 ? 5 : 3)
+template <typename TA, int KQ, int C, bool LOCAL>
+__global__ void __launch_bounds__(DS_THREADS, KQ <= 2 ? 5 : 3)
 delta_segment_kernel(DsIn in, const TA* __restrict__ v, long long ldv, float* __restrict__ state,
                      float* __restrict__ out, float* __restrict__ scr_s,
                      float* __restrict__ scr_a) {
-  constexpr int CW = 32 / LANES, COLS = DS_WARPS * CW;    // columns of a warp, of a block
-  constexpr int KP = LANES * KQ * 4;
+  constexpr int COLS = DS_GROUPS * C;                     // columns of a block
+  constexpr int KP = DS_LANES * KQ * 4;
   constexpr int ROWS = DS_CHUNK * KP;                     // floats of one operand's chunk
   constexpr int PV = DS_CHUNK * COLS / DS_THREADS;        // values a thread stages
   extern __shared__ __align__(16) float sm[];
@@ -88,15 +88,15 @@ delta_segment_kernel(DsIn in, const TA* __restrict__ v, long long ldv, float* __
   float* kq_s = b_s + 2 * DS_CHUNK;         // [2][DS_CHUNK]
   IX_PDL_WAIT();
   const int K = in.K, V = in.V, H = in.H;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int l = lane % LANES;               // entries 4 (l + LANES i) + {0..3}, i < KQ
-  const int my_col = warp * CW + lane / LANES;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int l = lane % DS_LANES;
+  const int my_col = (tid / DS_LANES) * C;  // the first of this thread's columns
   const int vtiles = (V + COLS - 1) / COLS;
   const int tiles = vtiles + (LOCAL ? (K + COLS - 1) / COLS : 0);
   const int seg = blockIdx.x / tiles, tile = blockIdx.x % tiles;
   const bool a_tile = tile >= vtiles;       // columns of the segment's transition matrix
   const int v0 = (a_tile ? tile - vtiles : tile) * COLS, h = blockIdx.y, s = blockIdx.z;
-  const int col = v0 + my_col, width = a_tile ? K : V;
+  const int col = v0 + my_col, width = a_tile ? K : V;    // columns col .. col + C - 1
   const int j = h / (H / in.HK);
   const int seq_begin = in.cu_q[s], seq_end = in.cu_q[s + 1];
   const int nseg_s = (seq_end - seq_begin + in.seg_len - 1) / in.seg_len;
@@ -105,21 +105,23 @@ delta_segment_kernel(DsIn in, const TA* __restrict__ v, long long ldv, float* __
   const size_t cell = ((size_t)s * H + h) * in.nseg + seg;
   float* my_s = scr_s + cell * K * V;       // local: the segment's own state; walk: its start
   float* my_a = scr_a + cell * K * K;
-  auto entry = [&](int i) { return 4 * (l + LANES * (i >> 2)) + (i & 3); };
+  auto entry = [&](int i) { return 4 * (l + DS_LANES * (i >> 2)) + (i & 3); };
 
-  ds_pair S[KQ * 2];
+  ds_pair S[C][KQ * 2];
 #pragma unroll
-  for (int i = 0; i < KQ * 2; ++i) {
-    float f[2];
+  for (int y = 0; y < C; ++y)
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int kk = entry(2 * i + e);
-      const bool ok = kk < K && col < width;
-      f[e] = LOCAL ? (a_tile && ok && kk == col ? 1.f : 0.f)
-                   : (ok ? my_s[(size_t)kk * V + col] : 0.f);
+    for (int i = 0; i < KQ * 2; ++i) {
+      float f[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int kk = entry(2 * i + e);
+        const bool ok = kk < K && col + y < width;
+        f[e] = LOCAL ? (a_tile && ok && kk == col + y ? 1.f : 0.f)
+                     : (ok ? my_s[(size_t)kk * V + col + y] : 0.f);
+      }
+      S[y][i] = ds_pack(f[0], f[1]);
     }
-    S[i] = ds_pack(f[0], f[1]);
-  }
 
   float pv[PV];
   auto fetch_v = [&](int t0) {
@@ -170,45 +172,59 @@ delta_segment_kernel(DsIn in, const TA* __restrict__ v, long long ldv, float* __
     const ulonglong2* g4 = reinterpret_cast<const ulonglong2*>(g_s + buf * ROWS) + l;
     const ulonglong2* k4 = reinterpret_cast<const ulonglong2*>(k_s + buf * ROWS) + l;
     const ulonglong2* q4 = reinterpret_cast<const ulonglong2*>(q_s + buf * ROWS) + l;
-    const float* vc = v_s + buf * DS_CHUNK * COLS + my_col;
+    const int own = my_col + ds_own<C>(l);        // the column whose sums this lane gets
+    const float* vc = v_s + buf * DS_CHUNK * COLS + own;
     const float* bc = b_s + buf * DS_CHUNK;
     const float* dc = kq_s + buf * DS_CHUNK;
-    float* dst = LOCAL ? nullptr : out + ((size_t)t0 * H + h) * V + col;
-#pragma unroll 2
+    float* dst = LOCAL ? nullptr : out + ((size_t)t0 * H + h) * V + v0 + own;
+    // (the lanes that share a column write it once)
+    const bool writes = (l & (DS_LANES / C - 1)) == 0 && v0 + own < V;
     for (int c = 0; c < n; ++c) {
-      ds_pair ka = 0, kb = 0, qa = 0, qb = 0;
+      ds_pair ka[C], qa[C];
       ulonglong2 kv[KQ];
 #pragma unroll
       for (int i = 0; i < KQ; ++i) {
-        const ulonglong2 gv = g4[i * LANES];
-        kv[i] = k4[i * LANES];
-        S[2 * i] = ds_mul2(gv.x, S[2 * i]);
-        S[2 * i + 1] = ds_mul2(gv.y, S[2 * i + 1]);
-        ka = ds_fma2(S[2 * i], kv[i].x, ka);
-        kb = ds_fma2(S[2 * i + 1], kv[i].y, kb);
-        if (!LOCAL) {
-          const ulonglong2 qv = q4[i * LANES];
-          qa = ds_fma2(S[2 * i], qv.x, qa);
-          qb = ds_fma2(S[2 * i + 1], qv.y, qb);
+        const ulonglong2 gv = g4[i * DS_LANES];
+        kv[i] = k4[i * DS_LANES];
+        ulonglong2 qv;
+        if (!LOCAL) qv = q4[i * DS_LANES];
+#pragma unroll
+        for (int y = 0; y < C; ++y) {
+          S[y][2 * i] = ds_mul2(gv.x, S[y][2 * i]);
+          S[y][2 * i + 1] = ds_mul2(gv.y, S[y][2 * i + 1]);
+          ka[y] = i ? ds_fma2(S[y][2 * i], kv[i].x, ka[y]) : ds_mul2(S[y][0], kv[0].x);
+          ka[y] = ds_fma2(S[y][2 * i + 1], kv[i].y, ka[y]);
+          if (!LOCAL) {
+            qa[y] = i ? ds_fma2(S[y][2 * i], qv.x, qa[y]) : ds_mul2(S[y][0], qv.x);
+            qa[y] = ds_fma2(S[y][2 * i + 1], qv.y, qa[y]);
+          }
         }
       }
-      const float2 k0 = ds_unpack(ka), k1 = ds_unpack(kb);
-      float kd = (k0.x + k0.y) + (k1.x + k1.y);
+      float part[C], u[C];
 #pragma unroll
-      for (int o = 1; o < LANES; o <<= 1) kd += __shfl_xor_sync(0xffffffffu, kd, o);
-      const float u = __fmul_rn(bc[c], vc[c * COLS] - kd);
-      const ds_pair uu = ds_pack(u, u);
+      for (int y = 0; y < C; ++y) {
+        const float2 f = ds_unpack(ka[y]);
+        part[y] = f.x + f.y;
+      }
+      const float mine = __fmul_rn(bc[c], vc[c * COLS] - ds_sum<C>(part, l));
+      ds_share<C>(mine, u, l);
 #pragma unroll
-      for (int i = 0; i < KQ; ++i) {
-        S[2 * i] = ds_fma2(kv[i].x, uu, S[2 * i]);
-        S[2 * i + 1] = ds_fma2(kv[i].y, uu, S[2 * i + 1]);
+      for (int y = 0; y < C; ++y) {
+        const ds_pair uu = ds_pack(u[y], u[y]);
+#pragma unroll
+        for (int i = 0; i < KQ; ++i) {
+          S[y][2 * i] = ds_fma2(kv[i].x, uu, S[y][2 * i]);
+          S[y][2 * i + 1] = ds_fma2(kv[i].y, uu, S[y][2 * i + 1]);
+        }
       }
       if (!LOCAL) {
-        const float2 q0 = ds_unpack(qa), q1 = ds_unpack(qb);
-        float qd = (q0.x + q0.y) + (q1.x + q1.y);
 #pragma unroll
-        for (int o = 1; o < LANES; o <<= 1) qd += __shfl_xor_sync(0xffffffffu, qd, o);
-        if (l == 0 && col < V) *dst = __fmaf_rn(dc[c], u, qd);
+        for (int y = 0; y < C; ++y) {
+          const float2 f = ds_unpack(qa[y]);
+          part[y] = f.x + f.y;
+        }
+        const float qd = ds_sum<C>(part, l);
+        if (writes) *dst = __fmaf_rn(dc[c], mine, qd);
         dst += (size_t)H * V;
       }
       g4 += KP / 4;
@@ -220,67 +236,88 @@ delta_segment_kernel(DsIn in, const TA* __restrict__ v, long long ldv, float* __
   if (!LOCAL && seg != nseg_s - 1) return;
   float* st = state + ((size_t)in.state_slot[s] * H + h) * K * V;
 #pragma unroll
-  for (int i = 0; i < KQ * 2; ++i) {
-    const float2 f = ds_unpack(S[i]);
+  for (int y = 0; y < C; ++y)
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int kk = entry(2 * i + e);
-      const float x = e ? f.y : f.x;
-      if (kk >= K || col >= width) continue;
-      if (!LOCAL) st[(size_t)kk * V + col] = x;
-      else if (a_tile) my_a[(size_t)kk * K + col] = x;
-      else my_s[(size_t)kk * V + col] = x;
+    for (int i = 0; i < KQ * 2; ++i) {
+      const float2 f = ds_unpack(S[y][i]);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int kk = entry(2 * i + e);
+        const float x = e ? f.y : f.x;
+        if (kk >= K || col + y >= width) continue;
+        if (!LOCAL) st[(size_t)kk * V + col + y] = x;
+        else if (a_tile) my_a[(size_t)kk * K + col + y] = x;
+        else my_s[(size_t)kk * V + col + y] = x;
+      }
     }
-  }
 }
 
 // ---------------------------------------------------------------------------
-// join: grid (tiles of 32 value columns, heads, sequences); eight warps share the rows.  A
-// segment's own state in scratch gives way to its start state.
+// join: grid (tiles of 16 value columns, heads, sequences); a thread owns a column and every
+// sixteenth row, four at a time.  A segment's own state in scratch gives way to its start state.
+// STAGED (K a multiple of 4 up to 128): the next segment's transitions come into shared memory
+// while this one's are applied; reading them from L2 where they are used made a step of 64 x 64
+// wait some 6 us.
 // ---------------------------------------------------------------------------
-#define DJ_ROWS 8             // warps; each takes rows warp, warp + 8, ...
+#define DJ_COLS 16
+#define DJ_THREADS 256
+#define DJ_GROUPS (DJ_THREADS / DJ_COLS)
+#define DJ_MAX_STAGED 128
 
-__global__ void __launch_bounds__(DJ_ROWS * 32)
+template <bool STAGED>
+__global__ void __launch_bounds__(DJ_THREADS)
 delta_join_kernel(float* __restrict__ scr_s, const float* __restrict__ scr_a,
                   const float* __restrict__ state, const int* __restrict__ cu_q,
                   const int* __restrict__ state_slot, int H, int K, int V, int seg_len, int nseg) {
-  extern __shared__ __align__(16) float sm[];   // [2][K][32]: the state's columns
+  extern __shared__ __align__(16) float sm[];   // [2][K][DJ_COLS] the state's columns, [2][K][K]
   IX_PDL_WAIT();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int h = blockIdx.y, s = blockIdx.z, col = blockIdx.x * 32 + lane;
+  const int tid = threadIdx.x, c = tid % DJ_COLS, group = tid / DJ_COLS;
+  const int h = blockIdx.y, s = blockIdx.z, col = blockIdx.x * DJ_COLS + c;
   const int nseg_s = (cu_q[s + 1] - cu_q[s] + seg_len - 1) / seg_len;
   if (nseg_s <= 0) return;
   const bool ok = col < V;
   const float* st = state + ((size_t)state_slot[s] * H + h) * K * V;
   const size_t cell = ((size_t)s * H + h) * nseg;
-  float *x = sm, *y = sm + K * 32;
-  for (int kk = warp; kk < K; kk += DJ_ROWS) x[kk * 32 + lane] = ok ? st[(size_t)kk * V + col] : 0.f;
-  __syncthreads();
+  float *x = sm, *y = sm + K * DJ_COLS;
+  float* a_s = sm + 2 * K * DJ_COLS;
+  auto fetch = [&](int e) {
+    if (STAGED && e + 1 < nseg_s) {              // (the last segment has no transitions)
+      const float* A = scr_a + (cell + e) * K * K;
+      float* to = a_s + (size_t)(e & 1) * K * K;
+      for (int i = tid * 4; i < K * K; i += DJ_THREADS * 4) ds_async(to + i, A + i, 16);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(0);
+  for (int kk = group; kk < K; kk += DJ_GROUPS)
+    x[kk * DJ_COLS + c] = ok ? st[(size_t)kk * V + col] : 0.f;
   for (int e = 0; e < nseg_s; ++e) {
     float* own = scr_s + (cell + e) * K * V;
-    const float* A = scr_a + (cell + e) * K * K;
+    const float* A = STAGED ? a_s + (size_t)(e & 1) * K * K : scr_a + (cell + e) * K * K;
     const bool more = e + 1 < nseg_s;
-    // four rows at a time share the reads of x; a row's entries of A reach every lane at once
-    for (int k0 = warp; k0 < K; k0 += 4 * DJ_ROWS) {
+    fetch(e + 1);                                // its buffer was last read before the barrier
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    for (int k0 = group; k0 < K; k0 += 4 * DJ_GROUPS) {
       float acc[4];
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
-        const int kk = k0 + r * DJ_ROWS;
+        const int kk = k0 + r * DJ_GROUPS;
         acc[r] = 0.f;
         if (kk < K && ok) {
           if (more) acc[r] = own[(size_t)kk * V + col];
-          own[(size_t)kk * V + col] = x[kk * 32 + lane];
+          own[(size_t)kk * V + col] = x[kk * DJ_COLS + c];
         }
       }
       if (!more) continue;
       if ((K & 3) == 0) {
-#pragma unroll 2
+#pragma unroll 4
         for (int i = 0; i < K; i += 4) {
-          const float x0 = x[i * 32 + lane], x1 = x[(i + 1) * 32 + lane];
-          const float x2 = x[(i + 2) * 32 + lane], x3 = x[(i + 3) * 32 + lane];
+          const float x0 = x[i * DJ_COLS + c], x1 = x[(i + 1) * DJ_COLS + c];
+          const float x2 = x[(i + 2) * DJ_COLS + c], x3 = x[(i + 3) * DJ_COLS + c];
 #pragma unroll
           for (int r = 0; r < 4; ++r) {
-            const int kk = k0 + r * DJ_ROWS;
+            const int kk = k0 + r * DJ_GROUPS;
             if (kk < K) {
               const float4 a = *reinterpret_cast<const float4*>(A + (size_t)kk * K + i);
               acc[r] = fmaf(a.w, x3, fmaf(a.z, x2, fmaf(a.y, x1, fmaf(a.x, x0, acc[r]))));
@@ -289,16 +326,16 @@ delta_join_kernel(float* __restrict__ scr_s, const float* __restrict__ scr_a,
         }
       } else {
         for (int i = 0; i < K; ++i) {
-          const float x0 = x[i * 32 + lane];
+          const float x0 = x[i * DJ_COLS + c];
 #pragma unroll
           for (int r = 0; r < 4; ++r)
-            if (k0 + r * DJ_ROWS < K)
-              acc[r] = fmaf(A[(size_t)(k0 + r * DJ_ROWS) * K + i], x0, acc[r]);
+            if (k0 + r * DJ_GROUPS < K)
+              acc[r] = fmaf(A[(size_t)(k0 + r * DJ_GROUPS) * K + i], x0, acc[r]);
         }
       }
 #pragma unroll
       for (int r = 0; r < 4; ++r)
-        if (k0 + r * DJ_ROWS < K) y[(k0 + r * DJ_ROWS) * 32 + lane] = acc[r];
+        if (k0 + r * DJ_GROUPS < K) y[(k0 + r * DJ_GROUPS) * DJ_COLS + c] = acc[r];
     }
     __syncthreads();
     float* z = x;
@@ -322,8 +359,7 @@ IX_API int ix_delta_recurrence_segments(int S, int H, int K, int V, int max_q_le
   if (S <= 0 || H <= 0 || K <= 0 || V <= 0 || K > 8 * 64 || max_q_len < min_tokens) return 1;
   const int cols = ds_cols(K);
   const long long per = (long long)S * H * ((V + cols - 1) / cols + (K + cols - 1) / cols);
-  const int resident = K <= 64 ? 5 : K <= 256 ? 3 : 1;
-  long long want = (long long)resident * 148 / per + 1;    // (the last segment has no local pass)
+  long long want = (long long)ds_resident(K) * 148 / per + 1;    // (the last segment has no local pass)
   if (want > max_segments) want = max_segments;
   if (want < 2) return 1;
   int len = (int)((max_q_len + want - 1) / want);
@@ -368,9 +404,12 @@ IX_API int ix_delta_segments(const void* q, long long ldq, const void* k, long l
   const int vtiles = (V + cols - 1) / cols, atiles = (K + cols - 1) / cols;
   const DsIn in = {qn, kn, kq, beta, decay, cu_q, state_slot, H, HK, K, V, seg_len, nseg,
                    K % 4 == 0 && ((uintptr_t)decay & 15) == 0 ? 1 : 0};
-  const size_t smem = ds_smem(K), join = (size_t)2 * K * 32 * sizeof(float);
+  const bool staged = K % 4 == 0 && K <= DJ_MAX_STAGED;
+  const size_t smem = ds_smem(K);
+  const size_t join = ((size_t)2 * K * DJ_COLS + (staged ? (size_t)2 * K * K : 0)) * sizeof(float);
+  auto join_kern = staged ? delta_join_kernel<true> : delta_join_kernel<false>;
   if (join > 48 * 1024)
-    cudaFuncSetAttribute(delta_join_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)join);
+    cudaFuncSetAttribute(join_kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)join);
 #define DS_ONE(L, Q, LOCAL, TILES)                                                              \
   do {                                                                                          \
     auto kern = delta_segment_kernel<TA, L, Q, LOCAL>;                                          \
@@ -386,8 +425,8 @@ IX_API int ix_delta_segments(const void* q, long long ldq, const void* k, long l
               ldq, (const TA*)k, ldk, (const TA*)beta_raw, ldb, qn, kn, kq, beta, T, H, HK, K, KP,
               unit_eps, q_scale);
     DS_BY_K(K, DS_LOCAL);
-    ix_launch(delta_join_kernel, dim3((V + 31) / 32, H, S), dim3(DJ_ROWS * 32), join, stream, scr_s,
-              (const float*)scr_a, (const float*)state, cu_q, state_slot, H, K, V, seg_len, nseg);
+    ix_launch(join_kern, dim3((V + DJ_COLS - 1) / DJ_COLS, H, S), dim3(DJ_THREADS), join, stream,
+              scr_s, (const float*)scr_a, (const float*)state, cu_q, state_slot, H, K, V, seg_len, nseg);
     DS_BY_K(K, DS_WALK);
   });
 #undef DS_WALK

@@ -12,10 +12,11 @@
 //   walk     every segment from its start state, with outputs; the last one leaves the slot's state
 // All of it is fp32, as in the walk from end to end, and differs from it by rounding only.
 //
-// Lanes, packed arithmetic and the chunks' copies are laid out as in delta_segments.cu; what bounds
-// it is the issue of the multiplies and adds.  Walks whose eight warps were slices of the key over
-// 32 shared columns took 217 us for the two passes over 1,777 tokens of 16 heads of 64 x 128, 237
-// with the bonus for 32 heads of 64 x 64; over 2,048 tokens of 16 heads 243 us, these four 203.
+// Lanes and columns, packed arithmetic and the chunks' copies are laid out as in delta_segments.cu
+// (segments.cuh); what bounds it is the arithmetic (three multiply-adds an entry and token, two in
+// local).  Walks whose eight warps were slices of the key over 32 shared columns took 243 us for
+// the two passes over 2,048 tokens of 16 heads of 64 x 128, 261 with the bonus, these four
+// 111 and 125 (32 heads 472 and 217, 8 heads 161 and 67, 256 tokens 49 and 32).
 #include "segments.cuh"
 
 // ---------------------------------------------------------------------------
@@ -48,14 +49,14 @@ struct LsIn {
 };
 enum { LS_LOCAL = 0, LS_WALK = 1, LS_BONUS = 2 };
 
-template <typename TA, int LANES, int KQ, int FORM>
-__global__ void __launch_bounds__(DS_THREADS, KQ <= 4 ? 5 : 3)
+template <typename TA, int KQ, int C, int FORM>
+__global__ void __launch_bounds__(DS_THREADS, KQ <= 2 ? 5 : 3)
 linear_segment_kernel(LsIn in, const TA* __restrict__ v, long long ldv, float* __restrict__ state,
                       float* __restrict__ out, float* __restrict__ scr_s,
                       float* __restrict__ scr_p) {
   constexpr bool LOCAL = FORM == LS_LOCAL, BONUS = FORM == LS_BONUS;
-  constexpr int CW = 32 / LANES, COLS = DS_WARPS * CW;    // columns of a warp, of a block
-  constexpr int KP = LANES * KQ * 4;
+  constexpr int COLS = DS_GROUPS * C;                     // columns of a block
+  constexpr int KP = DS_LANES * KQ * 4;
   constexpr int ROWS = DS_CHUNK * KP;                     // floats of one operand's chunk
   constexpr int PV = DS_CHUNK * COLS / DS_THREADS;        // values a thread stages
   extern __shared__ __align__(16) float sm[];
@@ -66,8 +67,8 @@ linear_segment_kernel(LsIn in, const TA* __restrict__ v, long long ldv, float* _
   IX_PDL_WAIT();
   const int K = in.K, V = in.V, H = in.H;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int l = lane % LANES;               // entries 4 (l + LANES i) + {0..3}, i < KQ
-  const int my_col = warp * CW + lane / LANES;
+  const int l = lane % DS_LANES;
+  const int my_col = (tid / DS_LANES) * C;  // the first of this thread's columns
   const int tiles = (V + COLS - 1) / COLS;
   const int seg = blockIdx.x / tiles, v0 = (blockIdx.x % tiles) * COLS;
   const int h = blockIdx.y, s = blockIdx.z, col = v0 + my_col;
@@ -79,21 +80,29 @@ linear_segment_kernel(LsIn in, const TA* __restrict__ v, long long ldv, float* _
   float* my_s = scr_s + cell * K * V;       // local: the segment's own state; walk: its start
   float* my_p = scr_p + cell * K;
   const bool keeps_p = LOCAL && v0 == 0 && warp == 0;     // the decays' products
-  auto entry = [&](int i) { return 4 * (l + LANES * (i >> 2)) + (i & 3); };
+  auto entry = [&](int i) { return 4 * (l + DS_LANES * (i >> 2)) + (i & 3); };
 
-  ds_pair S[KQ * 2], u[KQ * 2], P[KQ * 2];
+  ds_pair S[C][KQ * 2], u[KQ * 2], P[KQ * 2];
 #pragma unroll
   for (int i = 0; i < KQ * 2; ++i) {
-    float f[2], uf[2];
+    float uf[2];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int kk = entry(2 * i + e);
-      f[e] = !LOCAL && kk < K && col < V ? my_s[(size_t)kk * V + col] : 0.f;
       uf[e] = BONUS && kk < K ? in.bonus[(size_t)h * K + kk] : 0.f;
     }
-    S[i] = ds_pack(f[0], f[1]);
     u[i] = ds_pack(uf[0], uf[1]);
     P[i] = ds_pack(1.f, 1.f);
+#pragma unroll
+    for (int y = 0; y < C; ++y) {
+      float f[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int kk = entry(2 * i + e);
+        f[e] = !LOCAL && kk < K && col + y < V ? my_s[(size_t)kk * V + col + y] : 0.f;
+      }
+      S[y][i] = ds_pack(f[0], f[1]);
+    }
   }
 
   float pv[PV];
@@ -142,39 +151,50 @@ linear_segment_kernel(LsIn in, const TA* __restrict__ v, long long ldv, float* _
     const ulonglong2* w4 = reinterpret_cast<const ulonglong2*>(w_s + buf * ROWS) + l;
     const ulonglong2* k4 = reinterpret_cast<const ulonglong2*>(k_s + buf * ROWS) + l;
     const ulonglong2* q4 = reinterpret_cast<const ulonglong2*>(q_s + buf * ROWS) + l;
+    const int own = my_col + ds_own<C>(l);        // the column whose sum this lane gets
     const float* vc = v_s + buf * DS_CHUNK * COLS + my_col;
-    float* dst = LOCAL ? nullptr : out + ((size_t)t0 * H + h) * V + col;
-#pragma unroll 2
+    float* dst = LOCAL ? nullptr : out + ((size_t)t0 * H + h) * V + v0 + own;
+    // (the lanes that share a column write it once)
+    const bool writes = (l & (DS_LANES / C - 1)) == 0 && v0 + own < V;
     for (int c = 0; c < n; ++c) {
-      const float vf = vc[c * COLS];
-      const ds_pair vj = ds_pack(vf, vf);
-      ds_pair acc[2] = {0, 0};
+      ds_pair vj[C], acc[C];
+#pragma unroll
+      for (int y = 0; y < C; ++y) {
+        vj[y] = ds_pack(vc[c * COLS + y], vc[c * COLS + y]);
+        acc[y] = 0;
+      }
 #pragma unroll
       for (int i = 0; i < KQ; ++i) {
-        const ulonglong2 kv = k4[i * LANES], wv = w4[i * LANES];
+        const ulonglong2 kv = k4[i * DS_LANES], wv = w4[i * DS_LANES];
         const ds_pair k2[2] = {kv.x, kv.y}, w2[2] = {wv.x, wv.y};
         ds_pair q2[2];
         if (!LOCAL) {
-          const ulonglong2 qv = q4[i * LANES];
+          const ulonglong2 qv = q4[i * DS_LANES];
           q2[0] = qv.x;
           q2[1] = qv.y;
         }
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          ds_pair& x = S[2 * i + e];
-          const ds_pair p = ds_mul2(k2[e], vj);
-          if (BONUS) acc[e] = ds_fma2(ds_fma2(u[2 * i + e], p, x), q2[e], acc[e]);
-          x = ds_fma2(w2[e], x, p);
-          if (!LOCAL && !BONUS) acc[e] = ds_fma2(x, q2[e], acc[e]);
           if (keeps_p) P[2 * i + e] = ds_mul2(P[2 * i + e], w2[e]);
+#pragma unroll
+          for (int y = 0; y < C; ++y) {
+            ds_pair& x = S[y][2 * i + e];
+            const ds_pair p = ds_mul2(k2[e], vj[y]);
+            if (BONUS) acc[y] = ds_fma2(ds_fma2(u[2 * i + e], p, x), q2[e], acc[y]);
+            x = ds_fma2(w2[e], x, p);
+            if (!LOCAL && !BONUS) acc[y] = ds_fma2(x, q2[e], acc[y]);
+          }
         }
       }
       if (!LOCAL) {
-        const float2 a0 = ds_unpack(acc[0]), a1 = ds_unpack(acc[1]);
-        float total = (a0.x + a0.y) + (a1.x + a1.y);
+        float part[C];
 #pragma unroll
-        for (int o = 1; o < LANES; o <<= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-        if (l == 0 && col < V) *dst = total;
+        for (int y = 0; y < C; ++y) {
+          const float2 f = ds_unpack(acc[y]);
+          part[y] = f.x + f.y;
+        }
+        const float total = ds_sum<C>(part, l);
+        if (writes) *dst = total;
         dst += (size_t)H * V;
       }
       w4 += KP / 4;
@@ -187,13 +207,17 @@ linear_segment_kernel(LsIn in, const TA* __restrict__ v, long long ldv, float* _
   float* st = LOCAL ? my_s : state + ((size_t)in.state_slot[s] * H + h) * K * V;
 #pragma unroll
   for (int i = 0; i < KQ * 2; ++i) {
-    const float2 f = ds_unpack(S[i]), p = ds_unpack(P[i]);
+    const float2 p = ds_unpack(P[i]);
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int kk = entry(2 * i + e);
       if (kk >= K) continue;
-      if (col < V) st[(size_t)kk * V + col] = e ? f.y : f.x;
-      if (keeps_p && lane < LANES) my_p[kk] = e ? p.y : p.x;
+      if (keeps_p && lane < DS_LANES) my_p[kk] = e ? p.y : p.x;
+#pragma unroll
+      for (int y = 0; y < C; ++y) {
+        const float2 f = ds_unpack(S[y][i]);
+        if (col + y < V) st[(size_t)kk * V + col + y] = e ? f.y : f.x;
+      }
     }
   }
 }
@@ -248,8 +272,7 @@ IX_API int ix_linear_recurrence_segments(int S, int H, int K, int V, int max_q_l
   *seg_len = 0;
   if (S <= 0 || H <= 0 || K <= 0 || V <= 0 || K > 8 * 64 || max_q_len < min_tokens) return 1;
   const long long per = (long long)S * H * ((V + ds_cols(K) - 1) / ds_cols(K));
-  const int resident = K <= 64 ? 5 : K <= 256 ? 3 : 1;
-  long long want = (long long)resident * 148 / per;
+  long long want = (long long)ds_resident(K) * 148 / per;
   if (want > max_segments) want = max_segments;
   if (want < 2) return 1;
   int len = (int)((max_q_len + want - 1) / want);

@@ -38,18 +38,71 @@ __device__ __forceinline__ void ds_async(void* dst, const void* src, int bytes) 
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
 }
 
-// Lanes a column, float4 of it a lane, by the key's size.
-#define DS_BY_K(K, GO)          \
-  do {                          \
-    if ((K) <= 16) GO(4, 1);    \
-    else if ((K) <= 32) GO(4, 2);  \
-    else if ((K) <= 64) GO(4, 4);  \
-    else if ((K) <= 128) GO(4, 8); \
-    else if ((K) <= 256) GO(16, 4);  \
-    else GO(16, 8);             \
+// How the state lies over a warp: DS_LANES neighbouring lanes share C neighbouring columns, and
+// each holds KQ float4 of every one of them, entries 4 (lane + DS_LANES i) + {0..3}, so that a
+// float4 of k, q or a decay from shared memory serves C columns of a thread.  (A warp's 16-byte
+// read takes four cycles of shared memory, also where its lanes share addresses: with one column a
+// thread and four lanes a column those reads, and not the arithmetic, bounded the walks: 2,048
+// tokens of 16 heads of 64 x 128 took 330 us in the delta rule and 203 us in the linear
+// recurrence.)
+#define DS_LANES 8
+#define DS_GROUPS (DS_WARPS * (32 / DS_LANES))    // of columns, a block
+
+// float4 a lane, columns a thread, by the key's size
+#define DS_BY_K(K, GO)           \
+  do {                           \
+    if ((K) <= 32) GO(1, 4);     \
+    else if ((K) <= 64) GO(2, 4);   \
+    else if ((K) <= 128) GO(4, 4);  \
+    else if ((K) <= 256) GO(8, 2);  \
+    else GO(16, 1);              \
   } while (0)
 
-static inline int ds_cols(int K) { return DS_WARPS * (K <= 128 ? 8 : 2); }
+static inline int ds_cols(int K) { return DS_GROUPS * (K <= 128 ? 4 : K <= 256 ? 2 : 1); }
 static inline int ds_pitch(int K) {
-  return K <= 16 ? 16 : K <= 32 ? 32 : K <= 64 ? 64 : K <= 128 ? 128 : K <= 256 ? 256 : 512;
+  return K <= 32 ? 32 : K <= 64 ? 64 : K <= 128 ? 128 : K <= 256 ? 256 : 512;
+}
+// Blocks of a pass that an SM holds at once, by registers and shared memory.
+static inline int ds_resident(int K) { return K <= 64 ? 5 : K <= 256 ? 3 : 1; }
+
+// The sums of C columns over the DS_LANES lanes that share them; lane l of them gets column
+// ds_own<C>(l)'s.
+template <int C> __device__ __forceinline__ int ds_own(int l) {
+  return C == 4 ? (l >> 1) & 3 : C == 2 ? (l >> 2) & 1 : 0;
+}
+template <int C> __device__ __forceinline__ float ds_sum(const float* v, int l) {
+  float r;
+  if (C == 4) {
+    const bool up = l & 4, up2 = l & 2;
+    const float s0 = up ? v[0] : v[2], s1 = up ? v[1] : v[3];
+    const float r0 = (up ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, s0, 4);
+    const float r1 = (up ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, s1, 4);
+    r = (up2 ? r1 : r0) + __shfl_xor_sync(0xffffffffu, up2 ? r0 : r1, 2);
+  } else if (C == 2) {
+    const bool up = l & 4;
+    r = (up ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, up ? v[0] : v[1], 4);
+    r += __shfl_xor_sync(0xffffffffu, r, 2);
+  } else {
+    r = v[0] + __shfl_xor_sync(0xffffffffu, v[0], 4);
+    r += __shfl_xor_sync(0xffffffffu, r, 2);
+  }
+  return r + __shfl_xor_sync(0xffffffffu, r, 1);
+}
+// The other way round: every lane gets the C columns' values.
+template <int C> __device__ __forceinline__ void ds_share(float own, float* v, int l) {
+  if (C == 4) {
+    const float o = __shfl_xor_sync(0xffffffffu, own, 2);
+    const float p0 = l & 2 ? o : own, p1 = l & 2 ? own : o;
+    const float q0 = __shfl_xor_sync(0xffffffffu, p0, 4), q1 = __shfl_xor_sync(0xffffffffu, p1, 4);
+    v[0] = l & 4 ? q0 : p0;
+    v[1] = l & 4 ? q1 : p1;
+    v[2] = l & 4 ? p0 : q0;
+    v[3] = l & 4 ? p1 : q1;
+  } else if (C == 2) {
+    const float o = __shfl_xor_sync(0xffffffffu, own, 4);
+    v[0] = l & 4 ? o : own;
+    v[1] = l & 4 ? own : o;
+  } else {
+    v[0] = own;
+  }
 }

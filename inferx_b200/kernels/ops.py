@@ -2043,11 +2043,13 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: 
     return out
 
 
-# A sequence's tokens are walked in order by one block per (head, 32 value columns): a long
+# A sequence's tokens are walked in order by one block per (head, some value columns): a long
 # prompt alone leaves most of the GPU idle.  From RECURRENCE_SEGMENT_MIN tokens on, the
-# longest sequence of a step is cut into segments that are walked side by side (one pass
-# for the segments' own states, one that joins them and writes the outputs), as many as
-# fill the multiprocessors about once (RECURRENCE_BLOCKS), none shorter than 64 tokens.
+# longest sequence of a step is cut into segments that are walked side by side (a pass
+# for the segments' own states, one that joins them, one that writes the outputs), as many as
+# fill the multiprocessors about once, none shorter than 64 tokens.  The linear recurrence and
+# the delta rule decide beside their kernels; ``recurrence_segments`` (RECURRENCE_BLOCKS) is for
+# the state space where it is not chunked.
 RECURRENCE_SEGMENT_MIN = 128
 RECURRENCE_BLOCKS = 1024
 RECURRENCE_MAX_SEGMENTS = 64
