@@ -1,0 +1,64 @@
+"""Rules by which prompts take the forms made for them: what they promise the kernels, over shapes
+drawn at random (no device)."""
+import ctypes
+import random
+
+import pytest
+
+from inferx_b200.kernels import library, ops
+
+
+def test_widened_rows_hold_every_visible_key():
+    rng = random.Random(1)
+    taken = 0
+    for _ in range(3000):
+        S = rng.randint(1, 6)
+        q_lens = [rng.choice([2, 33, 64, 200, 1000, 3000]) for _ in range(S)]
+        starts = [rng.randint(0, 6000) for _ in range(S)]
+        window = rng.choice([0, 0, 1, 64, 100, 4096])
+        slack = rng.choice([0, 17, 4000])             # a recorded step's bound lies above
+        heads, rank = rng.choice([(8, 256), (16, 512), (32, 512), (128, 512)])
+        bound = max(a + n for a, n in zip(starts, q_lens)) + slack
+        rows = ops.widened_latent_rows(q_lens, bound, window, heads, rank, 64, 320,
+                                       mixed=rng.random() < 0.3)
+        if not rows:
+            continue
+        taken += 1
+        assert rows % 64 == 0 and S * rows * heads * 320 * 2 <= ops.WIDENED_MAX_BYTES
+        for n, a in zip(q_lens, starts):
+            base = max(0, a - window + 1) // 64 * 64 if window else 0
+            assert rows >= a + n - base
+    assert taken > 500
+
+
+def test_widened_form_is_for_many_queries():
+    rows = lambda q, kv, **k: ops.widened_latent_rows(q, kv, 0, 16, 512, 64, 320, **k)
+    assert rows([3000], 3000) and rows([1500], 9692) and rows([128], 640)
+    assert not rows([33], 8225) and not rows([2], 4098) and not rows([], 100)
+    assert not rows([3000], 3000000)                  # more than the buffer may take
+
+
+@pytest.mark.parametrize("M,N,K", [(17, 8, 8), (600, 2048, 5632), (40, 1024, 2048), (1, 1, 8),
+                                   (800, 22016, 4096), (65, 3, 4096), (333, 1000, 1032)])
+def test_fp32_runs_are_never_empty(M, N, K):
+    splits = library.load().ix_gemm_fp32_tc_splits(M, N, K)
+    steps = -(-K // 64)
+    per = -(-steps // splits)
+    assert 1 <= splits <= 16 and per * (splits - 1) < steps
+
+
+@pytest.mark.parametrize("entry", ["ix_delta_recurrence_segments", "ix_linear_recurrence_segments"])
+def test_segments_cover_the_longest_sequence(entry):
+    f = getattr(library.load(), entry)
+    rng = random.Random(2)
+    for _ in range(2000):
+        S, H = rng.randint(1, 40), rng.choice([1, 8, 16, 64])
+        K, V = rng.choice([7, 16, 64, 100, 128, 256, 512]), rng.choice([8, 64, 128, 333])
+        longest, most = rng.randint(1, 20000), rng.choice([2, 64])
+        seg = ctypes.c_int(-1)
+        n = f(S, H, K, V, longest, 128, most, ctypes.byref(seg))
+        if n == 1:
+            assert seg.value == 0
+            continue
+        assert longest >= 128 and 2 <= n <= most and seg.value >= 64 and seg.value % 16 == 0
+        assert (n - 1) * seg.value < longest <= n * seg.value
