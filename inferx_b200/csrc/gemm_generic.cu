@@ -10,9 +10,9 @@
 // silu(gate) * up, which is the reference's GroupedGemmBf16 + SiluMulFused
 // (src/backends/cuda/ops/moe.cu:324-392, src/backends/cuda/ops/layers.cu:512-529).
 //
-// This is the whole matrix path of the 32-bit mode (true fp32 FFMA, no reduced
-// precision mode) and the fallback of the bfloat16 mode for shapes the tensor
-// core kernels refuse.  Two kernels:
+// This is the matrix path of the 32-bit mode for few rows, grouped products and what
+// gemm_fp32_tc.cu refuses (fp32 FFMA, no reduced precision mode), and the fallback of the
+// bfloat16 mode for shapes the tensor core kernels refuse.  Two kernels:
 //
 // * tiles (many rows): a block computes BM x BN outputs (128 x 128, or 64 x 128 where
 //   a weight matrix meets few rows; half as many columns for the SwiGLU form, which
