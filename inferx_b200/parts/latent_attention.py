@@ -110,7 +110,7 @@ class LatentAttentionMixer:
         self.o_w = w[self._n("o")]
         applies = getattr(self.ctx.ops, "widened_latent_applies", None)
         self.kv_w = None
-        if applies is not None and self.in_w.is_cuda and applies(
+        if applies is not None and self.in_w.is_cuda and s.scale > 0 and applies(
                 self.in_w.dtype, s.dim, s.rot_dim, s.vdim, s.kv_rank,
                 (self.kv_off, self.gate_off, self.in_w.shape[0])):
             # one matrix from records to the keys of every head, then the values: the record's

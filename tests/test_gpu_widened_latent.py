@@ -184,3 +184,16 @@ def test_mixer_forms_agree(dim, rot, vdim, rank, heads, q_rank, own, gated, exac
     # the folded one shows here (two roundings of a quarter more each would still pass)
     assert off_w <= 1.25 * off_f and off_f < 0.02, (off_f, off_w)
     assert torch.equal(rec_f, rec_w)
+
+
+def test_a_scale_that_is_not_positive_keeps_the_folded_form():
+    from inferx_b200.parts.latent_attention import LatentAttentionMixer
+    from inferx_b200.parts.specs import LatentAttentionSpec
+    for scale, widened in ((0.1, True), (0.0, False), (-0.1, False)):
+        spec = LatentAttentionSpec(hidden=64, heads=2, dim=64, rot_dim=64, vdim=64, kv_rank=64,
+                                   scale=scale, window=0, position=None, latent_eps=1e-6)
+        mixer = LatentAttentionMixer(spec, SimpleNamespace(ops=_ops(), dtype=BF), "m")
+        mixer.bind({d.name: torch.ones(d.shape, device="cuda",
+                                       dtype=BF if len(d.shape) == 2 else torch.float32)
+                    for d in mixer.tensors()})
+        assert (mixer.kv_w is not None) == widened
