@@ -1671,9 +1671,11 @@ USE_WIDENED_LATENT = True
 def widened_latent_applies(dtype, dim: int, rot_dim: int, vdim: int, rank: int,
                            offsets: Sequence[int] = ()) -> bool:
     """Whether the widened form of latent attention takes these sizes: bf16, heads of the
-    kernel's widths, and records, products and column offsets in 16-byte chunks."""
-    return bool(USE_WIDENED_LATENT and dtype == torch.bfloat16 and rot_dim % 2 == 0
-                and rank % 8 == 0 and rot_dim % 8 == 0 and all(o % 8 == 0 for o in offsets)
+    kernel's widths, column offsets in 16-byte chunks, and records that the folded form attends
+    over on the tensor cores too.  Records of other sizes attend in the general form, whose
+    weights, keys and values stay in 32 bits."""
+    return bool(USE_WIDENED_LATENT and dtype == torch.bfloat16 and all(o % 8 == 0 for o in offsets)
+                and _lib().ix_latent_attention_mma_applies(rank, rot_dim)
                 and _lib().ix_widened_attention_applies(dim + rot_dim, vdim))
 
 

@@ -38,6 +38,19 @@ def test_widened_form_is_for_many_queries():
     assert not rows([3000], 3000000)                  # more than the buffer may take
 
 
+@pytest.mark.parametrize("dim,rot,vdim,rank,takes", [
+    (128, 64, 128, 512, True), (96, 32, 128, 256, True), (48, 16, 64, 64, True),
+    (128, 0, 128, 128, True),
+    # latents and rotated parts of the general form: it keeps what it computes in 32 bits
+    (128, 64, 128, 384, False), (128, 64, 128, 96, False), (128, 64, 128, 1024, False),
+    (120, 8, 128, 512, False), (104, 24, 64, 256, False),
+    (100, 64, 128, 512, False)])                      # no width of the kernel's
+def test_widened_form_leaves_the_general_forms_sizes_alone(dim, rot, vdim, rank, takes):
+    import torch
+    assert ops.widened_latent_applies(torch.bfloat16, dim, rot, vdim, rank, (512, 1024)) is takes
+    assert not ops.widened_latent_applies(torch.float32, dim, rot, vdim, rank, (512, 1024))
+
+
 @pytest.mark.parametrize("M,N,K", [(17, 8, 8), (600, 2048, 5632), (40, 1024, 2048), (1, 1, 8),
                                    (800, 22016, 4096), (65, 3, 4096), (333, 1000, 1032)])
 def test_fp32_runs_are_never_empty(M, N, K):
