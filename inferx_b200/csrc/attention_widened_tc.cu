@@ -11,24 +11,30 @@
 //                             cache slot, and the rotated parts of the queries turned in place
 //   ix_latent_collect         the records that the step's queries can see, out of the pages into
 //                             rows [sequence][position - base], zeros where there is none
-//   (the caller's product     rows x [K of every head | V of every head]; the key matrix has
-//    widens them)             identity columns that pass the rotated part on)
+//   (the caller's products    latents x key matrix in fp32, latents x value matrix)
+//   ix_latent_key_terms       the keys of every head, [plain | rotated part of the record], and
+//                             what bfloat16 leaves of the plain entries as a second term
 //   ix_widened_attention      this file's attention kernel
 //
+// The folded form keeps a record as it is and rounds the folded query; here the widened keys would
+// be rounded instead, and where attention is sharp that rounding weighs more than any other
+// (queries of four times unit size: 0.00623 with rounded keys against 0.00617 folded; eight times
+// 0.00817 against 0.00797).  So a key enters its product with the query as two bfloat16 terms,
+// 16 bits: 0.00553 and 0.00692, and less than the folded form's error at every sharpness.  A
+// softmax weight enters its product with the values as it does in the folded form, in one term or
+// (WT 2) in two, the second in the columns of the score buffer that the first leaves free.
+//
 // The attention kernel: a block owns two tiles of 128 queries of one sequence and head (a query
-// is a lane of tensor memory) and walks their keys in tiles of 64.  Warp 0 brings K and V tiles
-// with TMA into a ring of three stages that both query tiles read; one thread of warp 1 issues
-// the MMAs, S = Q K^T of tile j + 1 for both query tiles ahead of O += P V of tile j; warps 4-7
-// and 8-11 are the softmax of the two query tiles (a thread holds one query row), whose P goes
-// back into the columns of tensor memory that S came from.  What bounds a step of the walk is the
+// is a lane of tensor memory) and walks their keys in tiles of 64.  Warps 0 and 2 bring K and V
+// tiles with TMA into rings of two stages that both query tiles read (one warp for both would have
+// the next K wait for the V ahead of it, whose stage is freed a softmax later); one thread of warp
+// 1 issues the MMAs, S = Q K^T of tile j + 1 for both query tiles ahead of O += P V of tile j;
+// warps 4-7 and 8-11 are the softmax of the two query tiles (a thread holds one query row), whose P
+// goes back into the columns of tensor memory that S came from.  What bounds a step of the walk is the
 // latency of that chain (read S, mask, max, 64 exponentials, write P), so two independent query
 // tiles run on an SM: they hide each other's chain and halve what K and V tiles cost in L2
 // traffic.  Two blocks of one tile each, as in attention_prefill_tc.cu, do not fit: the keys'
 // 192 entries make Q and the ring 128 KB.  The running max is updated lazily, see there.
-//
-// Measured (B200, a whole mixer of 16 heads at a latent of 512 + 64, against the folded form):
-// 3,000 tokens 200 against 1,064 us, 1,500 tokens behind 2,048 190 against 967 us, 128 behind 512
-// 46 against 75 us.  Where the folded form stays ahead: WIDENED_RATES in kernels/ops.py.
 //
 // Every mbarrier wait is bounded; one that ran out records a code (31: copies, 32: MMA, 33:
 // softmax) in the caller's status word and the block runs to its end.
@@ -41,7 +47,7 @@
 #define WA_BM 128
 #define WA_BN 64
 #define WA_THREADS 384
-#define WA_STAGES 3
+#define WA_STAGES 2
 #define WA_RESCALE_STEP 8.0f   // log2 units
 
 enum { WA_ERR_COPY = 31, WA_ERR_MMA = 32, WA_ERR_SOFTMAX = 33, WA_ERR_ALIGN = 34 };
@@ -90,11 +96,9 @@ __device__ __forceinline__ int wa_base(int first_pos, int window) {
   return ix_first_key(first_pos, window, 0) & ~(WA_BN - 1);
 }
 
-// A softmax weight enters its product with the values as two bfloat16 terms (16 bits), the second
-// in the columns of the score buffer that the first leaves free: keys and values are rounded once
-// more than in the folded form, and 16-bit weights make up for it (a whole model against 64 bits:
-// 0.0092-0.0098 folded, 0.0099 with 8-bit weights here, 0.0090 with 16; 3.5 % of its time).
-template <int DK, int DV>
+// LP: 64-column panels of a head's second key terms in a row of kv (0: one term).  WT: bfloat16
+// terms of a softmax weight.
+template <int DK, int DV, int LP, int WT>
 __global__ void __launch_bounds__(WA_THREADS, 1)
 widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
                          const __grid_constant__ CUtensorMap map_kv,
@@ -104,7 +108,8 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
                          int* __restrict__ status) {
   constexpr int KP = DK / 64, VP = DV / 64;         // 64-column panels
   constexpr int Q_PANEL = WA_BM * 128, Q_BYTES = KP * Q_PANEL;
-  constexpr int PANEL = WA_BN * 128, K_TILE = KP * PANEL, V_TILE = VP * PANEL;
+  constexpr int PANEL = WA_BN * 128, V_TILE = VP * PANEL;
+  constexpr int K_LO = KP * PANEL, K_TILE = (KP + LP) * PANEL;   // second terms from K_LO on
   constexpr unsigned TMEM_COLS = 512;
   // O of the two query tiles from columns 0 and 128, S buffers of 64 columns from 256
   constexpr unsigned S_COL = 256;
@@ -143,6 +148,8 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
   const int kv_lo = ix_first_key(pos0, window, 0);
   const int kt0 = kv_lo & ~(WA_BN - 1);              // base is on a tile's edge too
   const int n_tiles = (pmax + 1 - kt0 + WA_BN - 1) / WA_BN;
+  // the first query tile of two ends its walk with its own last position
+  const int n_first = (min(pmax, pos0 + WA_BM - 1) + 1 - kt0 + WA_BN - 1) / WA_BN;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
   if ((smem_u32(smem) & 1023u) != 0) {
@@ -179,7 +186,7 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
   tc_fence_after();
   const unsigned tmem_base = bars->tmem_holder;
   volatile int* abortp = &bars->abort_flag;
-  int copied = 0;                                    // tiles whose copies were started (warp 0)
+  int copied = 0;                        // tiles whose copies this thread started (warps 0 and 2)
 
   if (warp == 0) {
     if (lane == 0) {
@@ -192,79 +199,105 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
       const int row0 = s * rows_per_seq + (kt0 - base);
       bool ok = true;
       for (int j = 0; j < n_tiles; ++j) {
-        const int st = j % WA_STAGES;
-        const unsigned par = ((j / WA_STAGES) & 1) ^ 1;
-        const int row = row0 + j * WA_BN;
-        ok = mbar_wait(&bars->k_empty[st], par, abortp);
+        const int st = j % WA_STAGES, row = row0 + j * WA_BN;
+        ok = mbar_wait(&bars->k_empty[st], ((j / WA_STAGES) & 1) ^ 1, abortp);
         if (!ok) break;
         mbar_expect_tx(&bars->k_full[st], K_TILE);
 #pragma unroll
         for (int p = 0; p < KP; ++p)
           tma_load_2d(Ks + st * K_TILE + p * PANEL, &map_kv, h * DK + p * 64, row,
                       &bars->k_full[st]);
+#pragma unroll
+        for (int p = 0; p < LP; ++p)
+          tma_load_2d(Ks + st * K_TILE + K_LO + p * PANEL, &map_kv,
+                      heads * DK + (h * LP + p) * 64, row, &bars->k_full[st]);
         copied = j + 1;
-        ok = mbar_wait(&bars->v_empty[st], par, abortp);
+      }
+      if (!ok && !*abortp) { atomicExch(status, WA_ERR_COPY); *abortp = 1; }
+    }
+  } else if (warp == 2) {
+    if (lane == 0) {
+      const int row0 = s * rows_per_seq + (kt0 - base);
+      bool ok = true;
+      for (int j = 0; j < n_tiles; ++j) {
+        const int st = j % WA_STAGES, row = row0 + j * WA_BN;
+        ok = mbar_wait(&bars->v_empty[st], ((j / WA_STAGES) & 1) ^ 1, abortp);
         if (!ok) break;
         mbar_expect_tx(&bars->v_full[st], V_TILE);
 #pragma unroll
         for (int p = 0; p < VP; ++p)
-          tma_load_2d(Vs + st * V_TILE + p * PANEL, &map_kv, heads * DK + h * DV + p * 64, row,
-                      &bars->v_full[st]);
+          tma_load_2d(Vs + st * V_TILE + p * PANEL, &map_kv,
+                      heads * (DK + LP * 64) + h * DV + p * 64, row, &bars->v_full[st]);
+        copied = j + 1;
       }
       if (!ok && !*abortp) { atomicExch(status, WA_ERR_COPY); *abortp = 1; }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      bool ok = mbar_wait(&bars->q_full, 0, abortp);
-      auto issue_s = [&](int j) {
-        const int st = j % WA_STAGES;
-        if (!mbar_wait(&bars->k_full[st], (j / WA_STAGES) & 1, abortp)) return false;
-        tc_fence_after();
-        for (int t = 0; t < halves; ++t) {
-          // the buffer's last reader, P V of tile j - 2, was issued before: the tensor pipe
-          // keeps the order
+    // The whole warp walks the tiles and one lane issues: where descriptors are the warp's and not a
+    // thread's they stay in uniform registers.  (One lane alone took some 130 cycles an MMA.)
+    bool ok = __all_sync(0xffffffffu, mbar_wait(&bars->q_full, 0, abortp));
+    // (a descriptor's low bits are the address in 16-byte units)
+    const unsigned long long q_desc = umma_desc(Qs), k_desc = umma_desc(Ks);
+    const unsigned long long v_desc = umma_desc_mn(Vs, PANEL, 1024);
+    auto issue_s = [&](int j) {
+      const int st = j % WA_STAGES;
+      if (!__all_sync(0xffffffffu, mbar_wait(&bars->k_full[st], (j / WA_STAGES) & 1, abortp)))
+        return false;
+      tc_fence_after();
+      const unsigned long long kd = k_desc + (unsigned)((st * K_TILE) >> 4);
+      for (int t = j < n_first ? 0 : 1; t < halves; ++t) {
+        // the buffer's last reader, P V of tile j - 2, was issued before: the tensor pipe
+        // keeps the order
+        const unsigned s_col = tmem_base + S_COL + (2 * t + (j & 1)) * WA_BN;
+        const unsigned long long qd = q_desc + (unsigned)((t * Q_BYTES) >> 4);
+        if (lane == 0) {
 #pragma unroll
-          for (int kk = 0; kk < DK / 16; ++kk) {
-            const unsigned long long qd =
-                umma_desc(Qs + t * Q_BYTES + (kk >> 2) * Q_PANEL) + 2 * (kk & 3);
-            const unsigned long long kd =
-                umma_desc(Ks + st * K_TILE + (kk >> 2) * PANEL) + 2 * (kk & 3);
-            tc_mma(tmem_base + S_COL + (2 * t + (j & 1)) * WA_BN, qd, kd, IDESC_S,
+          for (int kk = 0; kk < 4 * LP; ++kk)          // second terms first: the small ones
+            tc_mma(s_col, qd + (((kk >> 2) * Q_PANEL) >> 4) + 2 * (kk & 3),
+                   kd + ((K_LO + (kk >> 2) * PANEL) >> 4) + 2 * (kk & 3), IDESC_S,
                    kk > 0 ? 1u : 0u);
-          }
+#pragma unroll
+          for (int kk = 0; kk < 4 * KP; ++kk)
+            tc_mma(s_col, qd + (((kk >> 2) * Q_PANEL) >> 4) + 2 * (kk & 3),
+                   kd + (((kk >> 2) * PANEL) >> 4) + 2 * (kk & 3), IDESC_S,
+                   kk + LP > 0 ? 1u : 0u);
           tc_commit(&bars->s_full[t][j & 1]);
         }
-        tc_commit(&bars->k_empty[st]);
-        return true;
-      };
-      if (ok) ok = issue_s(0);
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        if (j + 1 < n_tiles) {
-          ok = issue_s(j + 1);
-          if (!ok) break;
-        }
-        const int st = j % WA_STAGES;
-        ok = mbar_wait(&bars->v_full[st], (j / WA_STAGES) & 1, abortp);
-        for (int t = 0; t < halves && ok; ++t) {
-          ok = mbar_wait(&bars->p_ready[t], j & 1, abortp);
-          if (!ok) break;
-          tc_fence_after();
-          const unsigned p_col = tmem_base + S_COL + (2 * t + (j & 1)) * WA_BN;
+        __syncwarp();
+      }
+      if (lane == 0) tc_commit(&bars->k_empty[st]);
+      __syncwarp();
+      return true;
+    };
+    if (ok) ok = issue_s(0);
+    for (int j = 0; j < n_tiles && ok; ++j) {
+      if (j + 1 < n_tiles) {
+        ok = issue_s(j + 1);
+        if (!ok) break;
+      }
+      const int st = j % WA_STAGES;
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars->v_full[st], (j / WA_STAGES) & 1, abortp));
+      const unsigned long long vd = v_desc + (unsigned)((st * V_TILE) >> 4);
+      for (int t = j < n_first ? 0 : 1; t < halves && ok; ++t) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&bars->p_ready[t], j & 1, abortp));
+        if (!ok) break;
+        tc_fence_after();
+        const unsigned p_col = tmem_base + S_COL + (2 * t + (j & 1)) * WA_BN;
+        if (lane == 0) {
 #pragma unroll
-          for (int k4 = 0; k4 < 2 * WA_BN / 16; ++k4) {
+          for (int k4 = 0; k4 < WT * WA_BN / 16; ++k4)
             // 16 keys: 8 columns of packed P (the second terms 32 columns on), two 8-key
             // groups of V's tile
-            const unsigned long long vd =
-                umma_desc_mn(Vs + st * V_TILE, PANEL, 1024) + 128 * (k4 & 3);
-            tc_mma_ts(tmem_base + t * 128, p_col + 8 * k4, vd, IDESC_PV,
+            tc_mma_ts(tmem_base + t * 128, p_col + 8 * k4, vd + 128 * (k4 & 3), IDESC_PV,
                       (j > 0 || k4 > 0) ? 1u : 0u);
-          }
           tc_commit(&bars->o_done[t]);
         }
-        if (ok) tc_commit(&bars->v_empty[st]);
+        __syncwarp();
       }
-      if (!ok && !*abortp) { atomicExch(status, WA_ERR_MMA); *abortp = 1; }
+      if (ok && lane == 0) tc_commit(&bars->v_empty[st]);
+      __syncwarp();
     }
+    if (!ok && lane == 0 && !*abortp) { atomicExch(status, WA_ERR_MMA); *abortp = 1; }
   } else if (warp >= 4 && ((warp - 4) >> 2) < halves) {
     // ---- softmax of query tile t ----
     const int t = (warp - 4) >> 2;
@@ -276,9 +309,10 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
     const int lo_r = ix_first_key(pos, window, 0);
     const unsigned lane_addr = tmem_base + ((unsigned)(quarter * 32) << 16);
     const unsigned o_addr = lane_addr + t * 128;
+    const int my_tiles = t == 0 ? n_first : n_tiles;
     float m_ref = -INFINITY, l_run = 0.f;
     bool ok = true;
-    for (int j = 0; j < n_tiles; ++j) {
+    for (int j = 0; j < my_tiles; ++j) {
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full[t][j & 1], (j >> 1) & 1, abortp));
       if (!ok) break;
       tc_fence_after();
@@ -311,7 +345,7 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
       }
       const float nbase = m_ref == -INFINITY ? 0.f : -m_ref;
       float pk[WA_BN / 2];
-      float pl[WA_BN / 2];           // what the rounding of each pair left over
+      float pl[WT == 2 ? WA_BN / 2 : 1];   // what the rounding of each pair left over
       float sum0 = 0.f, sum1 = 0.f, sum2 = 0.f, sum3 = 0.f;
 #pragma unroll
       for (int i = 0; i < WA_BN; i += 4) {
@@ -324,11 +358,13 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
         __nv_bfloat162 v = __floats2bfloat162_rn(p0, p1), v2 = __floats2bfloat162_rn(p2, p3);
         pk[i >> 1] = __uint_as_float(*reinterpret_cast<unsigned*>(&v));
         pk[(i >> 1) + 1] = __uint_as_float(*reinterpret_cast<unsigned*>(&v2));
-        const float2 f = __bfloat1622float2(v), f2 = __bfloat1622float2(v2);
-        __nv_bfloat162 r = __floats2bfloat162_rn(p0 - f.x, p1 - f.y);
-        __nv_bfloat162 r2 = __floats2bfloat162_rn(p2 - f2.x, p3 - f2.y);
-        pl[i >> 1] = __uint_as_float(*reinterpret_cast<unsigned*>(&r));
-        pl[(i >> 1) + 1] = __uint_as_float(*reinterpret_cast<unsigned*>(&r2));
+        if (WT == 2) {
+          const float2 f = __bfloat1622float2(v), f2 = __bfloat1622float2(v2);
+          __nv_bfloat162 r = __floats2bfloat162_rn(p0 - f.x, p1 - f.y);
+          __nv_bfloat162 r2 = __floats2bfloat162_rn(p2 - f2.x, p3 - f2.y);
+          pl[(i >> 1) * (WT - 1)] = __uint_as_float(*reinterpret_cast<unsigned*>(&r));
+          pl[((i >> 1) + 1) * (WT - 1)] = __uint_as_float(*reinterpret_cast<unsigned*>(&r2));
+        }
       }
       l_run += (sum0 + sum1) + (sum2 + sum3);
       if (j > 0) {
@@ -349,13 +385,13 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
         }
       }
       tc_st32(s_addr, pk);
-      tc_st32(s_addr + 32, pl);
+      if (WT == 2) tc_st32(s_addr + 32, pl);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars->p_ready[t]);
     }
     if (ok)
-      ok = __all_sync(0xffffffffu, mbar_wait(&bars->o_done[t], (n_tiles - 1) & 1, abortp));
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars->o_done[t], (my_tiles - 1) & 1, abortp));
     if (!ok) {
       if (lane == 0 && !*abortp) { atomicExch(status, WA_ERR_SOFTMAX); *abortp = 1; }
     } else {
@@ -398,13 +434,12 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
   }
   tc_fence_before();
   __syncthreads();
-  if (*abortp && tid == 0) {
+  if (*abortp && lane == 0 && (warp == 0 || warp == 2)) {
     // let copies in flight land before shared memory is given up
-    mbar_drain(&bars->q_full, 0);
-    for (int j = max(0, copied - WA_STAGES); j < copied; ++j) {
-      mbar_drain(&bars->k_full[j % WA_STAGES], (j / WA_STAGES) & 1);
-      mbar_drain(&bars->v_full[j % WA_STAGES], (j / WA_STAGES) & 1);
-    }
+    if (warp == 0) mbar_drain(&bars->q_full, 0);
+    unsigned long long* full = warp == 0 ? bars->k_full : bars->v_full;
+    for (int j = max(0, copied - WA_STAGES); j < copied; ++j)
+      mbar_drain(&full[j % WA_STAGES], (j / WA_STAGES) & 1);
   }
   __syncthreads();
   if (warp == 1) {
@@ -414,7 +449,7 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
   }
 }
 
-template <int DK, int DV>
+template <int DK, int DV, int LP, int WT>
 static int launch_widened(const void* q, long long q_ld, const void* kv, const int* cu_q,
                           const int* q_pos0, void* out, int T, int S, int heads, int rows_per_seq,
                           int window, float scale, const void* gate, long long gate_ld,
@@ -423,12 +458,13 @@ static int launch_widened(const void* q, long long q_ld, const void* kv, const i
   int rc = ix_tensor_map_bf16_2d(&map_q, q, T, (long long)heads * DK, 64, WA_BM, q_ld);
   if (rc != IX_OK) return rc;
   rc = ix_tensor_map_bf16_2d(&map_kv, kv, (long long)S * rows_per_seq,
-                             (long long)heads * (DK + DV), 64, WA_BN);
+                             (long long)heads * (DK + LP * 64 + DV), 64, WA_BN);
   if (rc != IX_OK) return rc;
-  int smem = 2 * WA_BM * DK * 2 + WA_STAGES * WA_BN * (DK + DV) * 2 + (int)sizeof(WaBars);
+  int smem = 2 * WA_BM * DK * 2 + WA_STAGES * WA_BN * (DK + LP * 64 + DV) * 2 +
+             (int)sizeof(WaBars);
   // more than half of an SM's: a second block could not have tensor memory anyway
   if (smem < 120 * 1024) smem = 120 * 1024;
-  auto kern = widened_attention_kernel<DK, DV>;
+  auto kern = widened_attention_kernel<DK, DV, LP, WT>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return (int)e;
   const int tiles = (T + 2 * WA_BM - 1) / (2 * WA_BM) + S;   // every sequence can add a part tile
@@ -443,35 +479,112 @@ IX_API int ix_widened_attention_applies(int dk, int dv) {
   return (dk == 64 || dk == 128 || dk == 192) && (dv == 64 || dv == 128);
 }
 
+// Entries a head's second key terms take in a row of kv, when its first `dn` of dk have some: dn
+// rounded up to what the kernel has a form for.
+IX_API int ix_widened_second(int dk, int dn) {
+  return dn <= 0 ? 0 : dk == 192 && dn <= 128 ? 128 : dk;
+}
+
 // q: rows of pitch q_ld (elements), head h's dk entries at h * dk, rotated parts turned.
-// kv: [S, rows_per_seq, heads * dk + heads * dv], row r of sequence s the key and value of
-// position base(s) + r (rows_per_seq a multiple of 64).  out: [T, heads * dv].  gate (null:
-// none): rows of pitch gate_ld, head h's entries at h * dv.
+// kv: [S, rows_per_seq, heads * dk + heads * lo + heads * dv], row r of sequence s the key, the
+// second terms of its first lo entries (ix_widened_second; 0: none) and the value of position
+// base(s) + r (rows_per_seq a multiple of 64).  weight_terms: 1 or 2.
+// out: [T, heads * dv].  gate (null: none): rows of pitch gate_ld, head h's entries at h * dv.
 IX_API int ix_widened_attention(const void* q, long long q_ld, const void* kv, const int* cu_q,
                                 const int* q_pos0, void* out, int T, int S, int heads, int dk,
-                                int dv, int rows_per_seq, int window, float scale,
-                                const void* gate, long long gate_ld, int* status,
+                                int dv, int lo, int weight_terms, int rows_per_seq, int window,
+                                float scale, const void* gate, long long gate_ld, int* status,
                                 cudaStream_t stream) {
   if (T <= 0 || S <= 0) return IX_OK;
   if (heads <= 0 || heads > 65535 || rows_per_seq <= 0 || rows_per_seq % WA_BN || window < 0 ||
       status == nullptr || !(scale > 0.f) || q_ld < (long long)heads * dk ||
-      (gate && gate_ld < (long long)heads * dv))
+      (gate && gate_ld < (long long)heads * dv) || weight_terms < 1 || weight_terms > 2)
     return IX_ERR_SIZE;
   if ((long long)S * rows_per_seq > 0x7fffffffLL) return IX_ERR_SIZE;
   if (((uintptr_t)q | (uintptr_t)kv | (uintptr_t)out | (uintptr_t)gate) & 15) return IX_ERR_ALIGN;
   if (q_ld % 8 || (gate && gate_ld % 8)) return IX_ERR_ALIGN;
-#define IX_WA(K, V)                                                                             \
-  if (dk == K && dv == V)                                                                       \
-    return launch_widened<K, V>(q, q_ld, kv, cu_q, q_pos0, out, T, S, heads, rows_per_seq,      \
-                                window, scale, gate, gate_ld, status, stream)
-  IX_WA(64, 64);
-  IX_WA(64, 128);
-  IX_WA(128, 64);
-  IX_WA(128, 128);
-  IX_WA(192, 64);
-  IX_WA(192, 128);
+#define IX_WA(K, V, L)                                                                          \
+  if (dk == K && dv == V && lo == L * 64) {                                                     \
+    auto go = weight_terms == 2 ? launch_widened<K, V, L, 2> : launch_widened<K, V, L, 1>;      \
+    return go(q, q_ld, kv, cu_q, q_pos0, out, T, S, heads, rows_per_seq, window, scale, gate,   \
+              gate_ld, status, stream);                                                         \
+  }
+#define IX_WA2(K, L)                                                                            \
+  IX_WA(K, 64, L)                                                                               \
+  IX_WA(K, 128, L)
+  IX_WA2(64, 0)
+  IX_WA2(64, 1)
+  IX_WA2(128, 0)
+  IX_WA2(128, 2)
+  IX_WA2(192, 0)
+  IX_WA2(192, 2)
+  IX_WA2(192, 3)
+#undef IX_WA2
 #undef IX_WA
   return IX_ERR_UNSUPPORTED;
+}
+
+// ---------------------------------------------------------------------------
+// Keys out of their fp32 product, in two bfloat16 terms: a block per row, a thread per 8 entries.
+// Bound by its bytes (fp32 in, 4 bytes out an entry).  Entries of a head in kv: dn plain and dr of
+// the record's rotated part, then at heads * (dn + dr) the second terms, `lo` a head (dn rounded up
+// to ix_widened_second, zeros from dn on).
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(512)
+latent_key_terms_kernel(const float* __restrict__ keys, const bf16* __restrict__ records,
+                        int rank, bf16* __restrict__ kv, long long kv_ld, int heads, int dn,
+                        int dr, int lo) {
+  IX_PDL_WAIT();
+  const size_t row = blockIdx.x;
+  const int per = (dn + dr) / 8, per_lo = lo / 8;
+  const float* k = keys + row * heads * dn;
+  const uint4* rot = reinterpret_cast<const uint4*>(records + row * (rank + dr) + rank);
+  uint4* hi_row = reinterpret_cast<uint4*>(kv + row * kv_ld);
+  uint4* lo_row = hi_row + (size_t)heads * per;
+  for (int i = threadIdx.x; i < heads * per; i += blockDim.x) {
+    const int h = i / per, c = i - h * per;
+    if (c * 8 >= dn) {
+      hi_row[i] = rot[c - dn / 8];
+      continue;
+    }
+    const float4* src = reinterpret_cast<const float4*>(k + (size_t)h * dn + c * 8);
+    const float4 a = src[0], b = src[1];
+    const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    unsigned t[4], u[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const __nv_bfloat162 p = __floats2bfloat162_rn(f[2 * e], f[2 * e + 1]);
+      t[e] = *reinterpret_cast<const unsigned*>(&p);
+      // an infinite first term is the whole of it (infinity minus infinity is not a number)
+      const float x = __low2float(p), y = __high2float(p);
+      const __nv_bfloat162 r = __floats2bfloat162_rn(isinf(x) ? 0.f : f[2 * e] - x,
+                                                     isinf(y) ? 0.f : f[2 * e + 1] - y);
+      u[e] = *reinterpret_cast<const unsigned*>(&r);
+    }
+    hi_row[i] = make_uint4(t[0], t[1], t[2], t[3]);
+    lo_row[h * per_lo + c] = make_uint4(u[0], u[1], u[2], u[3]);
+  }
+  const int pad = per_lo - dn / 8;
+  for (int i = threadIdx.x; i < heads * pad; i += blockDim.x)
+    lo_row[(i / pad) * per_lo + dn / 8 + i % pad] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// keys: [rows, heads * dn] fp32; records: [rows, rank + dr]; kv: rows of pitch kv_ld.
+IX_API int ix_latent_key_terms(const float* keys, const void* records, int rank, void* kv,
+                               long long kv_ld, long long rows, int heads, int dn, int dr, int lo,
+                               cudaStream_t stream) {
+  if (rows <= 0) return IX_OK;
+  if (rows > 0x7fffffffLL || heads <= 0 || dn <= 0 || dr < 0 || rank <= 0 ||
+      lo != ix_widened_second(dn + dr, dn) || kv_ld < (long long)heads * (dn + dr + lo))
+    return IX_ERR_SIZE;
+  if (dn % 8 || dr % 8 || rank % 8 || kv_ld % 8 ||
+      (((uintptr_t)keys | (uintptr_t)records | (uintptr_t)kv) & 15))
+    return IX_ERR_ALIGN;
+  const int chunks = heads * (dn + dr) / 8;
+  const int threads = chunks >= 512 ? 512 : (chunks + 31) / 32 * 32;
+  ix_launch(latent_key_terms_kernel, dim3((unsigned)rows), dim3(threads), 0, stream, keys,
+            (const bf16*)records, rank, (bf16*)kv, kv_ld, heads, dn, dr, lo);
+  return ix_launch_status();
 }
 
 // ---------------------------------------------------------------------------

@@ -1773,18 +1773,46 @@ def latent_collect(cache: torch.Tensor, block_table: torch.Tensor, q_pos0: torch
     return out
 
 
+def latent_widen(rec: torch.Tensor, rank: int, uk: torch.Tensor, uv: torch.Tensor, heads: int,
+                 dim: int):
+    """Keys and values of every head from the records ``rec`` [rows, rank + rot_dim]: rows of
+    [keys (dim plain, rot_dim rotated) of every head | second terms of the plain entries, padded
+    to ix_widened_second | values of every head].  ``uk`` [heads * dim, rank], ``uv``
+    [heads, vdim, rank].  A key is the bfloat16 rounding of its fp32 product, its second term the
+    rounding of what that leaves; values are rounded once."""
+    _chk("rec", rec, torch.bfloat16)
+    _chk("uk", uk, torch.bfloat16)
+    _chk("uv", uv, torch.bfloat16)
+    rows, rot = rec.shape[0], rec.shape[1] - rank
+    vdim = uv.shape[1]
+    if tuple(uk.shape) != (heads * dim, rank) or tuple(uv.shape) != (heads, vdim, rank) or rot < 0:
+        raise KernelError("latent_widen: records and matrices do not fit together")
+    lo = _lib().ix_widened_second(dim + rot, dim)
+    kv = torch.empty((rows, heads * (dim + rot + lo + vdim)), dtype=rec.dtype, device=rec.device)
+    latents = rec[:, :rank]
+    keys = torch.mm(latents, uk.t(), out_dtype=torch.float32)
+    torch.mm(latents, uv.view(heads * vdim, rank).t(), out=kv[:, heads * (dim + rot + lo):])
+    _check(_lib().ix_latent_key_terms(
+        _ptr(keys), _ptr(rec), rank, _ptr(kv), ctypes.c_longlong(kv.shape[1]),
+        ctypes.c_longlong(rows), heads, dim, rot, lo, _stream()), "latent_key_terms")
+    _count()
+    return kv
+
+
 def widened_attention(q: torch.Tensor, q_ld: int, kv: torch.Tensor, cu_q: torch.Tensor,
                       q_pos0: torch.Tensor, tokens: int, heads: int, dk: int, dv: int, rows: int,
-                      window: int, scale: float, gate: Optional[torch.Tensor] = None, gate_ld: int = 0,
-                      out: Optional[torch.Tensor] = None):
+                      window: int, scale: float, gate: Optional[torch.Tensor] = None,
+                      gate_ld: int = 0, out: Optional[torch.Tensor] = None, second: int = 0,
+                      fp32_weights: bool = True):
     """Causal attention of prompt portions over the step's own widened keys and values.
 
     ``q``: a one-dimensional view that starts at the first row's first query, rows of pitch
-    ``q_ld``, heads of ``dk`` beside each other; softmax weights keep 16 bits in their product
-    with the values; ``kv`` [S * rows, heads * (dk + dv)], the keys
-    of every head then the values, rows as ``latent_collect`` lays them out.  ``gate``: a
-    one-dimensional view likewise, whose sigmoid multiplies the result entry by entry.
-    Returns [tokens, heads * dv]."""
+    ``q_ld``, heads of ``dk`` beside each other.  ``kv`` [S * rows, heads * (dk + second terms +
+    dv)], the keys of every head, the second terms of their first ``second`` entries (0: none;
+    padded to ix_widened_second), then the values, rows as ``latent_collect`` lays them out.  With
+    ``fp32_weights`` a softmax weight keeps 16 bits in its product with the values (two bfloat16
+    terms) instead of 8.  ``gate``: a one-dimensional view likewise, whose sigmoid multiplies the
+    result entry by entry.  Returns [tokens, heads * dv]."""
     _chk("q", q, torch.bfloat16)
     _chk("kv", kv, torch.bfloat16)
     _chk("cu_q", cu_q, torch.int32)
@@ -1792,7 +1820,8 @@ def widened_attention(q: torch.Tensor, q_ld: int, kv: torch.Tensor, cu_q: torch.
     _chk("gate", gate, torch.bfloat16, optional=True)
     _chk("out", out, torch.bfloat16, optional=True)
     S = q_pos0.numel()
-    if cu_q.numel() != S + 1 or tuple(kv.shape) != (S * rows, heads * (dk + dv)):
+    lo = _lib().ix_widened_second(dk, second)
+    if cu_q.numel() != S + 1 or tuple(kv.shape) != (S * rows, heads * (dk + lo + dv)):
         raise KernelError("widened_attention: keys and values do not fit the sequences")
     for name, t, ld, width in (("q", q, q_ld, heads * dk), ("gate", gate, gate_ld, heads * dv)):
         if t is not None and (t.dim() != 1 or t.numel() < (tokens - 1) * ld + width):
@@ -1803,8 +1832,9 @@ def widened_attention(q: torch.Tensor, q_ld: int, kv: torch.Tensor, cu_q: torch.
         raise KernelError("widened_attention: out must be [tokens, heads * dv]")
     _check(_lib().ix_widened_attention(
         _ptr(q), ctypes.c_longlong(q_ld), _ptr(kv), _ptr(cu_q), _ptr(q_pos0), _ptr(out), tokens,
-        S, heads, dk, dv, rows, window, ctypes.c_float(scale), _ptr(gate), ctypes.c_longlong(gate_ld), _ptr(_tc_status(q.device)), _stream()),
-        "widened_attention")
+        S, heads, dk, dv, lo, 2 if fp32_weights else 1, rows, window,
+        ctypes.c_float(scale), _ptr(gate), ctypes.c_longlong(gate_ld),
+        _ptr(_tc_status(q.device)), _stream()), "widened_attention")
     _count()
     return out
 

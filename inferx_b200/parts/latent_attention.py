@@ -13,8 +13,8 @@ so attention runs with one shared key head of ``kv_rank + rot_dim`` entries whos
 are the latents themselves, and the head's output ``sum_j p_j c_j`` is widened by
 ``W_uv[h]`` afterwards.  That is the form for a few queries per sequence: a pair costs the
 latent's size instead of a head's.  Prompt portions of enough tokens (decided by the shape
-of the step) widen the records they can see once, with one product, and attend over keys
-and values of the head's own size.  Queries carry ``dim`` plain and ``rot_dim`` rotated entries per head;
+of the step) widen the records they can see once and attend over keys and values of the head's
+own size, keys in two bfloat16 terms.  Queries carry ``dim`` plain and ``rot_dim`` rotated entries per head;
 an optional sigmoid gate computed from the mixer's input multiplies the heads' outputs
 before the output projection.
 
@@ -113,15 +113,7 @@ class LatentAttentionMixer:
         if applies is not None and self.in_w.is_cuda and s.scale > 0 and applies(
                 self.in_w.dtype, s.dim, s.rot_dim, s.vdim, s.kv_rank,
                 (self.kv_off, self.gate_off, self.in_w.shape[0])):
-            # one matrix from records to the keys of every head, then the values: the record's
-            # rotated part passes through identity columns
-            kv = torch.zeros((s.heads * (s.dim + s.rot_dim + s.vdim), s.kv_rank + s.rot_dim),
-                             dtype=self.in_w.dtype, device=self.in_w.device)
-            keys = kv[:s.heads * (s.dim + s.rot_dim)].view(s.heads, s.dim + s.rot_dim, -1)
-            keys[:, :s.dim, :s.kv_rank] = w[self._n("uk")].view(s.heads, s.dim, s.kv_rank)
-            keys[:, s.dim:, s.kv_rank:] = torch.eye(s.rot_dim, dtype=kv.dtype, device=kv.device)
-            kv[s.heads * (s.dim + s.rot_dim):, :s.kv_rank] = w[self._n("uv")]
-            self.kv_w = kv
+            self.kv_w = w[self._n("uk")], self.uv
 
     def cache_needs(self):
         s = self.spec
@@ -227,11 +219,12 @@ class LatentAttentionMixer:
                                  s.dim, s.rot_dim, rot_dims, s.kv_rank, kept, slots)
         rec = ops.latent_collect(records, group.block_table[first:], step.q_pos0[first:],
                                  step.kv_len[first:], rows, s.window)
-        kv = ops.linear(rec, self.kv_w)
+        kv = ops.latent_widen(rec, s.kv_rank, *self.kv_w, s.heads, s.dim)
         ops.widened_attention(
             q, q_ld, kv, step.cu_q_prompt if first else step.cu_q, step.q_pos0[first:],
             x.shape[0] - first, s.heads, s.dim + s.rot_dim, s.vdim, rows, s.window, s.scale,
-            gate=flat[self.gate_off:] if s.output_gate else None, gate_ld=ld, out=out)
+            gate=flat[self.gate_off:] if s.output_gate else None, gate_ld=ld, out=out,
+            second=s.dim, fp32_weights=s.fp32_weights)
 
 
 register_part("mixer", "latent_attention", LatentAttentionMixer)

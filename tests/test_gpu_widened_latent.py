@@ -197,3 +197,108 @@ def test_a_scale_that_is_not_positive_keeps_the_folded_form():
                                        dtype=BF if len(d.shape) == 2 else torch.float32)
                     for d in mixer.tensors()})
         assert (mixer.kv_w is not None) == widened
+
+
+@pytest.mark.parametrize("H,dn,dr,rank,vdim", [(3, 48, 16, 64, 64), (16, 128, 64, 512, 128),
+                                               (5, 96, 32, 128, 128), (2, 64, 0, 64, 64)])
+def test_keys_are_two_terms(H, dn, dr, rank, vdim):
+    g = torch.Generator().manual_seed(dn + rank)
+    rows, lo = 130, {64: 64, 128: 128, 192: 128}[dn + dr]
+    rec = torch.randn(rows, rank + dr, generator=g).to(BF).cuda()
+    rec[100:] = 0                               # rows past a sequence's end
+    uk = (torch.randn(H * dn, rank, generator=g) * rank ** -0.5).to(BF).cuda()
+    uv = (torch.randn(H, vdim, rank, generator=g) * rank ** -0.5).to(BF).cuda()
+    kv = _ops().latent_widen(rec, rank, uk, uv, H, dn)
+    hi, second, v = kv.split([H * (dn + dr), H * lo, H * vdim], dim=1)
+    hi, second = hi.view(rows, H, dn + dr), second.view(rows, H, lo)
+    want = (rec[:, :rank].double() @ uk.double().T).view(rows, H, dn)
+    got = hi[..., :dn].double() + second[..., :dn].double()
+    # two roundings to 8 bits, and the product's own fp32 sums
+    assert float((got - want).norm() / want.norm()) <= 2.0 ** -16
+    assert float((hi[..., :dn].double() - want).norm() / want.norm()) >= 2.0 ** -11
+    assert torch.equal(hi[..., dn:], rec[:, None, rank:].expand(rows, H, dr))
+    assert not second[..., dn:].any() and not kv[100:].any()
+    want_v = (rec[:, :rank].double() @ uv.double().view(H * vdim, rank).T)
+    assert float((v.double() - want_v).norm() / want_v.norm()) <= 2.0 ** -8
+
+
+@pytest.mark.parametrize("dk,dv,second", [(64, 64, 48), (128, 128, 96), (128, 64, 128),
+                                          (192, 128, 128), (192, 64, 176)])
+@pytest.mark.parametrize("exact", [True, False])
+def test_second_key_terms_reach_the_scores(dk, dv, second, exact):
+    """Keys whose first terms are all alike: the second ones alone tell them apart."""
+    g = torch.Generator().manual_seed(dk + second)
+    H, q_lens, starts = 2, [3, 140, 300], [500, 70, 0]
+    st = _step(q_lens, starts)
+    rows, T, lo = 512, sum(q_lens), dk if dk < 192 or second > 128 else 128
+    q = (4.0 * torch.randn(T, H * dk, generator=g)).to(BF)
+    k1 = torch.ones(3 * rows, H, dk).to(BF)
+    k2 = torch.zeros(3 * rows, H, lo)
+    k2[..., :second] = torch.randn(3 * rows, H, second, generator=g)
+    v = torch.randn(3 * rows, H, dv, generator=g).to(BF)
+    k2 = k2.to(BF)
+    kv = torch.cat([t.reshape(3 * rows, -1) for t in (k1, k2, v)], 1).contiguous()
+    scale = 1.0 / math.sqrt(dk)
+    out = _ops().widened_attention(q.cuda().view(-1), H * dk, kv.cuda(), st.cu_q.cuda(),
+                                   st.q_pos0.cuda(), T, H, dk, dv, rows, 0, scale, second=second,
+                                   fp32_weights=exact).cpu().double().view(T, H, dv)
+    _ops().check_async_errors()
+    key = k1.double()
+    key[..., :second] += k2.double()[..., :second]
+    t0 = 0
+    for s, (n, a) in enumerate(zip(q_lens, starts)):
+        sl = slice(s * rows, s * rows + a + n)
+        sc = torch.einsum("thd,mhd->htm", q[t0:t0 + n].double().view(n, H, dk), key[sl]) * scale
+        seen = torch.arange(a + n)[None] <= torch.arange(a, a + n)[:, None]
+        want = torch.einsum("htm,mhd->thd", sc.masked_fill(~seen, -math.inf).softmax(-1),
+                            v.double()[sl])
+        # a result is a mean of values: rounded once, its weights to 8 or to 16 bits, its scores
+        # of some tens in fp32
+        most = float(v.double().abs().max())
+        bound = most * (2.0 ** -9 + 2.0 ** (-16 if exact else -8) + 2.0 ** -15)
+        assert float((out[t0:t0 + n] - want).abs().max()) <= bound
+        t0 += n
+
+
+@pytest.mark.parametrize("heads,dim,rot,rank,q_rank,gated,exact", [
+    (4, 128, 64, 512, 0, False, False), (4, 128, 64, 512, 96, False, True),
+    (8, 96, 32, 256, 0, True, False)])
+@pytest.mark.parametrize("sharp", [1.0, 4.0, 8.0])
+@pytest.mark.parametrize("n,before", [(70, 0), (400, 0), (90, 700)])
+def test_widened_is_no_further_from_exact_than_folded(heads, dim, rot, rank, q_rank, gated, exact,
+                                                      sharp, n, before):
+    """However decisive the scores are: rounded keys would weigh most where they are."""
+    from inferx_b200.parts.latent_attention import LatentAttentionMixer
+    from inferx_b200.parts.specs import LatentAttentionSpec
+    ops = _ops()
+    hidden, page, L = 256, 16, n + before
+    spec = LatentAttentionSpec(hidden=hidden, heads=heads, dim=dim, rot_dim=rot, vdim=128,
+                               kv_rank=rank, scale=sharp / math.sqrt(dim + rot), window=0,
+                               position=None, latent_eps=1e-6, output_gate=gated, q_rank=q_rank,
+                               own_records=True, fp32_weights=exact)
+    st = _cuda(_step([n], [before]))
+    pages = -(-L // page)
+    st.groups = [SimpleNamespace(
+        block_table=torch.arange(pages, dtype=torch.int32).view(1, -1).cuda(),
+        slots=torch.arange(before, L, dtype=torch.int32).cuda())]
+    g = torch.Generator().manual_seed(rank + n)
+    x = torch.randn(n, hidden, generator=g).to(BF).cuda()
+    cache = torch.randn(pages, 1, page, rank + rot, generator=g).to(BF).cuda()
+
+    def run(dtype, rows):
+        mixer = LatentAttentionMixer(spec, SimpleNamespace(ops=ops, dtype=dtype), "m")
+        gw = torch.Generator().manual_seed(5)
+        w = {d.name: (torch.randn(d.shape, generator=gw) * d.shape[-1] ** -0.5 if len(d.shape) == 2
+                      else 1 + 0.1 * torch.randn(d.shape, generator=gw)) for d in mixer.tensors()}
+        mixer.bind({k: (v.to(BF).to(dtype) if v.dim() == 2 else v).cuda() for k, v in w.items()})
+        before_rule, ops.widened_latent_rows = ops.widened_latent_rows, lambda *a, **k: rows
+        try:
+            return mixer.forward(x.to(dtype), st, SimpleNamespace(
+                group=0, pages={"latent": cache.to(dtype)}, writes=True)).double()
+        finally:
+            ops.widened_latent_rows = before_rule
+
+    want = run(torch.float32, 0)
+    off = [float((run(BF, rows) - want).norm() / want.norm()) for rows in (0, -(-L // 64) * 64)]
+    ops.check_async_errors()
+    assert off[1] <= off[0], off
