@@ -34,7 +34,8 @@
 // latency of that chain (read S, mask, max, 64 exponentials, write P), so two independent query
 // tiles run on an SM: they hide each other's chain and halve what K and V tiles cost in L2
 // traffic.  Two blocks of one tile each, as in attention_prefill_tc.cu, do not fit: the keys'
-// 192 entries make Q and the ring 128 KB.  The running max is updated lazily, see there.
+// 192 entries make Q and the ring 128 KB.  The running max is updated lazily, see there; a row
+// is rescaled by its own scores alone, so what it computes does not depend on its neighbours.
 //
 // Every mbarrier wait is bounded; one that ran out records a code (31: copies, 32: MMA, 33:
 // softmax) in the caller's status word and the block runs to its end.
@@ -338,8 +339,8 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
       const bool grow = m_new > m_ref + WA_RESCALE_STEP || (m_ref == -INFINITY && m_new > m_ref);
       const bool rescale = __any_sync(0xffffffffu, grow);
       float corr = 1.f;
-      if (rescale) {
-        corr = m_new == -INFINITY ? 1.f : wa_exp2(m_ref - m_new);
+      if (grow) {
+        corr = wa_exp2(m_ref - m_new);
         m_ref = m_new;
         l_run *= corr;
       }

@@ -302,3 +302,29 @@ def test_widened_is_no_further_from_exact_than_folded(heads, dim, rot, rank, q_r
     off = [float((run(BF, rows) - want).norm() / want.norm()) for rows in (0, -(-L // 64) * 64)]
     ops.check_async_errors()
     assert off[1] <= off[0], off
+
+
+@pytest.mark.parametrize("window", [0, 90])
+def test_a_row_does_not_depend_on_its_neighbours(window):
+    """The same query in another company, and in a portion that begins elsewhere: the same bits."""
+    g = torch.Generator().manual_seed(window)
+    H, dk, dv, n, rows = 2, 128, 128, 300, 320
+    q = torch.randn(n, H * dk, generator=g).to(BF)
+    kv = torch.randn(rows, H * (dk + dv), generator=g).to(BF)
+
+    def run(q, start):
+        st = _step([q.shape[0]], [start])
+        base = max(0, start - window + 1) // 64 * 64 if window else 0
+        own = torch.zeros_like(kv)
+        own[:rows - base] = kv[base:]
+        out = _ops().widened_attention(q.cuda().view(-1), H * dk, own.cuda(), st.cu_q.cuda(),
+                                       st.q_pos0.cuda(), q.shape[0], H, dk, dv, rows, window, 0.3)
+        _ops().check_async_errors()
+        return out.cpu()
+
+    whole = run(q, 0)
+    loud = q.clone()
+    loud[::2] *= 30.0                            # every other row's maxima grow all along its keys
+    assert torch.equal(run(loud, 0)[1::2], whole[1::2])
+    for cut in (1, 64, 129, 200):
+        assert torch.equal(run(q[cut:].contiguous(), cut), whole[cut:])
