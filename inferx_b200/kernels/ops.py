@@ -1679,44 +1679,103 @@ def widened_latent_applies(dtype, dim: int, rot_dim: int, vdim: int, rank: int,
                 and _lib().ix_widened_attention_applies(dim + rot_dim, vdim))
 
 
-# The widened rows of a step live in one buffer; beyond this the folded form runs.
-WIDENED_MAX_BYTES = 1 << 30
-# What either form takes, in microseconds, for the choice between them: operations a
-# microsecond of the folded kernel; microseconds that the folded form's two more products take
-# at least; microseconds a 64-key tile of the widened kernel's walk; operations a microsecond of
-# the widening product.  Fitted to whole mixers at a latent of 512 + 64 (folded / widened, us):
-# 16 heads, n new tokens behind b: (33, 0) 37 / 28, (33, 512) 50 / 42, (33, 2048) 63 / 77,
-# (64, 8192) 157 / 236, (128, 2048) 114 / 83, (128, 8192) 250 / 237, (3000, 0) 1064 / 200,
-# (3000, 8192) 5916 / 703; 32 heads: (33, 2048) 103 / 113, (64, 2048) 132 / 114, (3000, 0)
-# 2010 / 398; 8 heads, latent 256 + 32: (128, 512) 42 / 36, (256, 2048) 75 / 88, (700, 2048)
-# 154 / 100.
-WIDENED_RATES = (165e6, 12.0, 1.2, 800e6)
+# The widened rows of a step (keys, their second terms and values) live in one buffer; beyond this
+# size the folded form runs.
+WIDENED_MAX_BYTES = 3 << 29
+# Keys pass through fp32 in runs of rows of at most this size, which stay in L2 on the way.
+WIDENED_FP32_BYTES = 64 << 20
+# What either form takes, for the choice between them, fitted to 150 recorded steps at 8, 16 and 32
+# heads, 33 to 700 new tokens behind 0 to 16,380, with and without sequences that decode.  Folded:
+# microseconds a 32-key tile of a block by the latent's size, blocks an SM; microseconds a token
+# and 1,024 heads x latent entries / 512, and a round of blocks whose keys are cut (they write and
+# merge their partial sums).  Widened: microseconds of its further launches, and where single
+# tokens go first; bytes a microsecond of the widening; microseconds a 64-key tile of the walk
+# with one and with two query tiles.
+# Both forms measured (folded / widened, us, whole mixers in recorded steps whose bound is the next
+# power of two), n new tokens behind b.  16 heads, latent 512, less what both share: (128, 512) 12
+# slower folded, (128, 2020) 42 faster, (128, 8192) 123 faster, (256, 2300) 29 slower, (700, 0) 56
+# slower, (700, 8192) 1,215 slower.  128 heads: (128, 512) 187 / 138, (256, 2300) 1,064 / 387.
+# 16 heads, latent 128: (128, 2300) 69 / 116, (256, 8192) 349 / 470, (700, 2300) 256 / 179.  Over
+# all of them no widened step is slower than folded; folded ones are up to 12 % slower than they
+# could be at a latent of 512, up to 36 % at one of 64.
+LATENT_FOLDED_US = {64: (1.5, 6), 128: (2.3, 4), 256: (3.3, 2), 512: (2.1, 1)}
+LATENT_FOLDED_TOKEN_US, LATENT_FOLDED_ROUND_US = 2.05, 9.2
+WIDENED_STEP_US, WIDENED_MIXED_US, WIDENED_BYTES_US = 12.1, 17.0, 5.1e6
+WIDENED_TILE_US = (1.32, 2.4)
+
+
+def _latent_forms_us(q_lens, own, span: int, rows: int, window: int, heads: int, rank: int,
+                     rot_dim: int, dim: int, vdim: int, mixed: bool, fp32_weights: bool):
+    """(folded, widened) microseconds for portions of ``q_lens`` new tokens of which portion s
+    sees at least ``own[s]`` keys; ``span``, ``rows``: what the launches are sized for."""
+    lib = _lib()
+    per_tile = lib.ix_latent_attention_mma_tokens_per_tile(heads, 64)
+    tiles = [-(-n // per_tile) * -(-heads // 64) for n in q_lens]
+    ct = ctypes.c_int(0)
+    lib.ix_latent_attention_mma_chunks(sum(tiles), span, ctypes.byref(ct))
+    tile_us, resident = LATENT_FOLDED_US.get(rank, LATENT_FOLDED_US[512])
+    slots, work, longest, blocks, walk, sweep = 148 * resident, 0.0, 0.0, 0.0, 0.0, 0.0
+    for n, t, o in zip(q_lens, tiles, own):
+        mean = o - 0.5 * n
+        if window > 0:
+            mean, o = min(mean, window), min(o, window + n)
+        keys = o / 32.0 + 1.0
+        work += t * (mean / 32.0 + 1.0)
+        longest = max(longest, min(ct.value, keys) if ct.value else keys)
+        blocks += t * (-(-keys // ct.value) if ct.value else 1)
+        one, two = WIDENED_TILE_US
+        walk = max(walk, o / 64.0 * (one if n <= 128 else two))
+        for first in range(0, n, 256):
+            sweep += (one if n - first <= 128 else two) * min(o, o - n + first + 256) / 64.0
+    folded = tile_us * max(longest, work / slots + 0.5 * longest)
+    folded += LATENT_FOLDED_TOKEN_US * 1e-3 * sum(q_lens) * heads * rank / 512.0
+    folded += LATENT_FOLDED_ROUND_US * rank / 512.0 * (-(-blocks // slots) - (0 if ct.value else 1))
+    wide = dim + rot_dim + lib.ix_widened_second(dim + rot_dim, dim) + vdim
+    widened = WIDENED_STEP_US + (WIDENED_MIXED_US if mixed else 0.0)
+    widened += len(q_lens) * rows * (heads * (8 * dim + 2 * wide) + 4 * (rank + rot_dim)) \
+        / WIDENED_BYTES_US
+    widened += max(walk, heads * sweep / 148.0) * (1.13 if fp32_weights else 1.0) \
+        * (0.7 + 0.3 * wide / 448.0)
+    return folded, widened
 
 
 def widened_latent_rows(q_lens: Sequence[int], max_kv_len: int, window: int, heads: int,
-                        rank: int, rot_dim: int, width: int, mixed: bool = False) -> int:
+                        rank: int, rot_dim: int, width: int, mixed: bool = False, vdim: int = 128,
+                        fp32_weights: bool = False, kv_lens: Optional[Sequence[int]] = None,
+                        bound: bool = False):
     """Rows a sequence's collected records take when these portions (``q_lens`` new tokens
     each, at most ``max_kv_len`` with what the cache holds) should attend over widened keys
     and values, 0 when the folded form is the cheaper one.  Depends on the step's shape
-    only.  ``width``: key and value entries of a head together.  ``mixed``: ``max_kv_len``
-    covers other sequences too, so that half of it is taken for the portions' own."""
+    only.  ``width``: key and value entries of a head together, ``vdim`` of them the value's.
+    ``mixed``: single tokens run beside the portions.
+
+    The widened form pays for ``max_kv_len`` rows a portion, the folded one for the keys that
+    are there.  Those are ``kv_lens`` where the caller knows them.  Where ``max_kv_len`` is a
+    recorded step's bound, a table width rounded up to a power of two, one sequence holds at least
+    half of it (any of them; a decoding one where there are some) and the others their new
+    tokens; otherwise one holds all of it.  Both forms are charged for that least, at which the
+    folded form is at its best."""
     if not q_lens:
         return 0
     rows = int(max_kv_len)
     if window > 0:
         rows = min(rows, window + max(q_lens) + 63)
     rows = -(-rows // 64) * 64
-    S, tokens = len(q_lens), sum(q_lens)
-    if S * rows * heads * width * 2 > WIDENED_MAX_BYTES:
+    S, dim = len(q_lens), width - vdim - rot_dim
+    second = _lib().ix_widened_second(dim + rot_dim, dim)
+    if S * rows * heads * 2 * (width + second) > WIDENED_MAX_BYTES:
         return 0
-    folded_rate, products_us, walk_us, widen_rate = WIDENED_RATES
-    own = 0.5 * rows if mixed else float(rows)
-    pairs = tokens * max(own - 0.5 * tokens / S, 0.5 * own)
-    folded = products_us + pairs * heads * 2.0 * (2 * rank + rot_dim) / folded_rate
-    items = heads * sum(-(-n // 256) for n in q_lens)     # blocks of the walk, one an SM
-    walk = max(1.0, 0.75 * items / 148.0) * (own / 64.0) * walk_us
-    widen = S * rows * heads * width * 2.0 * (rank + rot_dim) / widen_rate
-    return rows if walk + widen < folded else 0
+    if kv_lens is not None:
+        own = [int(n) for n in kv_lens]
+    else:
+        own = [int(n) for n in q_lens]
+        if not mixed:
+            some = own.index(min(own))
+            own[some] = max(own[some], max_kv_len // 2 + 1 if bound else max_kv_len)
+    span = min(int(max_kv_len), window + max(q_lens)) if window > 0 else int(max_kv_len)
+    folded, widened = _latent_forms_us(q_lens, own, span, rows, window, heads, rank, rot_dim, dim,
+                                       vdim, mixed, fp32_weights)
+    return rows if widened < folded else 0
 
 
 def latent_front_inplace(q: Optional[torch.Tensor], q_ld: int, kv: Optional[torch.Tensor],
@@ -1789,13 +1848,15 @@ def latent_widen(rec: torch.Tensor, rank: int, uk: torch.Tensor, uv: torch.Tenso
         raise KernelError("latent_widen: records and matrices do not fit together")
     lo = _lib().ix_widened_second(dim + rot, dim)
     kv = torch.empty((rows, heads * (dim + rot + lo + vdim)), dtype=rec.dtype, device=rec.device)
-    latents = rec[:, :rank]
-    keys = torch.mm(latents, uk.t(), out_dtype=torch.float32)
-    torch.mm(latents, uv.view(heads * vdim, rank).t(), out=kv[:, heads * (dim + rot + lo):])
-    _check(_lib().ix_latent_key_terms(
-        _ptr(keys), _ptr(rec), rank, _ptr(kv), ctypes.c_longlong(kv.shape[1]),
-        ctypes.c_longlong(rows), heads, dim, rot, lo, _stream()), "latent_key_terms")
-    _count()
+    torch.mm(rec[:, :rank], uv.view(heads * vdim, rank).t(), out=kv[:, heads * (dim + rot + lo):])
+    run = max(256, WIDENED_FP32_BYTES // (heads * dim * 4) // 64 * 64)
+    for r in range(0, rows, run):
+        some = rec[r:r + run]
+        keys = torch.mm(some[:, :rank], uk.t(), out_dtype=torch.float32)
+        _check(_lib().ix_latent_key_terms(
+            _ptr(keys), _ptr(some), rank, _ptr(kv[r:]), ctypes.c_longlong(kv.shape[1]),
+            ctypes.c_longlong(some.shape[0]), heads, dim, rot, lo, _stream()), "latent_key_terms")
+        _count()
     return kv
 
 

@@ -156,9 +156,12 @@ class LatentAttentionMixer:
         alone, rows = T, 0
         if self.kv_w is not None and not step.all_decode:
             nd = step.num_decode_seqs
-            rows = ops.widened_latent_rows(step.q_lens[nd:], step.max_kv_len, s.window, s.heads,
-                                           s.kv_rank, s.rot_dim, s.dim + s.rot_dim + s.vdim,
-                                           mixed=nd > 0)
+            kv_lens = getattr(step, "kv_lens", None)
+            rows = ops.widened_latent_rows(
+                step.q_lens[nd:], step.max_kv_len, s.window, s.heads, s.kv_rank, s.rot_dim,
+                s.dim + s.rot_dim + s.vdim, mixed=nd > 0, vdim=s.vdim,
+                fp32_weights=s.fp32_weights, kv_lens=kv_lens[nd:] if kv_lens else None,
+                bound=getattr(step, "captured", False))
             if rows:
                 alone = nd
         if alone == T:

@@ -38,6 +38,30 @@ def test_widened_form_is_for_many_queries():
     assert not rows([3000], 3000000)                  # more than the buffer may take
 
 
+@pytest.mark.parametrize("new,before,bound,mixed,widened", [
+    # a recorded step's bound is a table width rounded up to a power of two: just above an edge the
+    # folded form walks half of it, while the widened form pays for all of it
+    (128, 1000, 2048, False, False), (128, 2020, 4096, False, False),
+    (128, 4000, 8192, False, False), (128, 8192, 16384, False, False),
+    (128, 16380, 32768, False, False), (64, 4200, 8192, False, False),
+    (256, 2020, 4096, False, False), (256, 8192, 16384, False, False),
+    # the bound is a decoding sequence's
+    (256, 1000, 2048, True, False), (128, 0, 4096, True, False), (64, 0, 8192, True, False),
+    # and where the widened form is far ahead it stays
+    (700, 0, 1024, False, True), (700, 2020, 4096, False, True), (700, 16380, 32768, False, True),
+    (3000, 0, 4096, False, True), (1024, 8192, 16384, False, True)])
+def test_a_bound_is_not_taken_for_a_length(new, before, bound, mixed, widened):
+    """16 heads of 128 + 64 over a latent of 512, measured in recorded steps both ways."""
+    assert new + before <= bound
+    rows = ops.widened_latent_rows([new], bound, 0, 16, 512, 64, 320, mixed=mixed, bound=True)
+    assert rows == (bound if widened else 0)
+
+
+def test_exact_lengths_decide_where_they_are_known():
+    rows = lambda own: ops.widened_latent_rows([200, 200], 8192, 0, 16, 512, 64, 320, kv_lens=own)
+    assert rows([8192, 8192]) and not rows([8192, 200])
+
+
 @pytest.mark.parametrize("dim,rot,vdim,rank,takes", [
     (128, 64, 128, 512, True), (96, 32, 128, 256, True), (48, 16, 64, 64, True),
     (128, 0, 128, 128, True),
