@@ -2314,14 +2314,16 @@ def ssd_recurrence(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tenso
         raise KernelError("ssd_recurrence: inputs and state do not fit together")
     out = torch.empty((T, heads * vdim), dtype=torch.float32, device=xbc.device)
     walked, longest = step.num_seqs, int(getattr(step, "max_q_len", 0) or T)
-    if _ssd_in_chunks(xbc, ld, state, longest, nstate, vdim):
+    singles = int(getattr(step, "num_decode_seqs", 0) or 0)
+    if _ssd_in_chunks(xbc, ld, state, longest, nstate, vdim) and _ssd_chunks_pay(
+            T - singles, step.num_seqs - singles, heads, nstate, vdim,
+            getattr(step, "q_lens", None) and step.q_lens[singles:]):
         # single tokens come first in a batch: they are walked, the sequences after them chunked
-        walked = int(getattr(step, "num_decode_seqs", 0) or 0)
+        walked = singles
         tokens, S = T - walked, step.num_seqs
-        size = _lib().ix_ssd_chunks_scratch_floats
-        size.restype = ctypes.c_longlong
-        scratch = torch.empty((size(tokens, S - walked, heads, nstate, vdim),),
-                              dtype=torch.float32, device=xbc.device)
+        scratch = torch.empty(
+            (ssd_chunks_scratch_bytes(tokens, S - walked, heads, nstate, vdim) // 4,),
+            dtype=torch.float32, device=xbc.device)
         _check(_lib().ix_ssd_chunks(
             _ptr(xbc), ctypes.c_longlong(ld), _ptr(dt_raw), ctypes.c_longlong(ld_dt),
             _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), _ptr(step.cu_q),
@@ -2349,6 +2351,29 @@ USE_SSD_CHUNKS = True
 # bfloat16 portions from this many tokens on run in chunks on the tensor cores (walk / chunks at
 # 32 heads of 128 x 64, us: 33 tokens 19 / 23, 64 31 / 25, 256 67 / 27, 2,048 441 / 92).
 SSD_CHUNK_MIN_TOKENS = 64
+
+
+# A chunk's state goes through scratch however few tokens it has: a step of many short portions
+# beside a long one is walked (64 heads; chunks / walk, us: 64 tokens and 32 portions of 8 227 / 113,
+# 256 and 128 of 8 946 / 466, 64 and 32 of 32 245 / 313, 32 portions of 64 265 / 575).
+SSD_TOKENS_A_CHUNK = 24
+SSD_MAX_SCRATCH_BYTES = 1 << 30
+
+
+def _ssd_chunks_pay(tokens: int, seqs: int, heads: int, nstate: int, vdim: int,
+                    q_lens: Optional[Sequence[int]] = None) -> bool:
+    """Whether ``seqs`` portions of ``tokens`` together are for the chunked form: chunks filled
+    well enough, a grid that holds heads x portions, scratch of a bounded size."""
+    chunks = sum(-(-n // 64) for n in q_lens) if q_lens else tokens // 64 + seqs
+    return (heads * seqs <= 65535 and tokens >= SSD_TOKENS_A_CHUNK * chunks
+            and ssd_chunks_scratch_bytes(tokens, seqs, heads, nstate, vdim)
+            <= SSD_MAX_SCRATCH_BYTES)
+
+
+def ssd_chunks_scratch_bytes(tokens: int, seqs: int, heads: int, nstate: int, vdim: int) -> int:
+    size = _lib().ix_ssd_chunks_scratch_floats
+    size.restype = ctypes.c_longlong
+    return 4 * size(tokens, seqs, heads, nstate, vdim)
 
 
 def _ssd_in_chunks(xbc, ld: int, state, longest: int, nstate: int, vdim: int) -> bool:

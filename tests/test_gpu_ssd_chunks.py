@@ -87,3 +87,27 @@ def test_decays_of_zero_and_infinite_rates():
         ops.USE_SSD_CHUNKS = True
     torch.testing.assert_close(got, ref, rtol=1e-5, atol=1e-5)
     torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("H,q_lens", [(2048, [2] * 31 + [64]), (2, [64] + [8] * 40)])
+def test_steps_that_are_left_to_the_walk(H, q_lens):
+    """Heads x portions beyond one dimension of a grid; portions of a few tokens each."""
+    ops = _ops()
+    V = N = 8
+    g = torch.Generator(device="cuda").manual_seed(H)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    S, T = len(q_lens), sum(q_lens)
+    step = _cuda(_step(q_lens, [5] * S))
+    xbc, dt = rnd(T, H * V + 2 * N).bfloat16(), rnd(T, H).bfloat16()
+    bias, a_log, d = rnd(H) - 2.0, 0.5 * rnd(H), rnd(H)
+    state = rnd(S, H, N, V)
+    before = ops.LAUNCHES[0]
+    got = state.clone()
+    out = ops.ssd_recurrence(xbc, dt, bias, a_log, d, got, step, H, V, N, 1)
+    assert ops.LAUNCHES[0] == before + 1                  # one pass: the walk
+    ops.USE_SSD_CHUNKS = False
+    try:
+        want = ops.ssd_recurrence(xbc, dt, bias, a_log, d, state, step, H, V, N, 1)
+    finally:
+        ops.USE_SSD_CHUNKS = True
+    assert torch.equal(out, want) and torch.equal(got, state)

@@ -62,6 +62,28 @@ def test_exact_lengths_decide_where_they_are_known():
     assert rows([8192, 8192]) and not rows([8192, 200])
 
 
+def test_chunked_state_space_leaves_what_it_cannot_hold_to_the_walk():
+    pay = lambda q, heads=64, K=128, V=64: ops._ssd_chunks_pay(sum(q), len(q), heads, K, V, q)
+    assert pay([64]) and pay([2048]) and pay([65, 128]) and pay([129, 2, 15], 4) and pay([64] * 100)
+    # heads x portions beyond a grid's 65,535
+    assert pay([64] * 511, 128, 8, 8) and not pay([64] * 512, 128, 8, 8)
+    # scratch beyond its bound: 32 KB of state a head and chunk
+    assert pay([16384]) and not pay([65536]) and not pay([64] * 1000)
+    # many portions of a few tokens beside one long enough
+    assert not pay([64] + [8] * 32) and not pay([256] + [8] * 128) and pay([64] + [32] * 32)
+
+
+def test_chunked_state_space_scratch_stays_below_its_bound():
+    rng = random.Random(3)
+    for _ in range(2000):
+        q = [rng.choice([2, 30, 64, 300, 5000, 60000]) for _ in range(rng.choice([1, 4, 300]))]
+        heads, N, V = rng.choice([(16, 128, 64), (64, 128, 64), (128, 256, 128), (3, 8, 8)])
+        if not ops._ssd_chunks_pay(sum(q), len(q), heads, N, V, q):
+            continue
+        cells = sum(-(-n // 64) for n in q)
+        assert cells * heads * N * V * 4 <= ops.SSD_MAX_SCRATCH_BYTES and heads * len(q) <= 65535
+
+
 @pytest.mark.parametrize("dim,rot,vdim,rank,takes", [
     (128, 64, 128, 512, True), (96, 32, 128, 256, True), (48, 16, 64, 64, True),
     (128, 0, 128, 128, True),
