@@ -12,14 +12,21 @@
 // a sequence's chunks: the scratch entry becomes the chunk's start state), out (every token's y).
 // The walk takes a token's 3 K V multiply-adds a head one token after the other, and its segments
 // side by side are bound by the FFMA and shared-memory rate (2,048 tokens, 32 heads of 128 x 64:
-// 144 + 311 us for its two passes, 92 us for these three).  Chunks do the same sums as products; what bounds them is the
-// scratch of a chunk's states (K V fp32 a head, written twice and read twice through L2).
+// 144 + 311 us for its two passes, 92 us for these three).  Chunks do the same sums as products;
+// what bounds them is the scratch of a chunk's states (K V fp32 a head, written twice and read
+// twice through L2).
 //
 // Nothing of 32 bits is narrowed: x, B and C enter the products as they are (bfloat16), and what is
 // fp32 (weighted inputs, weighted scores, start states) as three bfloat16 terms, 24 bits, small
 // terms first into fp32 accumulators.  The tensor cores do not round those sums to nearest, so sums
-// over the state's entries are taken 64 at a time and added in fp32.  G is summed in 64 bits, because exp(G_t - G_s) of close
-// tokens far down a chunk would lose the bits that their difference cancels.
+// over the state's entries are taken 64 at a time and added in fp32.  G is summed in 64 bits,
+// because exp(G_t - G_s) of close tokens far down a chunk would lose the bits that their difference
+// cancels.
+//
+// Products take numbers: a later token's weight of 0 times an infinite x is not a number, nor is
+// the second term of an infinite one.  So a block whose results are not all finite makes them again
+// token by token (walk_column): tokens ahead of an infinity keep their results, and what is
+// infinite in the walk is infinite here.
 //
 // Requires K and V multiples of 8, K at most 256, rows on 16-byte marks.
 #include "common.cuh"
@@ -100,7 +107,8 @@ __device__ __forceinline__ ScWhere sc_where(const int* cu_q, int s, int s0, int 
 __device__ __forceinline__ float sc_softplus(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
 // G and dt of the chunk's tokens by one warp; tokens past the end: G of the last, dt 0.
-__device__ __forceinline__ void sc_gates(double* G, float* dt, const ScIn& in, int h, int t0, int n) {
+__device__ __forceinline__ void sc_gates(double* G, float* dt, const ScIn& in, int h, int t0,
+                                         int n) {
   const int lane = threadIdx.x & 31;
   const float neg_a = -expf(in.a_log[h]), bias = in.dt_bias[h];
   double carry = 0.0;
@@ -123,6 +131,27 @@ __device__ __forceinline__ void sc_gates(double* G, float* dt, const ScIn& in, i
     carry = __shfl_sync(0xffffffffu, g, 31);
     G[t] = g;
     dt[t] = d;
+  }
+}
+
+// One value column of the chunk token by token, with the walk's operations: S, the column's state
+// with `pitch` floats from entry to entry, becomes the state behind the chunk; `y` (null: none)
+// takes the tokens' outputs, y_pitch floats apart.
+__device__ __noinline__ void walk_column(float a_log, float dsk, const float* dt, int n, int K,
+                                         int pk, const bf16* b_s, const bf16* c_s, const bf16* x,
+                                         long long ld, float* S, int pitch, float* y,
+                                         size_t y_pitch) {
+  const float neg_a = -expf(a_log);
+  for (int t = 0; t < n; ++t) {
+    const float d = dt[t], a = expf(neg_a * d), xv = __bfloat162float(x[(size_t)t * ld]);
+    float acc = 0.f;
+    for (int k = 0; k < K; ++k) {
+      const float kk = __fmul_rn(d, __bfloat162float(b_s[t * pk + k]));
+      const float s = __fmaf_rn(a, S[(size_t)k * pitch], __fmul_rn(kk, xv));
+      S[(size_t)k * pitch] = s;
+      if (y) acc = __fmaf_rn(s, __bfloat162float(c_s[t * pk + k]), acc);
+    }
+    if (y) y[t * y_pitch] = __fmaf_rn(dsk, xv, acc);
   }
 }
 
@@ -163,6 +192,7 @@ ssd_chunk_own_kernel(ScIn in, float* __restrict__ scr_s, float* __restrict__ scr
   const size_t cell = (size_t)at.entry * in.H + h;
   if (blockIdx.x == 0 && tid == 0) scr_p[cell] = expf((float)g_end);
   float* out = scr_s + cell * K * V;
+  bool bad = false;
   for (int mt = warp; mt < Kp >> 4; mt += SC_THREADS / 32) {
     float acc[SC_VT / 8][4];
 #pragma unroll
@@ -189,11 +219,20 @@ ssd_chunk_own_kernel(ScIn in, float* __restrict__ scr_s, float* __restrict__ scr
 #pragma unroll
     for (int j = 0; j < SC_VT / 8; ++j) {
       const int c = v0 + j * 8 + t2;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) bad |= !isfinite(acc[j][e]);
       if (c >= V) continue;
-      if (r < K) *reinterpret_cast<float2*>(out + (size_t)r * V + c) = make_float2(acc[j][0], acc[j][1]);
+      float* at_r = out + (size_t)r * V + c;
+      if (r < K) *reinterpret_cast<float2*>(at_r) = make_float2(acc[j][0], acc[j][1]);
       if (r + 8 < K)
-        *reinterpret_cast<float2*>(out + (size_t)(r + 8) * V + c) = make_float2(acc[j][2], acc[j][3]);
+        *reinterpret_cast<float2*>(at_r + (size_t)8 * V) = make_float2(acc[j][2], acc[j][3]);
     }
+  }
+  if (__syncthreads_or(bad) && tid < SC_VT && v0 + tid < V) {
+    float* S = out + v0 + tid;
+    for (int k = 0; k < K; ++k) S[(size_t)k * V] = 0.f;
+    walk_column(in.a_log[h], 0.f, dt, at.n, K, pk, b_s, nullptr, row + (size_t)h * V + v0 + tid,
+                in.ld, S, V, nullptr, 0);
   }
 }
 
@@ -278,128 +317,145 @@ ssd_chunk_out_kernel(ScIn in, const float* __restrict__ scr_s, float* __restrict
   if (warp == 0) sc_gates(G, dt, in, h, at.t0, at.n);
   sc_async_wait();
   __syncthreads();
-  if (warp * 16 >= at.n) return;                        // (no barrier follows)
-  const int t2 = (lane & 3) * 2;
-  const int ra = warp * 16 + (lane >> 2), rb = ra + 8;  // this thread's two tokens
-  float p[8][4], o[SC_VT / 8][4];
-#pragma unroll
-  for (int j = 0; j < 8; ++j)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) p[j][e] = 0.f;
-#pragma unroll
-  for (int j = 0; j < SC_VT / 8; ++j)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
-  const int arow = warp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, acol = (lane >> 4) * 8;
-  // scores of the warp's tokens against the chunk's tokens up to them
-  const int k_steps = Kp >> 4;
-  for (int k0 = 0; k0 < k_steps; k0 += 4) {
-    float t[8][4];
+  bool bad = false;
+  if (warp * 16 < at.n) {
+    const int t2 = (lane & 3) * 2;
+    const int ra = warp * 16 + (lane >> 2), rb = ra + 8;  // this thread's two tokens
+    float p[8][4], o[SC_VT / 8][4];
 #pragma unroll
     for (int j = 0; j < 8; ++j)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) t[j][e] = 0.f;
-    for (int kk = k0; kk < min(k0 + 4, k_steps); ++kk) {
-      unsigned a[4];
-      sc_ldm4(a, sc_smem(c_s + arow * pk + kk * 16 + acol));
+      for (int e = 0; e < 4; ++e) p[j][e] = 0.f;
 #pragma unroll
-      for (int j = 0; j < 8; j += 2) {
-        if (j <= 2 * warp + 1) {
-          unsigned b[4];
-          sc_ldm4(b, sc_smem(b_s + (j * 8 + (lane & 7) + ((lane >> 4) & 1) * 8) * pk + kk * 16 +
-                             ((lane >> 3) & 1) * 8));
-          sc_mma(t[j], a, b[0], b[1]);
-          sc_mma(t[j + 1], a, b[2], b[3]);
-        }
-      }
-    }
+    for (int j = 0; j < SC_VT / 8; ++j)
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) p[j][e] += t[j][e];
-  }
-  // the start state's part
-  for (int u = 2; u >= 0; --u) {
+      for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
+    const int arow = warp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, acol = (lane >> 4) * 8;
+    // scores of the warp's tokens against the chunk's tokens up to them
+    const int k_steps = Kp >> 4;
     for (int k0 = 0; k0 < k_steps; k0 += 4) {
-      float t[SC_VT / 8][4];
+      float t[8][4];
 #pragma unroll
-      for (int j = 0; j < SC_VT / 8; ++j)
+      for (int j = 0; j < 8; ++j)
 #pragma unroll
         for (int e = 0; e < 4; ++e) t[j][e] = 0.f;
       for (int kk = k0; kk < min(k0 + 4, k_steps); ++kk) {
         unsigned a[4];
         sc_ldm4(a, sc_smem(c_s + arow * pk + kk * 16 + acol));
-        const int brow = u * Kp + kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
 #pragma unroll
-        for (int j = 0; j < SC_VT / 8; j += 2) {
-          unsigned b[4];
-          sc_ldm4t(b, sc_smem(s_s + (size_t)brow * pv + j * 8 + ((lane >> 4) & 1) * 8));
-          sc_mma(t[j], a, b[0], b[1]);
-          sc_mma(t[j + 1], a, b[2], b[3]);
+        for (int j = 0; j < 8; j += 2) {
+          if (j <= 2 * warp + 1) {
+            unsigned b[4];
+            sc_ldm4(b, sc_smem(b_s + (j * 8 + (lane & 7) + ((lane >> 4) & 1) * 8) * pk + kk * 16 +
+                               ((lane >> 3) & 1) * 8));
+            sc_mma(t[j], a, b[0], b[1]);
+            sc_mma(t[j + 1], a, b[2], b[3]);
+          }
         }
       }
 #pragma unroll
-      for (int j = 0; j < SC_VT / 8; ++j)
+      for (int j = 0; j < 8; ++j)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) o[j][e] += t[j][e];
+        for (int e = 0; e < 4; ++e) p[j][e] += t[j][e];
     }
-  }
-  const double Ga = G[ra], Gb = G[rb];
-  const float ea = expf((float)Ga), eb = expf((float)Gb);
+    // the start state's part
+    for (int u = 2; u >= 0; --u) {
+      for (int k0 = 0; k0 < k_steps; k0 += 4) {
+        float t[SC_VT / 8][4];
 #pragma unroll
-  for (int j = 0; j < SC_VT / 8; ++j) {
-    o[j][0] *= ea; o[j][1] *= ea;
-    o[j][2] *= eb; o[j][3] *= eb;
-  }
+        for (int j = 0; j < SC_VT / 8; ++j)
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
+          for (int e = 0; e < 4; ++e) t[j][e] = 0.f;
+        for (int kk = k0; kk < min(k0 + 4, k_steps); ++kk) {
+          unsigned a[4];
+          sc_ldm4(a, sc_smem(c_s + arow * pk + kk * 16 + acol));
+          const int brow = u * Kp + kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int c = j * 8 + t2 + e;
-      const double Gc = G[c];
-      const float d = dt[c];
-      p[j][e] = c <= ra ? p[j][e] * (expf((float)(Ga - Gc)) * d) : 0.f;
-      p[j][2 + e] = c <= rb ? p[j][2 + e] * (expf((float)(Gb - Gc)) * d) : 0.f;
-    }
-  }
+          for (int j = 0; j < SC_VT / 8; j += 2) {
+            unsigned b[4];
+            sc_ldm4t(b, sc_smem(s_s + (size_t)brow * pv + j * 8 + ((lane >> 4) & 1) * 8));
+            sc_mma(t[j], a, b[0], b[1]);
+            sc_mma(t[j + 1], a, b[2], b[3]);
+          }
+        }
 #pragma unroll
-  for (int kk = 0; kk < 4; ++kk) {
-    if (kk > warp) break;
-    unsigned a[3][4];
+        for (int j = 0; j < SC_VT / 8; ++j)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {          // (row half, column half) of the fragment
-      unsigned t[3];
-      const float* f = p[2 * kk + (e >> 1)] + (e & 1) * 2;
-      sc_split(f[0], f[1], t);
-      a[0][e] = t[0]; a[1][e] = t[1]; a[2][e] = t[2];
-    }
-    const int brow = kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
-#pragma unroll
-    for (int j = 0; j < SC_VT / 8; j += 2) {
-      unsigned b[4];
-      sc_ldm4t(b, sc_smem(x_s + brow * pv + j * 8 + ((lane >> 4) & 1) * 8));
-#pragma unroll
-      for (int u = 2; u >= 0; --u) {
-        sc_mma(o[j], a[u], b[0], b[1]);
-        sc_mma(o[j + 1], a[u], b[2], b[3]);
+          for (int e = 0; e < 4; ++e) o[j][e] += t[j][e];
       }
     }
-  }
-  const float dsk = in.d_skip[h];
-  float* ya = y + ((size_t)(at.t0 + ra) * in.H + h) * V;
-  float* yb = y + ((size_t)(at.t0 + rb) * in.H + h) * V;
+    const double Ga = G[ra], Gb = G[rb];
+    const float ea = expf((float)Ga), eb = expf((float)Gb);
 #pragma unroll
-  for (int j = 0; j < SC_VT / 8; ++j) {
-    const int c = v0 + j * 8 + t2;
-    if (c >= V) continue;
-    const __nv_bfloat162 xa = *reinterpret_cast<const __nv_bfloat162*>(x_s + ra * pv + j * 8 + t2);
-    const __nv_bfloat162 xb = *reinterpret_cast<const __nv_bfloat162*>(x_s + rb * pv + j * 8 + t2);
-    if (ra < at.n)
-      *reinterpret_cast<float2*>(ya + c) = make_float2(fmaf(dsk, __low2float(xa), o[j][0]),
-                                                       fmaf(dsk, __high2float(xa), o[j][1]));
-    if (rb < at.n)
-      *reinterpret_cast<float2*>(yb + c) = make_float2(fmaf(dsk, __low2float(xb), o[j][2]),
-                                                       fmaf(dsk, __high2float(xb), o[j][3]));
+    for (int j = 0; j < SC_VT / 8; ++j) {
+      o[j][0] *= ea; o[j][1] *= ea;
+      o[j][2] *= eb; o[j][3] *= eb;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = j * 8 + t2 + e;
+        const double Gc = G[c];
+        const float d = dt[c];
+        p[j][e] = c <= ra ? p[j][e] * (expf((float)(Ga - Gc)) * d) : 0.f;
+        p[j][2 + e] = c <= rb ? p[j][2 + e] * (expf((float)(Gb - Gc)) * d) : 0.f;
+      }
+    }
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      if (kk > warp) break;
+      unsigned a[3][4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {          // (row half, column half) of the fragment
+        unsigned t[3];
+        const float* f = p[2 * kk + (e >> 1)] + (e & 1) * 2;
+        sc_split(f[0], f[1], t);
+        a[0][e] = t[0]; a[1][e] = t[1]; a[2][e] = t[2];
+      }
+      const int brow = kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
+#pragma unroll
+      for (int j = 0; j < SC_VT / 8; j += 2) {
+        unsigned b[4];
+        sc_ldm4t(b, sc_smem(x_s + brow * pv + j * 8 + ((lane >> 4) & 1) * 8));
+#pragma unroll
+        for (int u = 2; u >= 0; --u) {
+          sc_mma(o[j], a[u], b[0], b[1]);
+          sc_mma(o[j + 1], a[u], b[2], b[3]);
+        }
+      }
+    }
+    const float dsk = in.d_skip[h];
+    float* ya = y + ((size_t)(at.t0 + ra) * in.H + h) * V;
+    float* yb = y + ((size_t)(at.t0 + rb) * in.H + h) * V;
+#pragma unroll
+    for (int j = 0; j < SC_VT / 8; ++j) {
+      const int c = v0 + j * 8 + t2;
+      bad |= (ra < at.n && !(isfinite(o[j][0]) && isfinite(o[j][1]))) ||
+             (rb < at.n && !(isfinite(o[j][2]) && isfinite(o[j][3])));
+      if (c >= V) continue;
+      const bf16* x_at = x_s + ra * pv + j * 8 + t2;
+      const __nv_bfloat162 xa = *reinterpret_cast<const __nv_bfloat162*>(x_at);
+      const __nv_bfloat162 xb = *reinterpret_cast<const __nv_bfloat162*>(x_at + 8 * pv);
+      if (ra < at.n)
+        *reinterpret_cast<float2*>(ya + c) = make_float2(fmaf(dsk, __low2float(xa), o[j][0]),
+                                                         fmaf(dsk, __high2float(xa), o[j][1]));
+      if (rb < at.n)
+        *reinterpret_cast<float2*>(yb + c) = make_float2(fmaf(dsk, __low2float(xb), o[j][2]),
+                                                         fmaf(dsk, __high2float(xb), o[j][3]));
+    }
+  }
+  if (__syncthreads_or(bad)) {
+    float* S = reinterpret_cast<float*>(s_s);             // [K][SC_VT], where the terms were
+    for (int i = tid; i < K * SC_VT; i += SC_THREADS) {
+      const int c = v0 + i % SC_VT;
+      S[i] = c < V ? start[(size_t)(i / SC_VT) * V + c] : 0.f;
+    }
+    __syncthreads();
+    if (tid < SC_VT && v0 + tid < V)
+      walk_column(in.a_log[h], in.d_skip[h], dt, at.n, K, pk, b_s, c_s,
+                  row + (size_t)h * V + v0 + tid, in.ld, S + tid, SC_VT,
+                  y + ((size_t)at.t0 * in.H + h) * V + v0 + tid, (size_t)in.H * V);
   }
 }
 

@@ -111,3 +111,49 @@ def test_steps_that_are_left_to_the_walk(H, q_lens):
     finally:
         ops.USE_SSD_CHUNKS = True
     assert torch.equal(out, want) and torch.equal(got, state)
+
+
+@pytest.mark.parametrize("T", [100, 300])
+@pytest.mark.parametrize("what", ["nan in x", "inf in x", "inf in B", "inf in C", "nan in dt",
+                                  "inf in the state", "products beyond range"])
+def test_infinities_and_nan_stay_where_the_walk_has_them(T, what):
+    """Tokens ahead of one keep their results, those after it and the state are infinite or not a
+    number where the walk's are."""
+    ops = _ops()
+    H, V, N = 2, 72, 40
+    inner = H * V
+    g = torch.Generator(device="cuda").manual_seed(T)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    xbc, dt = rnd(T, inner + 2 * N).bfloat16(), rnd(T, H).bfloat16()
+    state = rnd(2, H, N, V)
+    t, slot = 70, 1
+    if what == "nan in x":
+        xbc[t, 5] = float("nan")
+    elif what == "inf in x":
+        xbc[t, 5], xbc[t + 3, inner - 1] = float("inf"), -float("inf")
+    elif what == "inf in B":
+        xbc[t, inner + 7] = float("inf")
+    elif what == "inf in C":
+        xbc[t, inner + N + 7] = -float("inf")
+    elif what == "nan in dt":
+        dt[t, 1] = float("nan")
+    elif what == "inf in the state":
+        state[slot, 1, 3, 8] = float("inf")
+    else:                                    # x of 1e38 against B of 1e-20: finite in the walk
+        xbc[t:, :inner], xbc[t:, inner:inner + N] = 1e38, 1e-20
+    step = _cuda(_step([T], [0], slots=[slot]))
+    par = (rnd(H) + 1.0, torch.tensor([-3.0, -2.0], device="cuda"), torch.ones(H, device="cuda"))
+    a, b = state.clone(), state.clone()
+    got = ops.ssd_recurrence(xbc, dt, *par, a, step, H, V, N, 1)
+    ops.USE_SSD_CHUNKS = False
+    try:
+        ref = ops.ssd_recurrence(xbc, dt, *par, b, step, H, V, N, 1)
+    finally:
+        ops.USE_SSD_CHUNKS = True
+    for x, y in ((got, ref), (a, b)):
+        assert torch.equal(x.isnan(), y.isnan()) and torch.equal(x.isinf(), y.isinf())
+        # a few 2^-24 of the sums either way, of the largest term in them
+        fine = y.isfinite()
+        torch.testing.assert_close(x[fine], y[fine], rtol=2e-4, atol=2e-5)
+    if what.endswith(("x", "B", "C", "dt")):
+        assert got[:t].isfinite().all()
