@@ -71,7 +71,7 @@ struct DsIn {
 };
 
 template <typename TA, int KQ, int C, bool LOCAL>
-__global__ void __launch_bounds__(DS_THREADS, KQ <= 2 ? 5 : 3)
+__global__ void __launch_bounds__(DS_THREADS, ds_min_blocks<KQ>())
 delta_segment_kernel(DsIn in, const TA* __restrict__ v, long long ldv, float* __restrict__ state,
                      float* __restrict__ out, float* __restrict__ scr_s,
                      float* __restrict__ scr_a) {
@@ -350,8 +350,8 @@ static inline size_t ds_smem(int K) {
 }
 
 // Segments for a step whose longest sequence brings max_q_len tokens: as many as keep the local
-// pass within the blocks the device holds at once (five an SM up to keys of 64, three beyond), none
-// shorter than 64 tokens.  Returns the number of segments and sets *seg_len; 1 and 0 when the
+// pass within the blocks the device holds at once (a second, nearly empty round would double it),
+// none shorter than 64 tokens.  Returns the number of segments and sets *seg_len; 1 and 0 when the
 // sequences are walked from end to end.
 IX_API int ix_delta_recurrence_segments(int S, int H, int K, int V, int max_q_len, int min_tokens,
                                         int max_segments, int* seg_len) {
@@ -359,7 +359,8 @@ IX_API int ix_delta_recurrence_segments(int S, int H, int K, int V, int max_q_le
   if (S <= 0 || H <= 0 || K <= 0 || V <= 0 || K > 8 * 64 || max_q_len < min_tokens) return 1;
   const int cols = ds_cols(K);
   const long long per = (long long)S * H * ((V + cols - 1) / cols + (K + cols - 1) / cols);
-  long long want = (long long)ds_resident(K) * 148 / per + 1;    // (the last segment has no local pass)
+  // (the last segment has no local pass)
+  long long want = ds_blocks_at_once(K, ds_smem(K)) / per + 1;
   if (want > max_segments) want = max_segments;
   if (want < 2) return 1;
   int len = (int)((max_q_len + want - 1) / want);
@@ -426,7 +427,8 @@ IX_API int ix_delta_segments(const void* q, long long ldq, const void* k, long l
               unit_eps, q_scale);
     DS_BY_K(K, DS_LOCAL);
     ix_launch(join_kern, dim3((V + DJ_COLS - 1) / DJ_COLS, H, S), dim3(DJ_THREADS), join, stream,
-              scr_s, (const float*)scr_a, (const float*)state, cu_q, state_slot, H, K, V, seg_len, nseg);
+              scr_s, (const float*)scr_a, (const float*)state, cu_q, state_slot, H, K, V, seg_len,
+              nseg);
     DS_BY_K(K, DS_WALK);
   });
 #undef DS_WALK

@@ -50,7 +50,7 @@ struct LsIn {
 enum { LS_LOCAL = 0, LS_WALK = 1, LS_BONUS = 2 };
 
 template <typename TA, int KQ, int C, int FORM>
-__global__ void __launch_bounds__(DS_THREADS, KQ <= 2 ? 5 : 3)
+__global__ void __launch_bounds__(DS_THREADS, ds_min_blocks<KQ>())
 linear_segment_kernel(LsIn in, const TA* __restrict__ v, long long ldv, float* __restrict__ state,
                       float* __restrict__ out, float* __restrict__ scr_s,
                       float* __restrict__ scr_p) {
@@ -264,15 +264,14 @@ static inline size_t ls_smem(int K) {
 }
 
 // Segments for a step whose longest sequence brings max_q_len tokens: as many as keep a pass within
-// the blocks the device holds at once (five an SM up to keys of 64, three beyond), none shorter
-// than 64 tokens.  Returns the number of segments and sets *seg_len; 1 and 0 when the sequences
-// are walked from end to end.
+// the blocks the device holds at once, none shorter than 64 tokens.  Returns the number of segments
+// and sets *seg_len; 1 and 0 when the sequences are walked from end to end.
 IX_API int ix_linear_recurrence_segments(int S, int H, int K, int V, int max_q_len, int min_tokens,
                                          int max_segments, int* seg_len) {
   *seg_len = 0;
   if (S <= 0 || H <= 0 || K <= 0 || V <= 0 || K > 8 * 64 || max_q_len < min_tokens) return 1;
   const long long per = (long long)S * H * ((V + ds_cols(K) - 1) / ds_cols(K));
-  long long want = (long long)ds_resident(K) * 148 / per;
+  long long want = ds_blocks_at_once(K, ls_smem(K)) / per;
   if (want > max_segments) want = max_segments;
   if (want < 2) return 1;
   int len = (int)((max_q_len + want - 1) / want);

@@ -62,8 +62,26 @@ static inline int ds_cols(int K) { return DS_GROUPS * (K <= 128 ? 4 : K <= 256 ?
 static inline int ds_pitch(int K) {
   return K <= 32 ? 32 : K <= 64 ? 64 : K <= 128 ? 128 : K <= 256 ? 256 : 512;
 }
-// Blocks of a pass that an SM holds at once, by registers and shared memory.
-static inline int ds_resident(int K) { return K <= 64 ? 5 : K <= 256 ? 3 : 1; }
+// Blocks of a pass that an SM holds at once: by registers what the launch bounds ask for, by shared
+// memory (228 KB, 1 KB of it for each block) three at keys of 128, two at 256, one beyond.
+template <int KQ> constexpr int ds_min_blocks() {
+  return KQ <= 2 ? 5 : KQ <= 4 ? 3 : KQ <= 8 ? 2 : 1;
+}
+static inline int ds_resident(int K, size_t smem) {
+  const int by_registers = K <= 64 ? 5 : K <= 128 ? 3 : K <= 256 ? 2 : 1;
+  const int by_smem = (int)(228 * 1024 / (smem + 1024));
+  return by_smem < by_registers ? by_smem : by_registers;
+}
+// Blocks of such a pass that the device holds at once (without a device, a B200's).
+static inline long long ds_blocks_at_once(int K, size_t smem) {
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    (void)cudaGetLastError();
+    sms = 148;
+  }
+  return (long long)ds_resident(K, smem) * sms;
+}
 
 // The sums of C columns over the DS_LANES lanes that share them; lane l of them gets column
 // ds_own<C>(l)'s.

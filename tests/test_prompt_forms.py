@@ -62,6 +62,28 @@ def test_exact_lengths_decide_where_they_are_known():
     assert rows([8192, 8192]) and not rows([8192, 200])
 
 
+@pytest.mark.parametrize("delta", [True, False])
+@pytest.mark.parametrize("K", [16, 64, 65, 128, 129, 256, 257, 512])
+def test_segments_fill_the_device_once(delta, K):
+    """Blocks of the pass that the segments are counted for stay within what 148 SMs hold: five an SM
+    by registers up to keys of 64, beyond that by two stages of 16 tokens in 228 KB."""
+    f = getattr(library.load(), "ix_delta_recurrence_segments" if delta
+                else "ix_linear_recurrence_segments")
+    pitch = next(p for p in (32, 64, 128, 256, 512) if K <= p)
+    cols = 16 * (4 if K <= 128 else 2 if K <= 256 else 1)
+    smem = 2 * 4 * (3 * 16 * pitch + 16 * cols + (32 if delta else 0))
+    most = 148 * min(5 if K <= 64 else 3, 228 * 1024 // (smem + 1024))
+    taken = 0
+    for H in (1, 2, 3, 5, 8, 16, 30):
+        for V in (8, 64, 128, 256):
+            seg = ctypes.c_int(0)
+            n = f(1, H, K, V, 20000, 128, 64, ctypes.byref(seg))
+            tiles = -(-V // cols) + (-(-K // cols) if delta else 0)
+            taken += n > 1
+            assert n == 1 or (n - 1 if delta else n) * H * tiles <= most
+    assert taken
+
+
 def test_chunked_state_space_leaves_what_it_cannot_hold_to_the_walk():
     pay = lambda q, heads=64, K=128, V=64: ops._ssd_chunks_pay(sum(q), len(q), heads, K, V, q)
     assert pay([64]) and pay([2048]) and pay([65, 128]) and pay([129, 2, 15], 4) and pay([64] * 100)
