@@ -67,7 +67,7 @@ delta_prepare_kernel(const TA* __restrict__ q, long long ldq, const TA* __restri
 struct DsIn {
   const float *qn, *kn, *kq, *beta, *decay;
   const int *cu_q, *state_slot;
-  int H, HK, K, V, seg_len, nseg, vec_g;
+  int H, HK, K, V, seg_len, vec_g;
 };
 
 template <typename TA, int KQ, int C, bool LOCAL>
@@ -102,7 +102,7 @@ delta_segment_kernel(DsIn in, const TA* __restrict__ v, long long ldv, float* __
   const int nseg_s = (seq_end - seq_begin + in.seg_len - 1) / in.seg_len;
   if (seg >= nseg_s || (LOCAL && seg == nseg_s - 1)) return;
   const int t_begin = seq_begin + seg * in.seg_len, t_end = min(seq_end, t_begin + in.seg_len);
-  const size_t cell = ((size_t)s * H + h) * in.nseg + seg;
+  const size_t cell = ds_cell(in.cu_q, s, in.seg_len, seg, H, h);
   float* my_s = scr_s + cell * K * V;       // local: the segment's own state; walk: its start
   float* my_a = scr_a + cell * K * K;
   auto entry = [&](int i) { return 4 * (l + DS_LANES * (i >> 2)) + (i & 3); };
@@ -268,7 +268,7 @@ template <bool STAGED>
 __global__ void __launch_bounds__(DJ_THREADS)
 delta_join_kernel(float* __restrict__ scr_s, const float* __restrict__ scr_a,
                   const float* __restrict__ state, const int* __restrict__ cu_q,
-                  const int* __restrict__ state_slot, int H, int K, int V, int seg_len, int nseg) {
+                  const int* __restrict__ state_slot, int H, int K, int V, int seg_len) {
   extern __shared__ __align__(16) float sm[];   // [2][K][DJ_COLS] the state's columns, [2][K][K]
   IX_PDL_WAIT();
   const int tid = threadIdx.x, c = tid % DJ_COLS, group = tid / DJ_COLS;
@@ -277,12 +277,12 @@ delta_join_kernel(float* __restrict__ scr_s, const float* __restrict__ scr_a,
   if (nseg_s <= 0) return;
   const bool ok = col < V;
   const float* st = state + ((size_t)state_slot[s] * H + h) * K * V;
-  const size_t cell = ((size_t)s * H + h) * nseg;
+  const size_t cell = ds_cell(cu_q, s, seg_len, 0, H, h);
   float *x = sm, *y = sm + K * DJ_COLS;
   float* a_s = sm + 2 * K * DJ_COLS;
   auto fetch = [&](int e) {
     if (STAGED && e + 1 < nseg_s) {              // (the last segment has no transitions)
-      const float* A = scr_a + (cell + e) * K * K;
+      const float* A = scr_a + (cell + (size_t)e * H) * K * K;
       float* to = a_s + (size_t)(e & 1) * K * K;
       for (int i = tid * 4; i < K * K; i += DJ_THREADS * 4) ds_async(to + i, A + i, 16);
     }
@@ -292,8 +292,9 @@ delta_join_kernel(float* __restrict__ scr_s, const float* __restrict__ scr_a,
   for (int kk = group; kk < K; kk += DJ_GROUPS)
     x[kk * DJ_COLS + c] = ok ? st[(size_t)kk * V + col] : 0.f;
   for (int e = 0; e < nseg_s; ++e) {
-    float* own = scr_s + (cell + e) * K * V;
-    const float* A = STAGED ? a_s + (size_t)(e & 1) * K * K : scr_a + (cell + e) * K * K;
+    float* own = scr_s + (cell + (size_t)e * H) * K * V;
+    const float* A = STAGED ? a_s + (size_t)(e & 1) * K * K
+                            : scr_a + (cell + (size_t)e * H) * K * K;
     const bool more = e + 1 < nseg_s;
     fetch(e + 1);                                // its buffer was last read before the barrier
     asm volatile("cp.async.wait_group 1;" ::: "memory");
@@ -363,6 +364,10 @@ IX_API int ix_delta_recurrence_segments(int S, int H, int K, int V, int max_q_le
   long long want = ds_blocks_at_once(K, ds_smem(K)) / per + 1;
   if (want > max_segments) want = max_segments;
   if (want < 2) return 1;
+  // two segments on a device that the sequences nearly fill: four passes over a few dozen tokens
+  // each take longer than one (64 heads of 128 x 128: 128 tokens 131 us against 109, 200 183
+  // against 168, 256 207 against 213)
+  if (want == 2 && K > 64 && max_q_len < 256) return 1;
   int len = (int)((max_q_len + want - 1) / want);
   len = (len + DS_CHUNK - 1) / DS_CHUNK * DS_CHUNK;
   if (len < 64) len = 64;
@@ -374,8 +379,8 @@ IX_API int ix_delta_recurrence_segments(int S, int H, int K, int V, int max_q_le
 
 // Floats of scratch: the segments' states and transitions, unit vectors, k . q and beta.
 IX_API long long ix_delta_segments_scratch_floats(int T, int S, int H, int HK, int K, int V,
-                                                  int nseg) {
-  const long long cells = (long long)S * H * nseg;
+                                                  int seg_len) {
+  const long long cells = ds_cells(T, S, seg_len, H);
   return ((cells * K * V + 3) & ~3LL) + ((cells * K * K + 3) & ~3LL) +
          2LL * T * HK * ds_pitch(K) + (long long)T * (HK + H) + 8;
 }
@@ -395,7 +400,7 @@ IX_API int ix_delta_segments(const void* q, long long ldq, const void* k, long l
   if (nseg < 2 || seg_len <= 0 || seg_len % DS_CHUNK || !scratch) return IX_ERR_SIZE;
   if ((uintptr_t)scratch & 15) return IX_ERR_ALIGN;
   const int KP = ds_pitch(K), cols = ds_cols(K);
-  const long long cells = (long long)S * H * nseg;
+  const long long cells = ds_cells(T, S, seg_len, H);
   float* scr_s = scratch;
   float* scr_a = scr_s + ((cells * K * V + 3) & ~3LL);
   float* qn = scr_a + ((cells * K * K + 3) & ~3LL);
@@ -403,7 +408,7 @@ IX_API int ix_delta_segments(const void* q, long long ldq, const void* k, long l
   float* kq = kn + (size_t)T * HK * KP;
   float* beta = kq + (size_t)T * HK;
   const int vtiles = (V + cols - 1) / cols, atiles = (K + cols - 1) / cols;
-  const DsIn in = {qn, kn, kq, beta, decay, cu_q, state_slot, H, HK, K, V, seg_len, nseg,
+  const DsIn in = {qn, kn, kq, beta, decay, cu_q, state_slot, H, HK, K, V, seg_len,
                    K % 4 == 0 && ((uintptr_t)decay & 15) == 0 ? 1 : 0};
   const bool staged = K % 4 == 0 && K <= DJ_MAX_STAGED;
   const size_t smem = ds_smem(K);
@@ -427,8 +432,7 @@ IX_API int ix_delta_segments(const void* q, long long ldq, const void* k, long l
               unit_eps, q_scale);
     DS_BY_K(K, DS_LOCAL);
     ix_launch(join_kern, dim3((V + DJ_COLS - 1) / DJ_COLS, H, S), dim3(DJ_THREADS), join, stream,
-              scr_s, (const float*)scr_a, (const float*)state, cu_q, state_slot, H, K, V, seg_len,
-              nseg);
+              scr_s, (const float*)scr_a, (const float*)state, cu_q, state_slot, H, K, V, seg_len);
     DS_BY_K(K, DS_WALK);
   });
 #undef DS_WALK

@@ -48,6 +48,17 @@ __device__ __forceinline__ void ds_async(void* dst, const void* src, int bytes) 
 #define DS_LANES 8
 #define DS_GROUPS (DS_WARPS * (32 / DS_LANES))    // of columns, a block
 
+// Where segment `seg` of sequence s lies in scratch, for head h: tokens before the sequence /
+// tokens a segment + the sequence's number + the segment's.  No two meet, and T / seg_len + S + 1
+// hold all, also where one sequence of many is long.
+__device__ __forceinline__ size_t ds_cell(const int* cu_q, int s, int seg_len, int seg, int H,
+                                          int h) {
+  return (size_t)(cu_q[s] / seg_len + s + seg) * H + h;
+}
+static inline long long ds_cells(int T, int S, int seg_len, int H) {
+  return ((long long)T / seg_len + S + 1) * H;
+}
+
 // float4 a lane, columns a thread, by the key's size
 #define DS_BY_K(K, GO)           \
   do {                           \

@@ -2111,28 +2111,34 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: 
     if bonus_form and (bonus is None or bonus.numel() != heads * dim):
         raise KernelError("linear_recurrence: the bonus form needs u [heads, dim]")
     out = torch.empty((T, heads, vdim), dtype=torch.float32, device=q.device)
-    views = (_ptr(q), ctypes.c_longlong(ldq), _ptr(k), ctypes.c_longlong(ldk), _ptr(v),
-             ctypes.c_longlong(ldv), _dtype_code(q), _ptr(decay), _ptr(bonus), _ptr(state),
-             _ptr(step.cu_q), _ptr(step.state_slot), _ptr(out))
+
+    def views(first):                    # from row and sequence `first` on
+        return (_ptr(q[first:]), ctypes.c_longlong(ldq), _ptr(k[first:]), ctypes.c_longlong(ldk),
+                _ptr(v[first:]), ctypes.c_longlong(ldv), _dtype_code(q), _ptr(decay[first:]),
+                _ptr(bonus), _ptr(state), _ptr(step.cu_q_prompt if first else step.cu_q),
+                _ptr(step.state_slot[first:]), _ptr(out[first:]))
+
     # the kernels' side knows how many of their blocks the device holds at once
+    first, seqs, busy, longest = _segmented_part(step, T)
     seg = ctypes.c_int(0)
-    nseg = _lib().ix_linear_recurrence_segments(
-        step.num_seqs, heads, dim, vdim, int(getattr(step, "max_q_len", 0) or T),
-        RECURRENCE_SEGMENT_MIN, RECURRENCE_MAX_SEGMENTS, ctypes.byref(seg))
-    if nseg <= 1:
+    nseg = _lib().ix_linear_recurrence_segments(busy, heads, dim, vdim, longest,
+                                                RECURRENCE_SEGMENT_MIN, RECURRENCE_MAX_SEGMENTS,
+                                                ctypes.byref(seg))
+    walked = first if nseg > 1 else step.num_seqs
+    if walked:
         _check(_lib().ix_linear_recurrence(
-            *views, step.num_seqs, heads, dim, vdim, ctypes.c_float(q_scale),
+            *views(0), walked, heads, dim, vdim, ctypes.c_float(q_scale),
             1 if bonus_form else 0, _stream()), "linear_recurrence")
         _count()
-        return out
-    size = _lib().ix_linear_segments_scratch_floats
-    size.restype = ctypes.c_longlong
-    scratch = torch.empty((size(T, step.num_seqs, heads, dim, vdim, nseg),), dtype=torch.float32,
-                          device=q.device)
-    _check(_lib().ix_linear_segments(
-        *views, T, step.num_seqs, heads, dim, vdim, ctypes.c_float(q_scale),
-        1 if bonus_form else 0, seg.value, nseg, _ptr(scratch), _stream()), "linear_segments")
-    _count(4)
+    if nseg > 1:
+        size = _lib().ix_linear_segments_scratch_floats
+        size.restype = ctypes.c_longlong
+        scratch = torch.empty((size(T - first, seqs, heads, dim, vdim, seg.value),),
+                              dtype=torch.float32, device=q.device)
+        _check(_lib().ix_linear_segments(
+            *views(first), T - first, seqs, heads, dim, vdim, ctypes.c_float(q_scale),
+            1 if bonus_form else 0, seg.value, nseg, _ptr(scratch), _stream()), "linear_segments")
+        _count(4)
     return out
 
 
@@ -2144,8 +2150,23 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: 
 # the delta rule decide beside their kernels; ``recurrence_segments`` (RECURRENCE_BLOCKS) is for
 # the state space where it is not chunked.
 RECURRENCE_SEGMENT_MIN = 128
+# From this many single tokens ahead of the prompts on they are walked by a launch of their own: in
+# the four passes a state moves through scratch and back (16 heads of 128 x 128, 32 single tokens
+# and a prompt of 256: 188 us in segments together, 175 walked together).
+RECURRENCE_SINGLES_APART = 8
 RECURRENCE_BLOCKS = 1024
 RECURRENCE_MAX_SEGMENTS = 64
+
+
+def _segmented_part(step, T: int):
+    """(first, sequences, busy, longest) for a recurrence that may be walked in segments: the
+    sequences from ``first`` on, which are as much work as ``busy`` ones of the longest's tokens
+    (that many keep blocks busy to the end of a pass)."""
+    S, longest = step.num_seqs, int(getattr(step, "max_q_len", 0) or T)
+    first = int(getattr(step, "num_decode_seqs", 0) or 0)
+    if not RECURRENCE_SINGLES_APART <= first < S or getattr(step, "cu_q_prompt", None) is None:
+        first = 0
+    return first, S - first, max(1, min(S - first, -(-(T - first) // longest))), longest
 
 
 def recurrence_segments(max_q_len: int, num_seqs: int, heads: int, vdim: int):
@@ -2403,28 +2424,35 @@ def delta_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta_raw
             decay.shape != (T, heads * dim) or tuple(state.shape[1:]) != (heads, dim, vdim):
         raise KernelError("delta_recurrence: inputs and state do not fit together")
     out = torch.empty((T, heads, vdim), dtype=torch.float32, device=q.device)
-    views = (_ptr(q), ctypes.c_longlong(ldq), _ptr(k), ctypes.c_longlong(ldk), _ptr(v),
-             ctypes.c_longlong(ldv), _ptr(beta_raw), ctypes.c_longlong(ldb), _dtype_code(q),
-             _ptr(decay), _ptr(state), _ptr(step.cu_q), _ptr(step.state_slot), _ptr(out))
+
+    def views(first):                    # from row and sequence `first` on
+        return (_ptr(q[first:]), ctypes.c_longlong(ldq), _ptr(k[first:]), ctypes.c_longlong(ldk),
+                _ptr(v[first:]), ctypes.c_longlong(ldv), _ptr(beta_raw[first:]),
+                ctypes.c_longlong(ldb), _dtype_code(q), _ptr(decay[first:]), _ptr(state),
+                _ptr(step.cu_q_prompt if first else step.cu_q), _ptr(step.state_slot[first:]),
+                _ptr(out[first:]))
+
     # the kernels' side knows how many of their blocks the device holds at once
+    first, seqs, busy, longest = _segmented_part(step, T)
     seg = ctypes.c_int(0)
-    nseg = _lib().ix_delta_recurrence_segments(
-        step.num_seqs, heads, dim, vdim, int(getattr(step, "max_q_len", 0) or T),
-        RECURRENCE_SEGMENT_MIN, RECURRENCE_MAX_SEGMENTS, ctypes.byref(seg))
-    if nseg <= 1:
+    nseg = _lib().ix_delta_recurrence_segments(busy, heads, dim, vdim, longest,
+                                               RECURRENCE_SEGMENT_MIN, RECURRENCE_MAX_SEGMENTS,
+                                               ctypes.byref(seg))
+    walked = first if nseg > 1 else step.num_seqs
+    if walked:
         _check(_lib().ix_delta_recurrence(
-            *views, step.num_seqs, heads, kv_heads, dim, vdim, ctypes.c_float(unit_eps),
+            *views(0), walked, heads, kv_heads, dim, vdim, ctypes.c_float(unit_eps),
             ctypes.c_float(q_scale), _stream()), "delta_recurrence")
         _count()
-        return out
-    size = _lib().ix_delta_segments_scratch_floats
-    size.restype = ctypes.c_longlong
-    scratch = torch.empty((size(T, step.num_seqs, heads, kv_heads, dim, vdim, nseg),),
-                          dtype=torch.float32, device=q.device)
-    _check(_lib().ix_delta_segments(
-        *views, T, step.num_seqs, heads, kv_heads, dim, vdim, ctypes.c_float(unit_eps),
-        ctypes.c_float(q_scale), seg.value, nseg, _ptr(scratch), _stream()), "delta_segments")
-    _count(4)
+    if nseg > 1:
+        size = _lib().ix_delta_segments_scratch_floats
+        size.restype = ctypes.c_longlong
+        scratch = torch.empty((size(T - first, seqs, heads, kv_heads, dim, vdim, seg.value),),
+                              dtype=torch.float32, device=q.device)
+        _check(_lib().ix_delta_segments(
+            *views(first), T - first, seqs, heads, kv_heads, dim, vdim, ctypes.c_float(unit_eps),
+            ctypes.c_float(q_scale), seg.value, nseg, _ptr(scratch), _stream()), "delta_segments")
+        _count(4)
     return out
 
 

@@ -33,3 +33,26 @@ def test_segments(dtype, H, HK, K, V, q_lens):
     off = lambda a, b: float((a.cpu() - b.view(a.shape)).norm() / b.norm())
     assert off(out, ref) <= 2e-5 and off(got, st_ref) <= 2e-5
     assert torch.equal(got[S].cpu(), state[S])
+
+
+@pytest.mark.parametrize("q_lens,launches", [([1] * 9 + [300, 2], 5), ([3] * 20 + [700], 4)])
+def test_long_prompts_among_many_short_sequences(q_lens, launches):
+    """Single tokens are walked by a launch of their own, the rest in segments; scratch holds one
+    long sequence beside many short ones."""
+    from inferx_b200.kernels import ops
+    g = torch.Generator().manual_seed(len(q_lens))
+    H, HK, K, V, S, T = 4, 2, 24, 40, len(q_lens), sum(q_lens)
+    st = _step(q_lens, [3] * S, slots=list(range(S))[::-1])
+    q, k = (torch.randn(T, HK * K, generator=g) for _ in range(2))
+    v, beta = torch.randn(T, H * V, generator=g), torch.randn(T, H, generator=g)
+    decay = torch.rand(T, H * K, generator=g) * 0.3 + 0.7
+    state = torch.randn(S + 1, H, K, V, generator=g)
+    st_ref, got = state.clone(), state.cuda()
+    ref = host_ops.delta_recurrence(q, k, v, beta, decay, st_ref, st, H, HK, K, V, 1e-6, K ** -0.5)
+    before = ops.LAUNCHES[0]
+    out = ops.delta_recurrence(q.cuda(), k.cuda(), v.cuda(), beta.cuda(), decay.cuda(), got,
+                               _cuda(st), H, HK, K, V, 1e-6, K ** -0.5)
+    assert ops.LAUNCHES[0] == before + launches
+    off = lambda a, b: float((a.cpu() - b.view(a.shape)).norm() / b.norm())
+    assert off(out, ref) <= 2e-5 and off(got, st_ref) <= 2e-5
+    assert torch.equal(got[S].cpu(), state[S])

@@ -80,8 +80,48 @@ def test_segments_fill_the_device_once(delta, K):
             n = f(1, H, K, V, 20000, 128, 64, ctypes.byref(seg))
             tiles = -(-V // cols) + (-(-K // cols) if delta else 0)
             taken += n > 1
+            if K > 256 and not delta and n == 2:
+                continue                # (two segments whatever the device holds: next test)
             assert n == 1 or (n - 1 if delta else n) * H * tiles <= most
     assert taken
+
+
+def test_segments_where_they_pay():
+    def count(entry, S, H, K, V, longest):
+        return getattr(library.load(), entry)(S, H, K, V, longest, 128, 64,
+                                              ctypes.byref(ctypes.c_int(0)))
+    # two segments of a few dozen tokens on a full device: one pass from end to end
+    assert count("ix_delta_recurrence_segments", 1, 64, 128, 128, 200) == 1
+    assert count("ix_delta_recurrence_segments", 4, 16, 96, 128, 128) == 1
+    assert count("ix_delta_recurrence_segments", 1, 64, 128, 128, 256) == 2
+    assert count("ix_delta_recurrence_segments", 4, 16, 64, 128, 128) == 2
+    # large keys: the walk from end to end of the linear recurrence is the slower one
+    assert count("ix_linear_recurrence_segments", 1, 16, 384, 128, 3000) == 2
+    assert count("ix_linear_recurrence_segments", 4, 64, 512, 256, 128) == 2
+
+
+@pytest.mark.parametrize("q_lens,first,seqs,busy", [
+    ([1024] + [8] * 32, 0, 33, 2), ([128] * 4, 0, 4, 4), ([1] * 32 + [256], 32, 1, 1),
+    ([1] * 200 + [2000, 100], 200, 2, 2), ([1, 1, 300, 2], 0, 4, 2), ([700], 0, 1, 1)])
+def test_segments_are_counted_by_the_tokens_there_are(q_lens, first, seqs, busy):
+    """One long prompt among short ones is not one of as many."""
+    from types import SimpleNamespace
+    step = SimpleNamespace(num_seqs=len(q_lens), max_q_len=max(q_lens), cu_q_prompt=object(),
+                           num_decode_seqs=sum(n == 1 for n in q_lens))
+    assert ops._segmented_part(step, sum(q_lens)) == (first, seqs, busy, max(q_lens))
+
+
+def test_segments_do_not_share_scratch():
+    """Cells of scratch as the segmented recurrences number them."""
+    rng = random.Random(4)
+    for _ in range(1000):
+        L = 16 * rng.randint(4, 40)
+        q = [rng.choice([1, 2, L, rng.randint(1, 3000)]) for _ in range(rng.randint(1, 40))]
+        begin, cells = 0, []
+        for s, n in enumerate(q):
+            cells += [begin // L + s + e for e in range(-(-n // L))]
+            begin += n
+        assert len(set(cells)) == len(cells) and max(cells) < begin // L + len(q) + 1
 
 
 def test_chunked_state_space_leaves_what_it_cannot_hold_to_the_walk():
