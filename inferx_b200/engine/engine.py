@@ -72,17 +72,32 @@ def cache_bytes_per_page(model, page_size: int) -> List[int]:
     return out
 
 
+def step_scratch_bytes(cfg: EngineConfig, model) -> int:
+    """The most that one mixer takes beside a step's activations (widened keys and values, the
+    states of a prompt's chunks or segments); the mixers of a step take it in turn."""
+    most, todo = 0, [p for b in getattr(model, "blocks", ()) for p in b.parts()]
+    while todo:
+        part = todo.pop()
+        if hasattr(part, "step_scratch_bytes"):
+            most = max(most, part.step_scratch_bytes(cfg.batched_tokens(), cfg.max_num_seqs,
+                                                     cfg.max_model_len))
+        # mixers made of two
+        todo += [x for x in vars(part).values() if hasattr(x, "step_scratch_bytes")
+                 or type(x).__name__.endswith("Mixer")]
+    return most
+
+
 def graph_reserve_bytes(cfg: EngineConfig, model) -> int:
     """Device memory to leave for recorded steps: each kept graph holds the logits of its
     wanted rows (at most one row per resident sequence, fp32 over the vocabulary), and
-    all of them share one pool of activations sized by the largest step (some dozens of
-    bytes per token and unit of width, taken generously)."""
+    all of them share one pool sized by the largest step: activations (some dozens of
+    bytes per token and unit of width, taken generously) and a mixer's scratch."""
     from .executor import GraphCache
     limits = GraphCache().limits
     spec = model.spec
     logits = (limits[True] + limits[False]) * cfg.max_num_seqs * spec.vocab_size * 4
     activations = cfg.batched_tokens() * spec.hidden * 64
-    return logits + activations
+    return logits + activations + step_scratch_bytes(cfg, model)
 
 
 def autosize_pages(cfg: EngineConfig, model, device) -> int:
@@ -98,8 +113,7 @@ def autosize_pages(cfg: EngineConfig, model, device) -> int:
     free, total = torch.cuda.mem_get_info(device)
     used = total - free
     budget = int(cfg.gpu_memory_utilization * total) - used - (1 << 30)
-    if not cfg.enforce_eager:
-        budget -= graph_reserve_bytes(cfg, model)
+    budget -= (step_scratch_bytes if cfg.enforce_eager else graph_reserve_bytes)(cfg, model)
     # no more than every resident sequence at full length can use
     want = cfg.max_num_seqs * floor
     return max(floor, min(want, budget // per_page))

@@ -1778,6 +1778,21 @@ def widened_latent_rows(q_lens: Sequence[int], max_kv_len: int, window: int, hea
     return rows if widened < folded else 0
 
 
+def widened_scratch_bytes(tokens: int, seqs: int, max_kv_len: int, window: int, heads: int,
+                          rank: int, rot_dim: int, dim: int, vdim: int) -> int:
+    """The most a step takes in the widened form: records, keys in fp32 on the way, and the
+    widened rows, of as many portions as their limit lets through."""
+    rows = int(max_kv_len) * 2                 # recorded tables are rounded up to a power of two
+    if window > 0:
+        rows = min(rows, window + tokens + 63)
+    rows = -(-rows // 64) * 64
+    row = heads * 2 * (dim + rot_dim + _lib().ix_widened_second(dim + rot_dim, dim) + vdim)
+    total = min(seqs * rows, WIDENED_MAX_BYTES // row)
+    keys = heads * dim * 4
+    return (total * (row + 2 * (rank + rot_dim))
+            + min(total * keys, max(WIDENED_FP32_BYTES, 256 * keys)))
+
+
 def latent_front_inplace(q: Optional[torch.Tensor], q_ld: int, kv: Optional[torch.Tensor],
                          kv_ld: int, positions: torch.Tensor, freq: torch.Tensor, mag: float,
                          gain: Optional[torch.Tensor], eps: float, heads: int, dim: int,
@@ -2156,6 +2171,17 @@ RECURRENCE_SEGMENT_MIN = 128
 RECURRENCE_SINGLES_APART = 8
 RECURRENCE_BLOCKS = 1024
 RECURRENCE_MAX_SEGMENTS = 64
+
+
+def segments_scratch_bytes(tokens: int, seqs: int, heads: int, kv_heads: int, dim: int, vdim: int,
+                           delta: bool) -> int:
+    """What a step of ``tokens`` in ``seqs`` portions takes where it is walked in segments."""
+    seg_len = max(64, tokens // RECURRENCE_MAX_SEGMENTS)
+    lib = _lib()
+    size = lib.ix_delta_segments_scratch_floats if delta else lib.ix_linear_segments_scratch_floats
+    size.restype = ctypes.c_longlong
+    return 4 * (size(tokens, seqs, heads, kv_heads, dim, vdim, seg_len) if delta
+                else size(tokens, seqs, heads, dim, vdim, seg_len))
 
 
 def _segmented_part(step, T: int):

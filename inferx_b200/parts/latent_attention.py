@@ -49,7 +49,7 @@ class LatentAttentionMixer:
         s = spec
         self.q_width = s.heads * (s.dim + s.rot_dim)
         self.q_rank = s.q_rank              # -1 until the checkpoint says it
-        self.uq_w = self.q_gain = None
+        self.uq_w = self.q_gain = self.kv_w = None
         self._place()
 
     def _place(self):
@@ -120,6 +120,14 @@ class LatentAttentionMixer:
         if not s.own_records:
             return []
         return [PagedKvNeed(1, s.kv_rank + s.rot_dim, s.window, entries=(ENTRY,))]
+
+    def step_scratch_bytes(self, tokens, seqs, max_len):
+        """The most that a step's attention takes beside its activations."""
+        s = self.spec
+        if self.kv_w is None:
+            return 0
+        return self.ctx.ops.widened_scratch_bytes(tokens, seqs, max_len, s.window, s.heads,
+                                                  s.kv_rank, s.rot_dim, s.dim, s.vdim)
 
     def _pair_table(self, x):
         if self.position is not None:

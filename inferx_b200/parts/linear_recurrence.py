@@ -10,11 +10,11 @@ order with a decay per key channel:
 
 The recurrence, the decays (sigmoid, logarithms, exponentials), the per-head norm of
 the output and the gate's silu are fp32; the projections are the run's matrix products.
-One kernel serves both recurrences (``ops.linear_recurrence``): a sequence's state
-column is owned by one thread from its first token of the step to its last, so a
-position's result does not depend on how the sequence was cut into steps or on what
-else is in the batch; long prompt portions are cut into segments that are walked side by
-side and joined, which changes results by rounding only.
+``ops.linear_recurrence`` serves both.  Single tokens and short portions are walked from
+end to end in an order of sums fixed by the sizes, so a position's result does not depend on
+how the sequence was cut into steps or on what else is in the batch; long prompt portions
+are cut into segments that are walked side by side and joined, by kernels of their own, which
+changes results by rounding only.
 """
 from __future__ import annotations
 
@@ -71,6 +71,13 @@ class GatedLinearAttention:
     def cache_needs(self):
         s = self.spec
         return [StateNeed(STATE, (s.heads, s.dim, s.vdim), torch.float32)]
+
+    def step_scratch_bytes(self, tokens, seqs, max_len):
+        """The most that a step's recurrence takes beside its activations."""
+        s, ops = self.spec, self.ctx.ops
+        if not hasattr(ops, "segments_scratch_bytes"):
+            return 0
+        return ops.segments_scratch_bytes(tokens, seqs, s.heads, s.heads, s.dim, s.vdim, False)
 
     def forward(self, x, step, cache):
         s, ops = self.spec, self.ctx.ops
@@ -129,6 +136,13 @@ class WkvMixer:
         s = self.spec
         return [StateNeed(STATE, (s.heads, s.dim, s.dim), torch.float32),
                 StateNeed(PREVIOUS, (s.hidden,), torch.float32)]
+
+    def step_scratch_bytes(self, tokens, seqs, max_len):
+        """The most that a step's recurrence takes beside its activations."""
+        s, ops = self.spec, self.ctx.ops
+        if not hasattr(ops, "segments_scratch_bytes"):
+            return 0
+        return ops.segments_scratch_bytes(tokens, seqs, s.heads, s.heads, s.dim, s.dim, False)
 
     def forward(self, x, step, cache):
         s, ops = self.spec, self.ctx.ops

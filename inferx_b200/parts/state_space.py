@@ -15,9 +15,10 @@ Both keep, per request, S in fp32 and the last taps - 1 inputs of their convolut
 the cache manager's state slots (zeroed when a slot is handed out: the zeros before
 position 0 and the empty state).  The recurrences, step sizes, decays, unit norms and
 output norms are fp32; the projections and convolutions are in the run's element type.
-A sequence's state column is owned by one thread from its first token of a step to its
-last and every sum has an order fixed by the sizes alone, so a position's result does
-not depend on how the sequence was cut into steps or on what else is in the batch.
+Walked token by token, every sum has an order fixed by the sizes alone, so a position's
+result does not depend on how the sequence was cut into steps or on what else is in the
+batch; prompts in segments (both) or in chunks on the tensor cores (the state space in
+bfloat16 runs) differ from that by rounding.
 """
 from __future__ import annotations
 
@@ -82,6 +83,14 @@ class StateSpaceMixer:
         if s.conv > 1:
             needs.append(StateNeed(SSD_CONV, (s.conv - 1, self.conv_width), torch.float32))
         return needs
+
+    def step_scratch_bytes(self, tokens, seqs, max_len):
+        """The most that a step's recurrence takes beside its activations."""
+        s, ops = self.spec, self.ctx.ops
+        if self.ctx.dtype != torch.bfloat16 or not hasattr(ops, "ssd_chunks_scratch_bytes"):
+            return 0
+        return min(ops.SSD_MAX_SCRATCH_BYTES,
+                   ops.ssd_chunks_scratch_bytes(tokens, seqs, s.heads, s.state, s.vdim))
 
     def forward(self, x, step, cache):
         s, ops = self.spec, self.ctx.ops
@@ -156,6 +165,12 @@ class GatedDeltaMixer:
         if s.conv > 1:
             needs.append(StateNeed(DELTA_CONV, (s.conv - 1, self.conv_width), torch.float32))
         return needs
+
+    def step_scratch_bytes(self, tokens, seqs, max_len):
+        s, ops = self.spec, self.ctx.ops
+        if not hasattr(ops, "segments_scratch_bytes"):
+            return 0
+        return ops.segments_scratch_bytes(tokens, seqs, s.heads, s.kv_heads, s.dim, s.vdim, True)
 
     def forward(self, x, step, cache):
         s, ops = self.spec, self.ctx.ops
