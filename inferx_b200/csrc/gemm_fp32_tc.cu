@@ -27,12 +27,17 @@
 // With fewer tiles than SMs, or a last wave that is nearly empty, k is cut into `splits` runs whose
 // partial sums a second kernel adds in ascending order.
 //
-// Infinities and NaN, and sums that overflow on the way, come out of the terms as NaN; such a
-// result is computed again from the operands, fp32 multiply-adds, a warp per element.  (Terms
-// below 2^-126 are bfloat16 subnormals: operands under some 1e-33 may lose their last bits.)
+// Infinities and NaN, and sums that overflow on the way, come out of the terms as infinities or
+// NaN; bfloat16 holds no third term of numbers below 2^-110.  A sum that is not finite, or below
+// 2^-64 and not 0, is computed again from the operands, fp32 multiply-adds, a warp per element.
+// (What is left: operands below 2^-110 that meet others above 2^40 lose last bits.)  That code
+// stands at the end of the block, unrolled: made a function on sums in shared memory, it costs the
+// loop over steps 10 %, by other registers.
 //
 // Every mbarrier wait is bounded (codes 41: splitting warps, 42: MMA).  Requires K a multiple of
 // 8 and bases on 32-byte marks.
+#include <cfloat>
+
 #include "common.cuh"
 #include "tma_common.cuh"
 #include "tcgen05_common.cuh"
@@ -105,6 +110,13 @@ __device__ __forceinline__ void f3_st16x16(unsigned taddr, const unsigned* r) {
       "tcgen05.st.sync.aligned.16x256b.x2.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr),
       "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
       : "memory");
+}
+
+// Whether a sum has to be made again: not finite, or so small that operands without a third term
+// may have gone into it.
+__device__ __forceinline__ bool f3_again(float s) {
+  const float a = fabsf(s);
+  return !(a <= FLT_MAX) || (a < 5.421010862427522e-20f && a > 0.f);
 }
 
 __global__ void __launch_bounds__(F3_THREADS, 1)
@@ -268,10 +280,10 @@ gemm_fp32_tc_kernel(const float* __restrict__ x, const float* __restrict__ w,
       if (lane == 0 && !*abortp) { atomicExch(status, F3_ERR_SPLIT); *abortp = 1; }
     } else {
       const int row = m0 + quarter * 32 + lane, col0 = n0 + half * 64;
-      // results that are not numbers, again from the operands: a warp per element
+      // sums that have to be, again from the operands: a warp per element
 #pragma unroll
       for (int i = 0; i < 64; ++i) {
-        unsigned bad = __ballot_sync(0xffffffffu, row < M && col0 + i < N && isnan(acc[i]));
+        unsigned bad = __ballot_sync(0xffffffffu, row < M && col0 + i < N && f3_again(acc[i]));
         while (bad) {
           const int l = __ffs(bad) - 1;
           bad &= bad - 1;
@@ -325,8 +337,9 @@ __global__ void gemm_fp32_tc_sum_kernel(const float* __restrict__ part, float* _
 // Runs to cut k into: the number for which waves x steps of a block, and what the partial sums
 // cost to write and read, is least.  A step is some 1.6 us; partial sums 0.35 us a MB both ways,
 // their kernel's launch 3 us (M 600, N 2048, K 5632: 3 runs 120 us, one 145; M 64, N 11264,
-// K 2048: one run 60 us, 3 runs 70; M 64, N 2048, K 5632: 9 runs 35.5 us, one 140).  No run is
-// shorter than 4 steps.
+// K 2048: one run 60 us, 3 runs 70; M 64, N 2048, K 5632: 9 runs 35.5 us, one 140).  Runs are 4
+// steps at least on average; the last may be shorter.  A row's last bits follow the number of runs,
+// and so the number of rows.
 IX_API int ix_gemm_fp32_tc_splits(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return 1;
   const long long tiles = ((M + F3_BM - 1) / F3_BM) * (long long)((N + F3_BN - 1) / F3_BN);

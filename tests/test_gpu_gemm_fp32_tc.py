@@ -72,3 +72,36 @@ def test_which_products_take_it():
     assert not ops._splits_fp32(off, w)
     torch.testing.assert_close(ops.linear(off, w), off @ w.T, rtol=1e-4, atol=1e-4)
     assert ops.LAUNCHES[0] == before + 1
+
+
+@pytest.mark.parametrize("scale_x,scale_w", [(1e-36, 1.0), (1e-38, 1.0), (1e-38, 1e6),
+                                             (1e-20, 1e-20), (1e-30, 1e-10), (1e-33, 1e-3)])
+@pytest.mark.parametrize("splits", [1, 4])
+def test_operands_too_small_for_three_terms(scale_x, scale_w, splits):
+    """Below 2^-110 the third term is a subnormal, below 2^-126 the second too: such sums are made
+    from the operands themselves."""
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn(40, 1024, generator=g, device="cuda") * scale_x
+    w = torch.randn(130, 1024, generator=g, device="cuda") * scale_w
+    x[7] = 0.0
+    ref = x.double() @ w.double().T
+    off = [_off(y, ref) for y in (ops.gemm_fp32_tc(x, w, splits=splits), ops.gemm_generic(
+        x, w.unsqueeze(0), None, None, dual=False))]
+    # a result that is itself subnormal carries 2^-150 of rounding in any order of sums
+    floor = 2.0 ** -150 * ref.numel() ** 0.5 / float(ref.norm())
+    assert off[0] <= max(off[1], 2.0 ** -22, 4 * floor), off
+
+
+def test_sums_that_overflow_in_another_order():
+    """What cancels in ascending k may pass infinity where products of 64 k are added together."""
+    ops = _ops()
+    x = torch.ones(20, 512, device="cuda")
+    w = torch.zeros(24, 512, device="cuda")
+    w[:, 0:512:4], w[:, 1:512:4] = 3e38, -3e38
+    w[3, 2] = 1.0
+    ref = ops.gemm_generic(x, w.unsqueeze(0), None, None, dual=False)
+    for splits in (1, 2):
+        got = ops.gemm_fp32_tc(x, w, splits=splits)
+        assert got.isfinite().all() == ref.isfinite().all()
+    ops.check_async_errors()
