@@ -278,7 +278,7 @@ def linear_act(x: torch.Tensor, w: torch.Tensor, activation: str):
         return gemm_small_m(x, w.unsqueeze(0), None, None, False, M, rows_per_pass=M,
                             activation=activation)
     if x.dtype == torch.float32:
-        if _splits_fp32(x, w):
+        if _splits_fp32(x, w) and _fp32_tc_pays(x.shape[0], w.shape[0], x.shape[1]):
             return gemm_fp32_tc(x, w, activation)
         return gemm_generic(x, w.unsqueeze(0), None, None, dual=False, activation=activation)
     y = linear(x, w)
@@ -304,7 +304,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = 
         if out_dtype == torch.bfloat16:
             return torch.mm(x, w.t())
         return torch.mm(x, w.t(), out_dtype=out_dtype)
-    if out_dtype == torch.float32 and _splits_fp32(x, w):
+    if out_dtype == torch.float32 and _splits_fp32(x, w) and _fp32_tc_pays(M, w.shape[0], K):
         return gemm_fp32_tc(x, w)
     return gemm_generic(x, w.unsqueeze(0), None, None, dual=False, out_dtype=out_dtype)
 
@@ -313,8 +313,18 @@ USE_FP32_TC = True
 # Fewer rows stream the weights past the CUDA cores (gemm_generic's rows kernel, bound by
 # reading them).  Above, that kernel's tiles are bound by the FFMA rate (us, tiles / this form):
 # 17 rows of 2048 x 2048 161 / 28, 600 rows of 11264 x 2048 794 / 175, 17 rows of 5632 x 1024
-# 85 / 29, 64 x 64 x 64 13 / 16.5.
+# 85 / 29.
 FP32_TC_MIN_ROWS = 17
+# This form has some 11 us to begin and end with, whatever the sizes: short inner sizes stay with
+# the tiles (us, tiles / this form, N 4096: 64 rows K 64 7.8 / 12.7, 128 12.8 / 13.9, 192 17.8 /
+# 15.2; 600 rows K 64 18.2 / 25.4, 96 24.1 / 27.7, 128 30.5 / 27.8).
+FP32_TC_MIN_K, FP32_TC_MIN_K_FEW_ROWS, FP32_TC_FEW_ROWS = 128, 160, 64
+
+
+def _fp32_tc_pays(rows: int, cols: int, k: int) -> bool:
+    """Whether a product that ``_splits_fp32`` takes is faster so, and within the kernel's grid."""
+    least = FP32_TC_MIN_K_FEW_ROWS if rows <= FP32_TC_FEW_ROWS else FP32_TC_MIN_K
+    return k >= least and cols <= 65535 * 128
 
 
 def _splits_fp32(x: torch.Tensor, w: torch.Tensor) -> bool:

@@ -105,3 +105,11 @@ def test_sums_that_overflow_in_another_order():
         got = ops.gemm_fp32_tc(x, w, splits=splits)
         assert got.isfinite().all() == ref.isfinite().all()
     ops.check_async_errors()
+
+
+def test_short_inner_sizes_stay_on_the_cuda_cores():
+    ops = _ops()
+    for rows, k in ((33, 64), (64, 128), (130, 96)):
+        x, w = torch.randn(rows, k, device="cuda"), torch.randn(48, k, device="cuda")
+        plain = ops.gemm_generic(x, w.unsqueeze(0), None, None, dual=False)
+        assert torch.equal(ops.linear(x, w), plain)

@@ -168,6 +168,16 @@ def test_fp32_runs_are_never_empty(M, N, K):
     assert 1 <= splits <= 16 and per * (splits - 1) < steps
 
 
+@pytest.mark.parametrize("rows,cols,k,pays", [
+    (17, 2048, 2048, True), (600, 11264, 2048, True), (64, 4096, 192, True), (600, 4096, 128, True),
+    # the tiles on the CUDA cores are ahead
+    (64, 64, 64, False), (64, 4096, 128, False), (600, 4096, 96, False), (2048, 11264, 64, False),
+    (17, 8, 8, False),
+    (17, 65535 * 128 + 1, 2048, False)])              # columns beyond its grid
+def test_fp32_products_take_the_faster_form(rows, cols, k, pays):
+    assert ops._fp32_tc_pays(rows, cols, k) is pays
+
+
 @pytest.mark.parametrize("entry", ["ix_delta_recurrence_segments", "ix_linear_recurrence_segments"])
 def test_segments_cover_the_longest_sequence(entry):
     f = getattr(library.load(), entry)
