@@ -448,6 +448,8 @@ def fp32_points(cfg, batch, context, hbm_peak):
                                                 / hbm_peak, 4),
         "fp32_prefill_2048": round(2048 / (pms / 1e3), 1),
         "fp32_prefill_2048_ms": round(pms, 2),
+        # useful operations against the CUDA cores' rate; most products run on the tensor cores, in
+        # six bfloat16 products each, so this may pass 1
         "fp32_prefill_2048_ffma_frac": round(fl / (pms / 1e3) / peak, 4),
         "fp32_ffma_peak_tflops": round(peak / 1e12, 1),
         "fp32_library_gemms": lib,

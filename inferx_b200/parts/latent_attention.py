@@ -14,9 +14,9 @@ are the latents themselves, and the head's output ``sum_j p_j c_j`` is widened b
 ``W_uv[h]`` afterwards.  That is the form for a few queries per sequence: a pair costs the
 latent's size instead of a head's.  Prompt portions of enough tokens (decided by the shape
 of the step) widen the records they can see once and attend over keys and values of the head's
-own size, keys in two bfloat16 terms.  Queries carry ``dim`` plain and ``rot_dim`` rotated entries per head;
-an optional sigmoid gate computed from the mixer's input multiplies the heads' outputs
-before the output projection.
+own size, keys in two bfloat16 terms.  Queries carry ``dim`` plain and ``rot_dim`` rotated
+entries per head; an optional sigmoid gate computed from the mixer's input multiplies the heads'
+outputs before the output projection.
 
 The projections that read the input (query, down-projection, gate) are one product over
 concatenated weights; the per-head products are library calls batched over heads.
