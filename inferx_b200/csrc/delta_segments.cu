@@ -16,11 +16,12 @@
 // In local and walk lanes share columns of the state, in registers (segments.cuh): a token's two
 // sums over the key's entries are met by shuffles inside the warp, and warps meet once per 16
 // tokens.  Multiplies and adds are packed, two to an instruction; the chunks arrive by cp.async,
-// two buffers.  By count, the arithmetic (four multiply-adds an entry and token, 1.5 times in local
-// for the transitions) and shared-memory reads take about as long.  Measured (B200, 16 heads of
-// 64 x 128, 2,048 tokens): walks whose eight warps were slices of the key that met at a barrier for
-// every token, and that made the unit vectors once per column tile, took 595 us for both passes,
-// these four 216 us (32 heads 1,104 and 384, 8 heads 477 and 158, 256 tokens 144 and 59).
+// two buffers.  What bounds them is a token's chain of sums, shuffles and updates with four to five
+// warps a scheduler (2.1 instructions a cycle of 4; FMA pipe 34 %, shared memory 40 %).  Measured
+// (B200, 16 heads of 64 x 128, 2,048 tokens): walks whose eight warps were slices of the key that
+// met at a barrier for every token, and that made the unit vectors once per column tile, took 595
+// us for both passes, these four 216 us (32 heads 1,104 and 384, 8 heads 477 and 158, 256 tokens
+// 144 and 59).
 #include "segments.cuh"
 
 // ---------------------------------------------------------------------------

@@ -13,10 +13,11 @@
 // All of it is fp32, as in the walk from end to end, and differs from it by rounding only.
 //
 // Lanes and columns, packed arithmetic and the chunks' copies are laid out as in delta_segments.cu
-// (segments.cuh); by count, the arithmetic takes longest (three multiply-adds an entry and token, two
-// in local).  Walks whose eight warps were slices of the key over 32 shared columns took 243 us for
-// the two passes over 2,048 tokens of 16 heads of 64 x 128, 261 with the bonus, these four
-// 111 and 125 (32 heads 472 and 217, 8 heads 161 and 67, 256 tokens 49 and 32).
+// (segments.cuh); what bounds the walks is a token's chain with four to five warps a scheduler (2
+// instructions a cycle of 4; FMA pipe 31 %, shared memory 40 to 47 %).  Walks whose eight warps were
+// slices of the key over 32 shared columns took 243 us for the two passes over 2,048 tokens of 16
+// heads of 64 x 128, 261 with the bonus, these four 111 and 125 (32 heads 472 and 217, 8 heads 161
+// and 67, 256 tokens 49 and 32).
 #include "segments.cuh"
 
 // ---------------------------------------------------------------------------

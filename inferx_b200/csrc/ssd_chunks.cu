@@ -12,9 +12,10 @@
 // a sequence's chunks: the scratch entry becomes the chunk's start state), out (every token's y).
 // The walk takes a token's 3 K V multiply-adds a head one token after the other, and its segments
 // side by side are bound by the FFMA and shared-memory rate (2,048 tokens, 32 heads of 128 x 64:
-// 144 + 311 us for its two passes, 92 us for these three).  Chunks do the same sums as products;
-// what bounds them is the scratch of a chunk's states (K V fp32 a head, written twice and read
-// twice through L2).
+// 144 + 311 us for its two passes, 92 us for these three).  Chunks do the same sums as products.
+// What bounds them is how few warps an SM holds (8 in out, by shared memory) between stages that
+// wait for one another: tensor pipe 16 %, L2 at 9 to 26 % with the chunks' states (K V fp32 a head,
+// written twice and read twice).
 //
 // Nothing of 32 bits is narrowed: x, B and C enter the products as they are (bfloat16), and what is
 // fp32 (weighted inputs, weighted scores, start states) as three bfloat16 terms, 24 bits, small
