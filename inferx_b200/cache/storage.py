@@ -81,6 +81,10 @@ class CacheStorage:
     def zero_slots(self, slots) -> None:
         if not slots:
             return
+        if self.device.type == "cuda":
+            from ..kernels import ops
+            ops.zero_slots([t for per in self.state.values() for t in per.values()], list(slots))
+            return
         idx = torch.tensor(list(slots), dtype=torch.long, device=self.device)
         for per in self.state.values():
             for t in per.values():

@@ -1241,6 +1241,24 @@ def gather_rows(x: torch.Tensor, rows: torch.Tensor):
     return out
 
 
+def zero_slots(tensors: Sequence[torch.Tensor], slots: Sequence[int]) -> None:
+    """Zero ``t[slot]`` of every state tensor ``[slots, ...]``: nothing is copied to the
+    device and nothing waits for it."""
+    for t in tensors:
+        _chk("state", t)
+        if slots and not (0 <= min(slots) and max(slots) < t.shape[0]):
+            raise KernelError(f"zero_slots: a slot of {list(slots)} is outside 0..{t.shape[0] - 1}")
+    tensors = [t for t in tensors if t.numel()]
+    if not tensors or not slots:
+        return
+    n, m = len(tensors), len(slots)
+    bases = (ctypes.c_ulonglong * n)(*[t.data_ptr() for t in tensors])
+    sizes = (ctypes.c_ulonglong * n)(*[t.stride(0) * t.element_size() for t in tensors])
+    _check(_lib().ix_zero_slots(bases, sizes, n, (ctypes.c_int * m)(*[int(s) for s in slots]), m,
+                                _stream()), "zero_slots")
+    _count()
+
+
 _TC_STATUS = {}
 
 

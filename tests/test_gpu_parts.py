@@ -152,6 +152,23 @@ def _step_context(ctx, mixer, tokens_per_seq, page=4):
     return step, ex.caches[0]
 
 
+@pytest.mark.parametrize("slots", [[2], [0, 3, 3], list(range(1, 70))])
+def test_slots_of_new_requests_start_from_zero(slots):
+    """State of sixteen-byte, odd and block-crossing sizes, more tensors and slots than one
+    launch takes; other slots keep theirs."""
+    from inferx_b200.kernels import ops
+    shapes = [(4,), (1,), (3, 5), (64, 128), (64, 65)] * 6
+    state = [torch.ones((71,) + s, dtype=(torch.float32, torch.bfloat16, torch.int32)[i % 3],
+                        device="cuda") for i, s in enumerate(shapes)]
+    ops.zero_slots(state, slots)
+    for t in state:
+        want = torch.ones_like(t)
+        want[slots] = 0
+        assert torch.equal(t, want)
+    with pytest.raises(ops.KernelError, match="slot"):
+        ops.zero_slots(state, [71])
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("heads,kvh,hd,window,bias", [(4, 2, 16, 0, True), (3, 1, 32, 5, False),
                                                       (2, 2, 64, 0, True)])
