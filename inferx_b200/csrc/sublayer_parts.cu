@@ -168,6 +168,39 @@ __global__ void group_norm_add_vec_kernel(float* __restrict__ resid, const TD* _
   }
 }
 
+// Parts of at most 256 entries: a warp a part, eight parts a block, a part's values read once and
+// all reads on their way before the sum (the same sums as above: a lane holds one piece of 8).
+// 3,000 tokens of 8 parts of 256, fp32: 10.2 us (7.3 TB/s, the stream partly in L2) against 25.4
+// with a block of one warp a part, whose 24,000 launches of blocks bounded it.
+#define GN_WARPS 8
+template <typename TD, bool CAST>
+__global__ void __launch_bounds__(GN_WARPS * 32)
+group_norm_add_warp_kernel(float* __restrict__ resid, const TD* __restrict__ delta,
+                           const float* __restrict__ gain, bf16* __restrict__ cast, int parts,
+                           int groups, int part, float eps) {
+  IX_PDL_WAIT();
+  const int i = blockIdx.x * GN_WARPS + (threadIdx.x >> 5), c = (threadIdx.x & 31) * 8;
+  if (i >= parts) return;
+  const size_t base = (size_t)i * part;
+  const bool mine = c < part;
+  float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, r[8], w[8];
+  if (mine) {
+    Load8<TD>::at(delta + base + c, f);
+    Load8<float>::at(resid + base + c, r);
+    Load8<float>::at(gain + (size_t)(i % groups) * part + c, w);
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+  const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)part + eps);
+  if (!mine) return;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) r[j] += f[j] * inv * w[j];
+  *reinterpret_cast<float4*>(resid + base + c) = make_float4(r[0], r[1], r[2], r[3]);
+  *reinterpret_cast<float4*>(resid + base + c + 4) = make_float4(r[4], r[5], r[6], r[7]);
+  if (CAST) *reinterpret_cast<uint4*>(cast + base + c) = f32_to_bf8(r);
+}
+
 template <typename TA>
 __global__ void group_norm_rows_kernel(const float* __restrict__ resid, const int* __restrict__ rows,
                                        const float* __restrict__ gain, TA* __restrict__ out, int W,
@@ -202,13 +235,21 @@ IX_API int ix_group_norm_add(float* resid, const void* delta, int delta_dtype, c
     int th = 32;
     while (th < 256 && th * 8 < part) th *= 2;
     const dim3 vgrid(T, groups), vblock(th);
+    const long long parts = (long long)T * groups;
+    const bool warps = part <= 256 && parts <= 0x7fffffffLL;
 #define IX_GNV(TD, CAST)                                                                       \
-  ix_launch(group_norm_add_vec_kernel<TD, CAST>, vgrid, vblock, 0, stream, resid,                \
+  if (warps)                                                                                   \
+    ix_launch(group_norm_add_warp_kernel<TD, CAST>,                                            \
+              dim3((unsigned)((parts + GN_WARPS - 1) / GN_WARPS)), dim3(GN_WARPS * 32), 0,     \
+              stream, resid, (const TD*)delta, gain, (bf16*)cast, (int)parts, groups, part,    \
+              eps);                                                                            \
+  else                                                                                         \
+    ix_launch(group_norm_add_vec_kernel<TD, CAST>, vgrid, vblock, 0, stream, resid,                \
             (const TD*)delta, gain, (bf16*)cast, W, part, eps)
     if (delta_dtype == IX_F32) {
-      if (cast) IX_GNV(float, true); else IX_GNV(float, false);
+      if (cast) { IX_GNV(float, true); } else { IX_GNV(float, false); }
     } else if (delta_dtype == IX_BF16) {
-      if (cast) IX_GNV(bf16, true); else IX_GNV(bf16, false);
+      if (cast) { IX_GNV(bf16, true); } else { IX_GNV(bf16, false); }
     } else {
       return IX_ERR_DTYPE;
     }
