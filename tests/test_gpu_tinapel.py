@@ -203,6 +203,20 @@ def test_lowrank_decay(dtype, T, C, R):
         assert float(out.min()) >= 0.0 and float(out.max()) <= 1.0
 
 
+@pytest.mark.parametrize("R", [7, 36, 64])
+def test_lowrank_decay_of_many_tokens(R):
+    """Sixteen tokens a block instead of four, weights read ahead and the entries after them:
+    the same sums, so a token's row does not depend on how many come with it."""
+    g = torch.Generator().manual_seed(R)
+    x = torch.randn(301, R, generator=g).to(torch.bfloat16)
+    w2, b = torch.randn(R, 4096, generator=g), torch.randn(4096, generator=g) * 2.0
+    ref = host_ops.lowrank_decay(x, w2, b, "exp_exp_tanh", 1.0)
+    out = _ops().lowrank_decay(x.cuda(), w2.cuda(), b.cuda(), "exp_exp_tanh", 1.0)
+    torch.testing.assert_close(out.cpu(), ref, rtol=2e-5, atol=2e-6)
+    few = _ops().lowrank_decay(x.cuda()[290:], w2.cuda(), b.cuda(), "exp_exp_tanh", 1.0)
+    assert torch.equal(few, out[290:])
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("H,K,V", [(3, 8, 12), (2, 64, 64), (1, 40, 24), (5, 7, 7), (2, 128, 96),
                                    (4, 3, 5), (1, 200, 33)])
