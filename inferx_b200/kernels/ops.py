@@ -2417,7 +2417,7 @@ def ssd_recurrence(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tenso
         _ptr(xbc), ctypes.c_longlong(ld), _ptr(dt_raw), ctypes.c_longlong(ld_dt),
         _dtype_code(xbc), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), _ptr(step.cu_q),
         _ptr(step.state_slot), _ptr(out), walked, heads, vdim, nstate, groups, seg_len,
-        nseg, _ptr(scratch), _stream()), "ssd_recurrence")
+        nseg, _ptr(scratch), 1 if walked <= singles else 0, _stream()), "ssd_recurrence")
     _count(2 if nseg > 1 else 1)
     return out
 
@@ -2496,7 +2496,9 @@ def delta_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta_raw
     if walked:
         _check(_lib().ix_delta_recurrence(
             *views(0), walked, heads, kv_heads, dim, vdim, ctypes.c_float(unit_eps),
-            ctypes.c_float(q_scale), _stream()), "delta_recurrence")
+            ctypes.c_float(q_scale),
+            1 if walked <= int(getattr(step, "num_decode_seqs", 0) or 0) else 0, _stream()),
+            "delta_recurrence")
         _count()
     if nseg > 1:
         size = _lib().ix_delta_segments_scratch_floats

@@ -650,3 +650,32 @@ def test_greedy_generation_through_the_engine(tmp_path):
             assert tok == int(lg.argmax()) or float(top[0] - top[1]) < 1e-4 * float(lg.abs().max())
             seq.append(tok)
         assert len(c_out.output_tokens) == 12
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("K,V", [(64, 128), (128, 64), (64, 16), (128, 256), (64, 256)])
+def test_single_tokens_give_the_walk_s_bits(dtype, K, V):
+    """A batch of single tokens (``num_decode_seqs`` covers it) takes the kernels that hold a whole
+    head's state; told nothing, the walk.  States of other slots stay."""
+    S, H, HK, G = 5, 4, 2, 2
+    g = torch.Generator().manual_seed(K + V)
+
+    def rand(*shape):
+        return torch.randn(shape, generator=g)
+    step = _cuda(_step([1] * S, [7, 0, 3, 1, 9], slots=[6, 0, 2, 5, 1]))
+    xbc, dt = rand(S, H * V + 2 * G * K).to(dtype).cuda(), rand(S, H + 3).to(dtype).cuda()[:, 1:H + 1]
+    per_head = [rand(H).cuda() for _ in range(3)]
+    q, k = (rand(S, HK * K).to(dtype).cuda() for _ in range(2))
+    v, beta = rand(S, H * V).to(dtype).cuda(), rand(S, H).to(dtype).cuda()
+    decay = torch.rand(S, H * K, generator=g).cuda()
+    state = rand(8, H, K, V).cuda()
+    got = []
+    for singles in (0, S):
+        step.num_decode_seqs = singles
+        a, b = state.clone(), state.clone()
+        got.append((_ops().ssd_recurrence(xbc, dt, *per_head, a, step, H, V, K, G), a,
+                    _ops().delta_recurrence(q, k, v, beta, decay, b, step, H, HK, K, V, 1e-6,
+                                            K ** -0.5), b))
+    for walk, single in zip(*got):
+        assert torch.equal(walk, single)
+    assert torch.equal(got[1][1][3], state[3]) and not torch.equal(got[1][1][6], state[6])
