@@ -274,6 +274,14 @@ paged_attention_tiled_kernel(const TA* __restrict__ q, const TA* __restrict__ kc
   }
 }
 
+// attention_fp32_mma.cu
+bool ix_attention_fp32_mma_applies(int hd, int vd);
+int ix_attention_fp32_mma(const float* q, const float* k_cache, const float* v_cache,
+                          const int* block_table, const int* cu_q, const int* q_pos0, float* out,
+                          int T, int S, int heads, int kvh, int hd, int vd, int page_size,
+                          int max_blocks, int window, float scale, float softcap, int keep_first,
+                          const IxRows& rows, cudaStream_t stream);
+
 IX_API int ix_paged_attention_tiled_applies(int hd) { return hd > 0 && hd % 4 == 0 && hd <= 256; }
 
 // q: [T, heads, hd]; out: [T, heads, vd]; caches [pages, kvh, page_size, hd or vd];
@@ -296,6 +304,11 @@ static int tiled_checked(const void* q, const void* k_cache, const void* v_cache
   if (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)out) % (4 * esize))
     return IX_ERR_ALIGN;
   if (rows.q_ld % 4 || rows.o_ld % 4) return IX_ERR_ALIGN;
+  if (act_dtype == IX_F32 && !dist.temp && ix_attention_fp32_mma_applies(hd, vd))
+    return ix_attention_fp32_mma((const float*)q, (const float*)k_cache, (const float*)v_cache,
+                                 block_table, cu_q, q_pos0, (float*)out, T, S, heads, kvh, hd, vd,
+                                 page_size, max_blocks, window, scale, softcap, keep_first, rows,
+                                 stream);
   const int ld = hd + 4, ldv = vd + 4;
   const size_t smem = ((size_t)(TA_BQ + TA_BK) * ld + (size_t)TA_BK * ldv + TA_BQ * (TA_BK + 4) +
                        3 * TA_BQ) * 4;
