@@ -151,7 +151,8 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
   const int n_tiles = (pmax + 1 - kt0 + WA_BN - 1) / WA_BN;
   // the first query tile of two ends its walk with its own last position
   const int n_first = (min(pmax, pos0 + WA_BM - 1) + 1 - kt0 + WA_BN - 1) / WA_BN;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
 
   if ((smem_u32(smem) & 1023u) != 0) {
     if (tid == 0) atomicExch(status, WA_ERR_ALIGN);
@@ -185,10 +186,13 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const unsigned tmem_base = bars->tmem_holder;
+  const unsigned tmem_base = __shfl_sync(0xffffffffu, bars->tmem_holder, 0);
   volatile int* abortp = &bars->abort_flag;
   int copied = 0;                        // tiles whose copies this thread started (warps 0 and 2)
 
+  // The copying warps walk the tiles whole too, one lane issuing, so that coordinates stay in
+  // uniform registers; with that and with one load of a row's 64 scores, 3,000 queries of 16 heads
+  // take 104 us instead of 130, 1,500 of 32 heads 56 instead of 69.
   if (warp == 0) {
     if (lane == 0) {
       mbar_expect_tx(&bars->q_full, halves * Q_BYTES);
@@ -197,12 +201,16 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
         for (int p = 0; p < KP; ++p)
           tma_load_2d(Qs + t * Q_BYTES + p * Q_PANEL, &map_q, h * DK + p * 64,
                       tok0 + q0 + t * WA_BM, &bars->q_full);
-      const int row0 = s * rows_per_seq + (kt0 - base);
-      bool ok = true;
-      for (int j = 0; j < n_tiles; ++j) {
-        const int st = j % WA_STAGES, row = row0 + j * WA_BN;
-        ok = mbar_wait(&bars->k_empty[st], ((j / WA_STAGES) & 1) ^ 1, abortp);
-        if (!ok) break;
+    }
+    __syncwarp();
+    const int row0 = __shfl_sync(0xffffffffu, s * rows_per_seq + (kt0 - base), 0);
+    bool ok = true;
+    for (int j = 0; j < n_tiles; ++j) {
+      const int st = j % WA_STAGES, row = row0 + j * WA_BN;
+      ok = __all_sync(0xffffffffu,
+                      mbar_wait(&bars->k_empty[st], ((j / WA_STAGES) & 1) ^ 1, abortp));
+      if (!ok) break;
+      if (lane == 0) {
         mbar_expect_tx(&bars->k_full[st], K_TILE);
 #pragma unroll
         for (int p = 0; p < KP; ++p)
@@ -212,27 +220,30 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
         for (int p = 0; p < LP; ++p)
           tma_load_2d(Ks + st * K_TILE + K_LO + p * PANEL, &map_kv,
                       heads * DK + (h * LP + p) * 64, row, &bars->k_full[st]);
-        copied = j + 1;
       }
-      if (!ok && !*abortp) { atomicExch(status, WA_ERR_COPY); *abortp = 1; }
+      __syncwarp();
+      copied = j + 1;
     }
+    if (!ok && lane == 0 && !*abortp) { atomicExch(status, WA_ERR_COPY); *abortp = 1; }
   } else if (warp == 2) {
-    if (lane == 0) {
-      const int row0 = s * rows_per_seq + (kt0 - base);
-      bool ok = true;
-      for (int j = 0; j < n_tiles; ++j) {
-        const int st = j % WA_STAGES, row = row0 + j * WA_BN;
-        ok = mbar_wait(&bars->v_empty[st], ((j / WA_STAGES) & 1) ^ 1, abortp);
-        if (!ok) break;
+    const int row0 = __shfl_sync(0xffffffffu, s * rows_per_seq + (kt0 - base), 0);
+    bool ok = true;
+    for (int j = 0; j < n_tiles; ++j) {
+      const int st = j % WA_STAGES, row = row0 + j * WA_BN;
+      ok = __all_sync(0xffffffffu,
+                      mbar_wait(&bars->v_empty[st], ((j / WA_STAGES) & 1) ^ 1, abortp));
+      if (!ok) break;
+      if (lane == 0) {
         mbar_expect_tx(&bars->v_full[st], V_TILE);
 #pragma unroll
         for (int p = 0; p < VP; ++p)
           tma_load_2d(Vs + st * V_TILE + p * PANEL, &map_kv,
                       heads * (DK + LP * 64) + h * DV + p * 64, row, &bars->v_full[st]);
-        copied = j + 1;
       }
-      if (!ok && !*abortp) { atomicExch(status, WA_ERR_COPY); *abortp = 1; }
+      __syncwarp();
+      copied = j + 1;
     }
+    if (!ok && lane == 0 && !*abortp) { atomicExch(status, WA_ERR_COPY); *abortp = 1; }
   } else if (warp == 1) {
     // The whole warp walks the tiles and one lane issues: where descriptors are the warp's and not a
     // thread's they stay in uniform registers.  (One lane alone took some 130 cycles an MMA.)
@@ -319,8 +330,7 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
       tc_fence_after();
       const unsigned s_addr = lane_addr + S_COL + (2 * t + (j & 1)) * WA_BN;
       float sc[WA_BN];
-      tc_ld32(s_addr, sc);
-      tc_ld32(s_addr + 32, sc + 32);
+      tc_ld64(s_addr, sc);
       const int kbase = kt0 + j * WA_BN;
       if (kbase + WA_BN - 1 > tile_pos0 || kbase < lo_last) {
 #pragma unroll
