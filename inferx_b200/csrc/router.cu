@@ -419,17 +419,42 @@ __global__ void __launch_bounds__(ROUTER_THREADS)
 router_logits_bf16_vec_kernel(const bf16* __restrict__ x, const float* __restrict__ w,
                               const float* __restrict__ extra_w, int T, int H, int E,
                               float* __restrict__ logits, float* __restrict__ extra_out) {
-  IX_PDL_WAIT();
+  // A lane's first weights are on their way before the wait for the preceding kernel, which
+  // does not write them; behind it only the activations have to arrive.
+  constexpr int AHEAD = 8;
   const int lane = threadIdx.x & 31;
   const int pair = blockIdx.x * (ROUTER_THREADS / 32) + (threadIdx.x >> 5);
   const int rows_total = E + (extra_w ? 1 : 0);
-  if (pair >= T * rows_total) return;
-  const int t = pair / rows_total, e = pair - t * rows_total;
+  const bool mine = pair < T * rows_total;
+  const int t = mine ? pair / rows_total : 0, e = mine ? pair - t * rows_total : 0;
   const float4* wr = reinterpret_cast<const float4*>(e < E ? w + (size_t)e * H : extra_w);
   const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)t * H);
   const int chunks = H >> 3;
+  float4 wa[AHEAD], wb[AHEAD];
+#pragma unroll
+  for (int i = 0; i < AHEAD; ++i) {
+    const int c = lane + 32 * i;
+    if (mine && c < chunks) {
+      wa[i] = wr[2 * c];
+      wb[i] = wr[2 * c + 1];
+    }
+  }
+  IX_PDL_WAIT();
+  if (!mine) return;
   float acc = 0.f;
-  for (int c = lane; c < chunks; c += 32) {
+  uint4 xa[AHEAD];
+#pragma unroll
+  for (int i = 0; i < AHEAD; ++i)
+    if (lane + 32 * i < chunks) xa[i] = xr[lane + 32 * i];
+#pragma unroll
+  for (int i = 0; i < AHEAD; ++i) {
+    if (lane + 32 * i < chunks) {
+      float xf[8];
+      bf8_to_f32(xa[i], xf);
+      dot8(acc, xf, wa[i], wb[i]);
+    }
+  }
+  for (int c = lane + 32 * AHEAD; c < chunks; c += 32) {
     float xf[8];
     bf8_to_f32(xr[c], xf);
     dot8(acc, xf, wr[2 * c], wr[2 * c + 1]);
@@ -479,6 +504,28 @@ router_select_kernel(const float* __restrict__ logits, int E, int k, int renorm,
                  topk_idx + (size_t)t * k, lane);
 }
 
+static bool router_vec(const void* x, const float* w, const float* extra_w, int act_dtype, int H) {
+  return act_dtype == IX_BF16 && H % 8 == 0 &&
+         (((uintptr_t)x | (uintptr_t)w | (uintptr_t)extra_w) & 15) == 0;
+}
+
+// logits: [T, E] fp32
+static int router_few_logits(const void* x, const float* w, const float* extra_w, int act_dtype,
+                             int T, int H, int E, float* logits, float* extra_out,
+                             cudaStream_t stream) {
+  const long long pairs = (long long)T * (E + (extra_w ? 1 : 0));
+  const int blocks = (int)((pairs + ROUTER_THREADS / 32 - 1) / (ROUTER_THREADS / 32));
+  if (router_vec(x, w, extra_w, act_dtype, H)) {
+    ix_launch(router_logits_bf16_vec_kernel, dim3(blocks), dim3(ROUTER_THREADS), 0, stream,
+              (const bf16*)x, w, extra_w, T, H, E, logits, extra_out);
+    return ix_launch_status();
+  }
+  IX_DISPATCH_DTYPE(act_dtype, TA,
+                    (ix_launch(router_logits_kernel<TA>, dim3(blocks), dim3(ROUTER_THREADS), 0,
+                               stream, (const TA*)x, w, extra_w, T, H, E, logits, extra_out)));
+  return ix_launch_status();
+}
+
 // Sizes beyond which the router and dispatch kernels refuse a call; a model is checked
 // against them when it is built.
 IX_API int ix_router_max_topk() { return ROUTER_MAX_TOPK; }
@@ -524,26 +571,10 @@ static int router_topk_impl(const void* x, const float* w, const float* extra_w,
   if (T <= 0) return IX_OK;
   if (H <= 0 || E <= 0 || k <= 0 || k > E || k > ROUTER_MAX_TOPK) return IX_ERR_SIZE;
   if (extra_w && !extra_out) return IX_ERR_SIZE;
-  const bool vec = act_dtype == IX_BF16 && H % 8 == 0 &&
-                   (((uintptr_t)x | (uintptr_t)w | (uintptr_t)extra_w) & 15) == 0;
+  const bool vec = router_vec(x, w, extra_w, act_dtype, H);
   if (logits_scratch && (size_t)E * sizeof(float) <= 48 * 1024) {   // the caller's choice
-    // logits_scratch: [T, E] fp32
-    const long long pairs = (long long)T * (E + (extra_w ? 1 : 0));
-    const int blocks = (int)((pairs + ROUTER_THREADS / 32 - 1) / (ROUTER_THREADS / 32));
-    if (vec) {
-      ix_launch(router_logits_bf16_vec_kernel, dim3(blocks), dim3(ROUTER_THREADS), 0, stream,
-                (const bf16*)x, w, extra_w, T, H, E, logits_scratch, extra_out);
-      int rc = ix_launch_status();
-      if (rc != 0) return rc;
-      ix_launch(router_select_kernel, dim3(T), dim3(32), (size_t)E * sizeof(float), stream,
-                (const float*)logits_scratch, E, k, renorm, scale, topk_w, topk_idx, rule);
-      return ix_launch_status();
-    }
-    IX_DISPATCH_DTYPE(act_dtype, TA,
-                      (ix_launch(router_logits_kernel<TA>, dim3(blocks), dim3(ROUTER_THREADS), 0,
-                                 stream, (const TA*)x, w, extra_w, T, H, E, logits_scratch,
-                                 extra_out)));
-    int rc = ix_launch_status();
+    const int rc = router_few_logits(x, w, extra_w, act_dtype, T, H, E, logits_scratch, extra_out,
+                                     stream);
     if (rc != 0) return rc;
     ix_launch(router_select_kernel, dim3(T), dim3(32), (size_t)E * sizeof(float), stream,
               (const float*)logits_scratch, E, k, renorm, scale, topk_w, topk_idx, rule);
@@ -678,6 +709,38 @@ moe_dispatch_kernel(const int* __restrict__ topk_idx, int A, int E, int k,
   dispatch_in_block(topk_idx, A, E, k, offsets, rows, dest, counts, topk_w, row_w);
 }
 
+// A few tokens: selection (a warp a token) and dispatch tables in one block, one launch and one
+// boundary of dependent kernels less than router_select_kernel followed by moe_dispatch_kernel,
+// whose results these are.
+#define ROUTER_CHOOSE_MAX_TOKENS 32
+#define ROUTER_CHOOSE_MAX_BYTES (48 * 1024)
+
+__global__ void __launch_bounds__(1024)
+router_choose_kernel(const float* __restrict__ logits, int T, int E, int k, int renorm,
+                     float scale, float* __restrict__ topk_w, int* __restrict__ topk_idx,
+                     RouteRule rule, int* __restrict__ offsets, int* __restrict__ rows,
+                     int* __restrict__ dest, float* __restrict__ row_w) {
+  extern __shared__ float prob[];                      // [T][E], then [T][k] twice, [E + 1]
+  float* w_s = prob + (size_t)T * E;
+  int* idx_s = reinterpret_cast<int*>(w_s + T * k);
+  int* counts = idx_s + T * k;
+  IX_PDL_WAIT();
+  const int t = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (t < T) {
+    float* p = prob + (size_t)t * E;
+    for (int e = lane; e < E; e += 32) p[e] = logits[(size_t)t * E + e];
+    __syncwarp();
+    select_by_rule(p, E, k, renorm, scale, rule, w_s + t * k, idx_s + t * k, lane);
+    __syncwarp();
+    if (lane < k) {
+      topk_w[(size_t)t * k + lane] = w_s[t * k + lane];
+      topk_idx[(size_t)t * k + lane] = idx_s[t * k + lane];
+    }
+  }
+  __syncthreads();
+  dispatch_in_block(idx_s, T * k, E, k, offsets, rows, dest, counts, w_s, row_w);
+}
+
 // ---------------------------------------------------------------------------
 // Dispatch for many assignments: blocks of 1024 assignments count their experts,
 // one block turns the counts into bases (per block and expert) and offsets, and the
@@ -775,5 +838,41 @@ IX_API int ix_moe_dispatch(const int* topk_idx, int T, int E, int k, int* offset
   const int threads = E >= 32 ? 1024 : 32 * E;
   ix_launch(moe_dispatch_kernel, dim3(1), dim3(threads), (E + 1) * sizeof(int), stream, topk_idx,
             A, E, k, offsets, rows, dest, topk_w, row_w);
+  return ix_launch_status();
+}
+
+static size_t router_choose_bytes(int T, int E, int k) {
+  return ((size_t)T * E + 2 * (size_t)T * k + E + 1) * sizeof(float);
+}
+
+// Whether ix_router_dispatch takes these sizes.
+IX_API int ix_router_dispatch_applies(int T, int E, int k) {
+  return T > 0 && E > 0 && k > 0 && k <= E && k <= ROUTER_MAX_TOPK &&
+         T <= ROUTER_CHOOSE_MAX_TOKENS && router_choose_bytes(T, E, k) <= ROUTER_CHOOSE_MAX_BYTES;
+}
+
+// ix_router_topk_ruled (ruled 0: ix_router_topk) and ix_moe_dispatch of its choice, for a few
+// tokens; the results are theirs.  logits: [T, E] fp32 scratch.
+IX_API int ix_router_dispatch(const void* x, const float* w, const float* extra_w, int act_dtype,
+                              int T, int H, int E, int k, int renorm, float scale, int ruled,
+                              const float* correction, int groups, int keep, float renorm_eps,
+                              int sigmoid, int pair_sum, float* topk_w, int* topk_idx,
+                              float* extra_out, float* logits, int* offsets, int* rows, int* dest,
+                              float* row_w, cudaStream_t stream) {
+  if (!ix_router_dispatch_applies(T, E, k) || H <= 0 || !logits || (extra_w && !extra_out))
+    return IX_ERR_SIZE;
+  RouteRule rule = {nullptr, 0, 0, -1.f, 0, 0, 0};
+  if (ruled) {
+    if (groups < 0 || groups > ROUTER_MAX_GROUPS) return IX_ERR_SIZE;
+    if (groups > 0 && (E % groups != 0 || keep <= 0 || keep > groups ||
+                       (long long)keep * (E / groups) < k))
+      return IX_ERR_SIZE;
+    rule = {correction, groups, keep, renorm_eps, 1, pair_sum, sigmoid};
+  }
+  const int rc = router_few_logits(x, w, extra_w, act_dtype, T, H, E, logits, extra_out, stream);
+  if (rc != 0) return rc;
+  ix_launch(router_choose_kernel, dim3(1), dim3(1024), router_choose_bytes(T, E, k), stream,
+            (const float*)logits, T, E, k, renorm, scale, topk_w, topk_idx, rule, offsets, rows,
+            dest, row_w);
   return ix_launch_status();
 }

@@ -663,6 +663,57 @@ def moe_dispatch(topk_idx: torch.Tensor, num_experts: int,
     return (offsets, rows, dest) if row_w is None else (offsets, rows, dest, row_w)
 
 
+def router_dispatch(x: torch.Tensor, w: torch.Tensor, top_k: int, renormalize: bool, scale: float,
+                    extra_w: Optional[torch.Tensor] = None, row_weights: bool = False,
+                    correction: Optional[torch.Tensor] = None, group_count: int = 0,
+                    group_keep: int = 0, renorm_eps: Optional[float] = None,
+                    score: str = "softmax", group_value: str = "max"):
+    """``router_topk`` and the ``moe_dispatch`` of its choice: (weights, experts, x.extra_w,
+    offsets, rows, dest, weight of every grouped row or None).  A few tokens' choice and tables
+    are made by one block in one launch (decode steps are chains of short kernels)."""
+    T, H = x.shape
+    E = w.shape[0]
+    ruled = (correction is not None or group_count > 0 or score != "softmax"
+             or (renorm_eps is not None and renorm_eps >= 0))
+    if not _lib().ix_router_dispatch_applies(T, E, top_k):
+        tw, ti, ex = router_topk(x, w, top_k, renormalize, scale, extra_w=extra_w,
+                                 correction=correction, group_count=group_count,
+                                 group_keep=group_keep, renorm_eps=renorm_eps, score=score,
+                                 group_value=group_value)
+        tables = moe_dispatch(ti, E, topk_w=tw if row_weights else None)
+        return (tw, ti, ex) + tuple(tables) + (() if row_weights else (None,))
+    _chk("x", x)
+    _chk("w", w, torch.float32)
+    _chk("extra_w", extra_w, torch.float32, optional=True)
+    _chk("correction", correction, torch.float32, optional=True)
+    if w.shape[1] != H or (extra_w is not None and extra_w.numel() != H):
+        raise KernelError("router_dispatch: weight width differs from the activations'")
+    if score not in ("softmax", "sigmoid"):
+        raise KernelError(f"router_dispatch: score {score!r}")
+    if correction is not None and correction.numel() != E:
+        raise KernelError("router_dispatch: one correction per router output")
+
+    def floats(*shape):
+        return torch.empty(shape, dtype=torch.float32, device=x.device)
+
+    def ints(*shape):
+        return torch.empty(shape, dtype=torch.int32, device=x.device)
+    tw, ti = floats(T, top_k), ints(T, top_k)
+    ex = floats(T) if extra_w is not None else None
+    offsets, rows, dest = ints(E + 1), ints(T * top_k), ints(T * top_k)
+    row_w = floats(T * top_k) if row_weights else None
+    logits = floats(T, E)
+    _check(_lib().ix_router_dispatch(
+        _ptr(x), _ptr(w), _ptr(extra_w), _dtype_code(x), T, H, E, top_k, 1 if renormalize else 0,
+        ctypes.c_float(scale), 1 if ruled else 0, _ptr(correction), int(group_count),
+        int(group_keep), ctypes.c_float(-1.0 if renorm_eps is None else renorm_eps),
+        1 if score == "sigmoid" else 0, 1 if group_value == "pair_sum" else 0, _ptr(tw), _ptr(ti),
+        _ptr(ex), _ptr(logits), _ptr(offsets), _ptr(rows), _ptr(dest), _ptr(row_w),
+        _stream()), "router_dispatch")
+    _count(2)
+    return tw, ti, ex, offsets, rows, dest, row_w
+
+
 def moe_combine(y: torch.Tensor, dest: torch.Tensor, topk_w: torch.Tensor,
                 shared: Optional[torch.Tensor], shared_logit: Optional[torch.Tensor],
                 weighted: bool = True):

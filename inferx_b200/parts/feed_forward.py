@@ -315,26 +315,27 @@ class MoeFeedForward:
             side = self._side_stream()
             main = torch.cuda.current_stream(x.device)
             ready = main.record_event()        # x is there; what follows is not waited for
+        rule = {"extra_w": self.shared_gate_w}
         if self.ruled:
-            topk_w, topk_idx, shared_logit = ops.router_topk(
-                x, self.router_w, s.top_k, s.renormalize, s.routed_scale,
-                extra_w=self.shared_gate_w, correction=self.correction,
-                group_count=self.group_count, group_keep=self.group_keep,
-                renorm_eps=self.renorm_eps,
-                **({} if self.score == "softmax" else {"score": self.score}),
-                **({} if self.group_value == "max" else {"group_value": self.group_value}))
-        else:
-            topk_w, topk_idx, shared_logit = ops.router_topk(
-                x, self.router_w, s.top_k, s.renormalize, s.routed_scale,
-                extra_w=self.shared_gate_w)
+            rule.update(correction=self.correction, group_count=self.group_count,
+                        group_keep=self.group_keep, renorm_eps=self.renorm_eps,
+                        **({} if self.score == "softmax" else {"score": self.score}),
+                        **({} if self.group_value == "max" else {"group_value": self.group_value}))
         # identity experts are the router's last outputs: the stable dispatch puts their
         # rows behind every expert's, where no product writes
         row_w = None
-        if self.weight_input:       # the weights travel with the rows into the experts
-            all_offsets, rows, dest, row_w = ops.moe_dispatch(topk_idx, self.outputs,
-                                                              topk_w=topk_w)
+        if hasattr(ops, "router_dispatch"):
+            topk_w, _, shared_logit, all_offsets, rows, dest, row_w = ops.router_dispatch(
+                x, self.router_w, s.top_k, s.renormalize, s.routed_scale,
+                row_weights=self.weight_input, **rule)
         else:
-            all_offsets, rows, dest = ops.moe_dispatch(topk_idx, self.outputs)
+            topk_w, topk_idx, shared_logit = ops.router_topk(
+                x, self.router_w, s.top_k, s.renormalize, s.routed_scale, **rule)
+            if self.weight_input:       # the weights travel with the rows into the experts
+                all_offsets, rows, dest, row_w = ops.moe_dispatch(topk_idx, self.outputs,
+                                                                  topk_w=topk_w)
+            else:
+                all_offsets, rows, dest = ops.moe_dispatch(topk_idx, self.outputs)
         offsets = all_offsets[:s.num_experts + 1] if self.identity else all_offsets
         if ready is not None:
             side.wait_event(ready)

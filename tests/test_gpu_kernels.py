@@ -933,3 +933,31 @@ def test_token_logprobs(R, V, top):
     for r in range(R):
         ref_lp, _ = plain.logprobs(logits[r], int(chosen[r]), 0)
         assert abs(float(lp_all[r]) - ref_lp) <= 2e-5 * max(1.0, abs(ref_lp))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("T,E,k", [(1, 60, 4), (16, 60, 4), (32, 32, 4), (32, 33, 32), (7, 5, 5),
+                                   (3, 400, 2), (1, 1, 1), (33, 60, 4)])
+@pytest.mark.parametrize("rule", ["plain", "groups", "sigmoid", "sigmoid_groups"])
+def test_router_dispatch_is_router_then_dispatch(dtype, T, E, k, rule):
+    """The one-block form gives what the router and the dispatch kernels give one after the
+    other, bit for bit, ties (equal rows of weights) included."""
+    ops = _ops()
+    groups = next(g for g in (4, 3, 5, 1) if E % g == 0)
+    keep = groups - 1 if E // groups * (groups - 1) >= k else groups
+    kw = {"plain": dict(),
+          "groups": dict(correction=_rand((E,), torch.float32, 0.1).cuda(), group_count=groups,
+                         group_keep=keep, renorm_eps=1e-6, group_value="pair_sum"),
+          "sigmoid": dict(score="sigmoid", renorm_eps=0.0),
+          "sigmoid_groups": dict(score="sigmoid", group_count=1, group_keep=1)}[rule]
+    H = 264
+    x, w = _rand((T, H), dtype, seed=T).cuda(), _rand((E, H), torch.float32, 0.2, seed=E).cuda()
+    w[E // 2] = w[0]
+    extra = _rand((H,), torch.float32, seed=3).cuda()
+    tw, ti, ex, off, rows, dest, row_w = ops.router_dispatch(
+        x, w, k, True, 1.5, extra_w=extra, row_weights=True, **kw)
+    tw2, ti2, ex2 = ops.router_topk(x, w, k, True, 1.5, extra_w=extra, **kw)
+    off2, rows2, dest2, row_w2 = ops.moe_dispatch(ti2, E, topk_w=tw2)
+    for a, b in zip((tw, ti, ex, off, rows, dest, row_w), (tw2, ti2, ex2, off2, rows2, dest2, row_w2)):
+        assert torch.equal(a, b)
+    assert ops.router_dispatch(x, w, k, True, 1.5, **kw)[6] is None
