@@ -33,10 +33,13 @@ __global__ void embed_sinusoid_kernel(const TT* __restrict__ table, const int* _
   const TT* row = table + (size_t)ids[t] * W;
   const float p = (float)positions[t];
   float* o = out + (size_t)t * W;
-  for (int i = threadIdx.x; i < W; i += blockDim.x) {
+  // a thread has the sine and the cosine of an angle: by entry, every warp took both ways for each of
+  // its entries, which is what the time went to (1,777 rows of 2,048: 13.2 us, now 7.8; 3,000 of
+  // 4,096: 37.2 and 19.6; one row 5.5 and 3.0)
+  for (int i = 2 * threadIdx.x; i < W; i += 2 * blockDim.x) {
     const float a = p * freq[i >> 1];
-    const float pe = (i & 1) ? cosf(a) : sinf(a);
-    o[i] = to_f32(row[i]) * scale + pe;
+    o[i] = to_f32(row[i]) * scale + sinf(a);
+    if (i + 1 < W) o[i + 1] = to_f32(row[i + 1]) * scale + cosf(a);
   }
 }
 
