@@ -302,6 +302,27 @@ def test_delta_recurrence_in_segments(dtype, H, HK, K, V):
     assert _rel(st2[2].cpu(), st[2].cpu()) <= 2e-5
 
 
+@pytest.mark.parametrize("H,K,V,lens", [(2, 28, 17, (700, 131)), (1, 60, 16, (700,)),
+                                        (13, 64, 128, (300, 1, 260)), (1, 112, 40, (520, 300)),
+                                        (1, 124, 16, (400,)), (2, 66, 20, (300,)),
+                                        (1, 132, 24, (600,))])
+def test_delta_segments_joined_by_every_buffering(H, K, V, lens):
+    """Start states from transitions in four buffers, in two (a row too wide, or more blocks than
+    are resident with four) and read where they are (no whole 16-byte parts, rows above 128)."""
+    g = torch.Generator().manual_seed(H * K + V)
+    T, S = sum(lens), len(lens)
+    step = _step(list(lens), [0] * S, slots=list(range(S))[::-1])
+    q, k = (torch.randn(T, H * K, generator=g).bfloat16() for _ in range(2))
+    v, beta = (torch.randn(T, n, generator=g).bfloat16() for n in (H * V, H))
+    decay = torch.rand(T, H * K, generator=g) * 0.1 + 0.9
+    state = torch.randn(S, H, K, V, generator=g)
+    st = state.cuda()
+    ref = host_ops.delta_recurrence(q, k, v, beta, decay, state, step, H, H, K, V, 1e-6, K ** -0.5)
+    out = _ops().delta_recurrence(*(t.cuda() for t in (q, k, v, beta, decay)), st, _cuda(step), H,
+                                  H, K, V, 1e-6, K ** -0.5)
+    assert _rel(out.cpu(), ref) <= 5e-5 and _rel(st.cpu(), state) <= 5e-5
+
+
 def test_recurrences_do_not_depend_on_the_cut():
     """The same tokens in one step, in portions and one by one, alone and beside another
     sequence: the same bits, in the outputs and in the states."""
