@@ -144,15 +144,6 @@ __device__ __forceinline__ void tc_cluster_sync() {
 __device__ __forceinline__ void tc_arrive_at(unsigned bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// into this block's shared memory, reporting to a barrier of either block
-__device__ __forceinline__ void tc_load_pair(void* dst, const CUtensorMap* map, int x, int y,
-                                             unsigned bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      ".cta_group::2 [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
-      "l"(map), "r"(x), "r"(y), "r"(bar)
-      : "memory");
-}
 __device__ __forceinline__ void tc_mma_pair(unsigned tmem_d, unsigned long long adesc,
                                             unsigned long long bdesc, unsigned idesc,
                                             unsigned accum) {
