@@ -20,8 +20,7 @@
 // warps a scheduler (2.1 instructions a cycle of 4; FMA pipe 34 %, shared memory 40 %).  Measured
 // (B200, 16 heads of 64 x 128, 2,048 tokens): walks whose eight warps were slices of the key that
 // met at a barrier for every token, and that made the unit vectors once per column tile, took 595
-// us for both passes, these four 204 us (32 heads 1,104 and 373, 8 heads 477 and 142, 256 tokens
-// 144 and 55).
+// us for both passes, these four 210 us (8 heads 477 and 148, 256 tokens 144 and 56).
 #include "segments.cuh"
 
 // ---------------------------------------------------------------------------
@@ -255,29 +254,27 @@ delta_segment_kernel(DsIn in, const TA* __restrict__ v, long long ldv, float* __
 
 // ---------------------------------------------------------------------------
 // join: grid (tiles of 16 value columns, heads, sequences).  A segment's own state in scratch gives
-// way to its start state.
+// way to its start state.  An entry is one chain of multiply-adds from the segment's own state on,
+// over the key in ascending order, in every form.
 //
-// STAGES > 0 (K a multiple of 4 up to 128): transitions come into shared memory STAGES - 1 segments
-// ahead and a segment's own state into registers one ahead, so that a step waits for neither.  What
-// is left is the reading of shared memory, 512 bytes of registers for a warp's 16-byte read however
-// few addresses it has: a thread takes four rows by four columns over a quarter of the key (a read
-// for eight multiplies and adds a lane, where one column a thread has a read for three), and the
-// quarters meet in shared memory.  Rows are an odd number of 16-byte parts apart, so that the eight
-// rows of a quarter-warp's read meet no bank twice.  Measured (one column a thread, transitions one
-// segment ahead, own states when their rows were reached, against this): 16 heads of 64 x 128, 2,048
-// tokens 38.5 and 26.9 us, 300 to 1,024 tokens side by side 27.8 and 18.5, 16 heads of 128 x 128,
-// 3,000 tokens 44.1 and 29.6, 64 heads of 64 x 128 (two buffers) 23.6 and 19.9.  Buffers alone were
-// worth 3 us of the first, and none where few heads leave many segments (54.7 and 56.7; now 42.3).
+// STAGES > 0 (K a multiple of 4 up to 128): a warp for every 32 rows makes the sums, the others bring
+// transitions into shared memory STAGES - 1 segments ahead and write the start states out; a
+// segment's own state comes into registers one ahead, so that a step waits for none of them.  What is
+// left is the reading of shared memory, 512 bytes of registers for a warp's 16-byte read however few
+// addresses it has, and the chains: a thread takes four rows by four columns (a read for eight
+// multiplies and adds a lane, where one column a thread has a read for three).  Rows are an odd number
+// of 16-byte parts apart, so that the eight rows of a quarter-warp's read meet no bank twice.  All four
+// passes, one column a thread with transitions one segment ahead against this, us: 16 heads of
+// 64 x 128, 2,048 tokens 216 and 210; 12 heads of 96 x 64, 1,000 tokens 170 and 142; 16 heads of
+// 128 x 128, 3,000 tokens 597 and 582.  (Quarters of the key summed side by side by all eight warps
+// take 205, 149 and 582 us, but theirs is another sum: last bits of every prompt's states follow.)
 //
 // STAGES 0: a thread owns a column and every sixteenth row, four at a time; transitions from L2.
 // ---------------------------------------------------------------------------
 #define DJ_COLS 16
 #define DJ_THREADS 256
 #define DJ_GROUPS (DJ_THREADS / DJ_COLS)
-#define DJ_MAX_STAGED 128
-#define DJ_ROWS 64                               // of a pass
-#define DJ_PASSES (DJ_MAX_STAGED / DJ_ROWS)
-#define DJ_PART (DJ_COLS * (DJ_ROWS + 4))        // floats of a quarter's sums
+#define DJ_MAX_STAGED 128                        // rows of four warps
 
 // floats between rows (of the transitions) and between columns (of the state)
 __host__ __device__ __forceinline__ int dj_pitch(int K) { return ((K >> 2) | 1) * 4; }
@@ -287,116 +284,103 @@ __global__ void __launch_bounds__(DJ_THREADS)
 delta_join_staged_kernel(float* __restrict__ scr_s, const float* __restrict__ scr_a,
                          const float* __restrict__ state, const int* __restrict__ cu_q,
                          const int* __restrict__ state_slot, int H, int K, int V, int seg_len) {
-  // the quarters' sums [4][DJ_COLS][DJ_ROWS + 4], the state [2][DJ_COLS][pitch], [STAGES][K][pitch]
-  extern __shared__ __align__(16) float sm[];
+  extern __shared__ __align__(16) float sm[];    // the state [2][DJ_COLS][pitch], [STAGES][K][pitch]
   IX_PDL_WAIT();
   const int tid = threadIdx.x, pitch = dj_pitch(K);
-  const int h = blockIdx.y, s = blockIdx.z;
+  const int h = blockIdx.y, s = blockIdx.z, col0 = blockIdx.x * DJ_COLS;
   const int nseg_s = (cu_q[s + 1] - cu_q[s] + seg_len - 1) / seg_len;
   if (nseg_s <= 0) return;
   const float* st = state + ((size_t)state_slot[s] * H + h) * K * V;
   const size_t cell = ds_cell(cu_q, s, seg_len, 0, H, h);
-  float *x = sm + 4 * DJ_PART, *y = x + DJ_COLS * pitch;
-  float* a_s = x + 2 * DJ_COLS * pitch;
+  float *x = sm, *y = x + DJ_COLS * pitch;
+  float* a_s = sm + 2 * DJ_COLS * pitch;
+  const int summing = (K + 31) & ~31;            // threads; the others copy
+  const int copier = tid - summing, copiers = DJ_THREADS - summing;
   auto fetch = [&](int e) {
-    if (e + 1 < nseg_s) {                        // (the last segment has no transitions)
+    if (copier >= 0 && e + 1 < nseg_s) {         // (the last segment has no transitions)
       const float* A = scr_a + (cell + (size_t)e * H) * K * K;
       float* to = a_s + (size_t)(e % STAGES) * K * pitch;
-      for (int i = tid * 4; i < K * K; i += DJ_THREADS * 4) {
+      for (int i = copier * 4; i < K * K; i += copiers * 4) {
         const int row = i / K;
         ds_async(to + row * pitch + (i - row * K), A + i, 16);
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  // sums: rows m + 16 r of a pass, columns n .. n + 3, every fourth 16-byte part of the key
-  const int m = (tid & 7) + ((tid >> 5) & 1) * 8, n = ((tid >> 3) & 3) * 4, quarter = tid >> 6;
-  // entries: column c, four rows of a pass
-  const int c = tid % DJ_COLS, four = tid / DJ_COLS * 4, col = blockIdx.x * DJ_COLS + c;
-  const bool ok = col < V;
-  float next[DJ_PASSES][4];                      // these entries of a segment's own state
+  // sums: rows m + 8 r, columns n .. n + 3
+  const int m = (tid & 7) + (tid & ~31), n = ((tid >> 3) & 3) * 4;
+  float next[4][4];                              // these entries of a segment's own state
   auto bring = [&](int e) {
-    const float* own = scr_s + (cell + (size_t)e * H) * K * V;
+    const float* own = scr_s + (cell + (size_t)e * H) * K * V + col0 + n;
 #pragma unroll
-    for (int p = 0; p < DJ_PASSES; ++p)
+    for (int r = 0; r < 4; ++r) {
+      const int kk = m + 8 * r;
+      const bool there = kk < K && e + 1 < nseg_s;
+      if ((V & 3) == 0) {
+        const float4 f = there && col0 + n < V ? *reinterpret_cast<const float4*>(own + (size_t)kk * V)
+                                               : make_float4(0.f, 0.f, 0.f, 0.f);
+        next[r][0] = f.x, next[r][1] = f.y, next[r][2] = f.z, next[r][3] = f.w;
+      } else {
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int kk = p * DJ_ROWS + four + r;
-        next[p][r] = kk < K && ok && e + 1 < nseg_s ? own[(size_t)kk * V + col] : 0.f;
+        for (int j = 0; j < 4; ++j)
+          next[r][j] = there && col0 + n + j < V ? own[(size_t)kk * V + j] : 0.f;
       }
+    }
   };
 #pragma unroll
   for (int e = 0; e < STAGES - 1; ++e) fetch(e);
-  bring(0);
-  for (int kk = tid / DJ_COLS; kk < K; kk += DJ_GROUPS)
-    x[c * pitch + kk] = ok ? st[(size_t)kk * V + col] : 0.f;
+  if (tid < summing) bring(0);
+  {
+    const int c = tid % DJ_COLS;
+    for (int kk = tid / DJ_COLS; kk < K; kk += DJ_GROUPS)
+      x[c * pitch + kk] = col0 + c < V ? st[(size_t)kk * V + col0 + c] : 0.f;
+  }
   for (int e = 0; e < nseg_s; ++e) {
-    float* own = scr_s + (cell + (size_t)e * H) * K * V;
-    const bool more = e + 1 < nseg_s;
     asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
-    __syncthreads();                             // x and A_e are there; y, A_(e-1) and the sums free
-    float add[DJ_PASSES][4];
-#pragma unroll
-    for (int p = 0; p < DJ_PASSES; ++p)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) add[p][r] = next[p][r];
+    __syncthreads();                             // x and A_e are there; y and A_(e-1) have been read
     fetch(e + STAGES - 1);
-    bring(e + 1);
-    const float* A = a_s + (size_t)(e % STAGES) * K * pitch;
-#pragma unroll
-    for (int p = 0; p < DJ_PASSES; ++p) {
-      if (p * DJ_ROWS >= K) break;
-      if (more) {
-        float acc[4][4] = {};                    // [row][column]
-        const float* row[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {            // (a row past the key's is read as its last)
-          const int kk = p * DJ_ROWS + m + 16 * r;
-          row[r] = A + (kk < K ? kk : K - 1) * pitch;
-        }
-#pragma unroll 1
-        for (int i = 4 * quarter; i < K; i += 16) {
-          float4 a[4];
-#pragma unroll
-          for (int r = 0; r < 4; ++r) a[r] = *reinterpret_cast<const float4*>(row[r] + i);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float4 v = *reinterpret_cast<const float4*>(x + (n + j) * pitch + i);
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-              acc[r][j] = fmaf(a[r].w, v.w, fmaf(a[r].z, v.z, fmaf(a[r].y, v.y,
-                                                                   fmaf(a[r].x, v.x, acc[r][j]))));
-          }
-        }
-        if (p > 0) __syncthreads();              // the sums of the pass before have been read
-        float* part = sm + quarter * DJ_PART + n * (DJ_ROWS + 4) + m;
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-          for (int r = 0; r < 4; ++r) part[j * (DJ_ROWS + 4) + 16 * r] = acc[r][j];
-        __syncthreads();
-      }
-      const int k0 = p * DJ_ROWS + four;
-      if (k0 < K) {                              // (K is a multiple of 4)
-        const float4 v = *reinterpret_cast<const float4*>(x + c * pitch + k0);
-        if (ok) {
+    if (tid >= summing) {                        // the start state, where the own one has been read
+      float* own = scr_s + (cell + (size_t)e * H) * K * V;
+      const int c = copier % DJ_COLS, col = col0 + c;
+      if (col < V)
+        for (int k0 = copier / DJ_COLS * 4; k0 < K; k0 += copiers / DJ_COLS * 4) {
+          const float4 v = *reinterpret_cast<const float4*>(x + c * pitch + k0);
           own[(size_t)k0 * V + col] = v.x;
           own[(size_t)(k0 + 1) * V + col] = v.y;
           own[(size_t)(k0 + 2) * V + col] = v.z;
           own[(size_t)(k0 + 3) * V + col] = v.w;
         }
-        if (more) {
-          float4 sum[4];
+    } else if (e + 1 < nseg_s) {
+      float acc[4][4];                           // [row][column]
 #pragma unroll
-          for (int q = 0; q < 4; ++q)
-            sum[q] = *reinterpret_cast<const float4*>(sm + q * DJ_PART + c * (DJ_ROWS + 4) + four);
-          *reinterpret_cast<float4*>(y + c * pitch + k0) =
-              make_float4(add[p][0] + ((sum[0].x + sum[1].x) + (sum[2].x + sum[3].x)),
-                          add[p][1] + ((sum[0].y + sum[1].y) + (sum[2].y + sum[3].y)),
-                          add[p][2] + ((sum[0].z + sum[1].z) + (sum[2].z + sum[3].z)),
-                          add[p][3] + ((sum[0].w + sum[1].w) + (sum[2].w + sum[3].w)));
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[r][j] = next[r][j];
+      bring(e + 1);
+      const float* A = a_s + (size_t)(e % STAGES) * K * pitch;
+      const float* row[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r)                // (a row past the key's is read as its last)
+        row[r] = A + min(m + 8 * r, K - 1) * pitch;
+#pragma unroll 2
+      for (int i = 0; i < K; i += 4) {
+        float4 a[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) a[r] = *reinterpret_cast<const float4*>(row[r] + i);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float4 v = *reinterpret_cast<const float4*>(x + (n + j) * pitch + i);
+#pragma unroll
+          for (int r = 0; r < 4; ++r)
+            acc[r][j] = fmaf(a[r].w, v.w, fmaf(a[r].z, v.z, fmaf(a[r].y, v.y,
+                                                                 fmaf(a[r].x, v.x, acc[r][j]))));
         }
       }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+          if (m + 8 * r < K) y[(n + j) * pitch + m + 8 * r] = acc[r][j];
     }
     float* z = x;
     x = y;
@@ -472,7 +456,7 @@ delta_join_kernel(float* __restrict__ scr_s, const float* __restrict__ scr_a,
 
 static inline size_t dj_smem(int K, int stages) {
   if (stages == 0) return (size_t)2 * K * DJ_COLS * sizeof(float);
-  return ((size_t)4 * DJ_PART + (size_t)(2 * DJ_COLS + stages * K) * dj_pitch(K)) * sizeof(float);
+  return (size_t)(2 * DJ_COLS + stages * K) * dj_pitch(K) * sizeof(float);
 }
 
 // Buffers of transitions: four where all blocks are resident with them, else two (blocks that come
