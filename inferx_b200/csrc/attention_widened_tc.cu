@@ -37,10 +37,6 @@
 // 192 entries make Q and the ring 128 KB.  The running max is updated lazily, see there; a row
 // is rescaled by its own scores alone, so what it computes does not depend on its neighbours.
 //
-// Where the longest walk is longer than an SM's share of all of them, a cluster of two blocks walks
-// (`cut`): either takes one half of the key tiles for both query tiles, and they exchange running
-// results through each other's shared memory, block r finishing query tile r (wa_cut says where).
-//
 // Every mbarrier wait is bounded; one that ran out records a code (31: copies, 32: MMA, 33:
 // softmax) in the caller's status word and the block runs to its end.
 //
@@ -110,7 +106,7 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
                          const int* __restrict__ cu_q, const int* __restrict__ q_pos0,
                          bf16* __restrict__ out, int S, int heads, int rows_per_seq, int window,
                          float scale_log2e, const bf16* __restrict__ gate, long long gate_ld,
-                         int cut, int* __restrict__ status) {
+                         int* __restrict__ status) {
   constexpr int KP = DK / 64, VP = DV / 64;         // 64-column panels
   constexpr int Q_PANEL = WA_BM * 128, Q_BYTES = KP * Q_PANEL;
   constexpr int PANEL = WA_BN * 128, V_TILE = VP * PANEL;
@@ -141,8 +137,7 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
     }
     if (!found) return;
   }
-  const int rank = cut ? (int)tc_rank() : 0;
-  const int h = blockIdx.x >> cut;
+  const int h = blockIdx.x;
   const int tok0 = cu_q[s];
   const int nq = cu_q[s + 1] - tok0;
   const int q0 = tile * 2 * WA_BM;
@@ -152,16 +147,10 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
   const int pos0 = q_pos0[s] + q0;
   const int pmax = pos0 + rows_valid - 1;
   const int kv_lo = ix_first_key(pos0, window, 0);
-  int kt0 = kv_lo & ~(WA_BN - 1);                    // base is on a tile's edge too
-  int n_tiles = (pmax + 1 - kt0 + WA_BN - 1) / WA_BN;
+  const int kt0 = kv_lo & ~(WA_BN - 1);              // base is on a tile's edge too
+  const int n_tiles = (pmax + 1 - kt0 + WA_BN - 1) / WA_BN;
   // the first query tile of two ends its walk with its own last position
-  int n_first = (min(pmax, pos0 + WA_BM - 1) + 1 - kt0 + WA_BN - 1) / WA_BN;
-  if (cut) {                                         // this block's half of the walk
-    const int half = (n_tiles + 1) / 2, skip = rank ? half : 0;
-    n_tiles = rank ? n_tiles - half : half;
-    n_first = min(max(n_first - skip, 0), n_tiles);
-    kt0 += skip * WA_BN;
-  }
+  const int n_first = (min(pmax, pos0 + WA_BM - 1) + 1 - kt0 + WA_BN - 1) / WA_BN;
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
 
@@ -199,15 +188,6 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
   tc_fence_after();
   const unsigned tmem_base = __shfl_sync(0xffffffffu, bars->tmem_holder, 0);
   volatile int* abortp = &bars->abort_flag;
-  // softmax: warps 4-7 and 8-11, a thread a row of query tile t
-  const int t = (warp - 4) >> 2, quarter = warp & 3;
-  const bool softmax = warp >= 4 && t < halves;
-  const int row = t * WA_BM + quarter * 32 + lane;
-  const unsigned lane_addr = tmem_base + ((unsigned)(quarter * 32) << 16);
-  const unsigned o_addr = lane_addr + t * 128;
-  const int my_tiles = t == 0 ? n_first : n_tiles;
-  float m_ref = -INFINITY, l_run = 0.f, mine = 1.f;
-  bool walked = false;
   int copied = 0;                        // tiles whose copies this thread started (warps 0 and 2)
 
   // The copying warps walk the tiles whole too, one lane issuing, so that coordinates stay in
@@ -301,7 +281,7 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
       __syncwarp();
       return true;
     };
-    if (ok && n_tiles > 0) ok = issue_s(0);
+    if (ok) ok = issue_s(0);
     for (int j = 0; j < n_tiles && ok; ++j) {
       if (j + 1 < n_tiles) {
         ok = issue_s(j + 1);
@@ -330,12 +310,19 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
       __syncwarp();
     }
     if (!ok && lane == 0 && !*abortp) { atomicExch(status, WA_ERR_MMA); *abortp = 1; }
-  } else if (softmax) {
+  } else if (warp >= 4 && ((warp - 4) >> 2) < halves) {
     // ---- softmax of query tile t ----
+    const int t = (warp - 4) >> 2;
+    const int quarter = warp & 3;
+    const int row = t * WA_BM + quarter * 32 + lane;
     const int pos = pos0 + row;
     const int tile_pos0 = pos0 + t * WA_BM;
     const int lo_last = ix_first_key(min(pmax, tile_pos0 + WA_BM - 1), window, 0);
     const int lo_r = ix_first_key(pos, window, 0);
+    const unsigned lane_addr = tmem_base + ((unsigned)(quarter * 32) << 16);
+    const unsigned o_addr = lane_addr + t * 128;
+    const int my_tiles = t == 0 ? n_first : n_tiles;
+    float m_ref = -INFINITY, l_run = 0.f;
     bool ok = true;
     for (int j = 0; j < my_tiles; ++j) {
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full[t][j & 1], (j >> 1) & 1, abortp));
@@ -414,95 +401,44 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars->p_ready[t]);
     }
-    if (ok && my_tiles > 0)
+    if (ok)
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->o_done[t], (my_tiles - 1) & 1, abortp));
-    if (!ok && lane == 0 && !*abortp) { atomicExch(status, WA_ERR_SOFTMAX); *abortp = 1; }
-    walked = ok;
-    tc_fence_after();
-  }
-  // a finished tile's running results, 32 columns at a time (every lane takes part in the load)
-  auto load_o = [&](int c0, float* o) {
-    if (my_tiles > 0) {
-      tc_ld32(o_addr + c0, o);
+    if (!ok) {
+      if (lane == 0 && !*abortp) { atomicExch(status, WA_ERR_SOFTMAX); *abortp = 1; }
     } else {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) o[i] = 0.f;
-    }
-  };
-  float other = 0.f;                     // what the other block's results count, if there are any
-  const float* theirs = reinterpret_cast<const float*>(smem) + (size_t)(row & (WA_BM - 1)) * (DV + 4);
-  if (cut) {
-    tc_fence_before();
-    __syncthreads();
-    tc_cluster_sync();                   // both blocks have used all of their tiles
-    if (softmax && t != rank) {
-      unsigned to = tc_of_rank(theirs, rank ^ 1);
+      tc_fence_after();
+      const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+      const size_t token = (size_t)(tok0 + q0 + row);
+      bf16* dst = out + token * ((size_t)heads * DV) + (size_t)h * DV;
+      const bf16* g = gate ? gate + token * gate_ld + (size_t)h * DV : nullptr;
 #pragma unroll
       for (int c0 = 0; c0 < DV; c0 += 32) {
         float o[32];
-        load_o(c0, o);
+        tc_ld32(o_addr + c0, o);               // every lane takes part in the load
+        if (row < rows_valid) {
 #pragma unroll
-        for (int i = 0; i < 32; i += 4)
-          asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to + (c0 + i) * 4),
-                       "f"(o[i]), "f"(o[i + 1]), "f"(o[i + 2]), "f"(o[i + 3])
-                       : "memory");
-      }
-      asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(to + DV * 4), "f"(m_ref),
-                   "f"(l_run)
-                   : "memory");
-    }
-    __syncwarp();
-    tc_cluster_sync();
-    if (softmax && t == rank) {
-      const float m_o = theirs[DV], l_o = theirs[DV + 1], top = fmaxf(m_ref, m_o);
-      mine = m_ref == -INFINITY ? 0.f : wa_exp2(m_ref - top);
-      other = m_o == -INFINITY ? 0.f : wa_exp2(m_o - top);
-      l_run = l_run * mine + l_o * other;
-    }
-    walked = walked && t == rank;
-  }
-  if (softmax && walked) {
-    const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-    const size_t token = (size_t)(tok0 + q0 + row);
-    bf16* dst = out + token * ((size_t)heads * DV) + (size_t)h * DV;
-    const bf16* g = gate ? gate + token * gate_ld + (size_t)h * DV : nullptr;
+          for (int i = 0; i < 32; i += 8) {
+            float f[8];
 #pragma unroll
-    for (int c0 = 0; c0 < DV; c0 += 32) {
-      float o[32];
-      load_o(c0, o);
-      if (cut) {
+            for (int u = 0; u < 8; ++u) f[u] = o[i + u] * inv;
+            if (g) {
+              const uint4 z4 = *reinterpret_cast<const uint4*>(g + c0 + i);
+              const unsigned zw[4] = {z4.x, z4.y, z4.z, z4.w};
 #pragma unroll
-        for (int i = 0; i < 32; i += 4) {
-          const float4 x = *reinterpret_cast<const float4*>(theirs + c0 + i);
-          o[i] = o[i] * mine + x.x * other;
-          o[i + 1] = o[i + 1] * mine + x.y * other;
-          o[i + 2] = o[i + 2] * mine + x.z * other;
-          o[i + 3] = o[i + 3] * mine + x.w * other;
-        }
-      }
-      if (row < rows_valid) {
-#pragma unroll
-        for (int i = 0; i < 32; i += 8) {
-          float f[8];
-#pragma unroll
-          for (int u = 0; u < 8; ++u) f[u] = o[i + u] * inv;
-          if (g) {
-            const uint4 z4 = *reinterpret_cast<const uint4*>(g + c0 + i);
-            const unsigned zw[4] = {z4.x, z4.y, z4.z, z4.w};
+              for (int u = 0; u < 4; ++u) {
+                const float2 z = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&zw[u]));
+                f[2 * u] *= __fdividef(1.f, 1.f + __expf(-z.x));
+                f[2 * u + 1] *= __fdividef(1.f, 1.f + __expf(-z.y));
+              }
+            }
+            unsigned w4[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-              const float2 z = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&zw[u]));
-              f[2 * u] *= __fdividef(1.f, 1.f + __expf(-z.x));
-              f[2 * u + 1] *= __fdividef(1.f, 1.f + __expf(-z.y));
+              __nv_bfloat162 v = __floats2bfloat162_rn(f[2 * u], f[2 * u + 1]);
+              w4[u] = *reinterpret_cast<unsigned*>(&v);
             }
+            *reinterpret_cast<uint4*>(dst + c0 + i) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
           }
-          unsigned w4[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            __nv_bfloat162 v = __floats2bfloat162_rn(f[2 * u], f[2 * u + 1]);
-            w4[u] = *reinterpret_cast<unsigned*>(&v);
-          }
-          *reinterpret_cast<uint4*>(dst + c0 + i) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
         }
       }
     }
@@ -522,28 +458,6 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
                  "r"(TMEM_COLS)
                  : "memory");
   }
-}
-
-// Whether clusters of two blocks share the walks: by the time of the longest walk or of an SM's share
-// of all (sequences taken as equally long), 2.1 us a key tile, and what a block costs beside its
-// walk, 5 us, with the exchange 12.  While the blocks leave SMs free it pays (2,048 queries of 16
-// heads: 53 us against 72), behind a full device not (1,500 of 32 heads: 71 against 56; 3,000 of 16:
-// 104 either way).
-static int wa_cut(int T, int S, int heads, int rows_per_seq, int window) {
-  const long long q_tiles = ((T + S - 1) / S + 2 * WA_BM - 1) / (2 * WA_BM);
-  long long longest = rows_per_seq / WA_BN, all = 0;
-  if (window > 0 && longest > (window + 2 * WA_BM) / WA_BN + 1)
-    longest = (window + 2 * WA_BM) / WA_BN + 1;
-  for (long long i = 0; i < q_tiles; ++i) {
-    const long long n = rows_per_seq / WA_BN - i * (2 * WA_BM / WA_BN);
-    all += n < 1 ? 1 : n < longest ? n : longest;
-  }
-  const double share = (double)all * heads * S / 148.0;
-  const double blocks = (double)q_tiles * heads * S / 148.0;
-  const double whole = 2.1 * (share > longest ? share : longest) + 5.0 * (blocks > 1 ? blocks : 1);
-  const double halves = 2.1 * (share > 0.5 * longest ? share : 0.5 * longest) +
-                        12.0 * (2 * blocks > 1 ? 2 * blocks : 1);
-  return halves < 0.9 * whole;
 }
 
 template <int DK, int DV, int LP, int WT>
@@ -566,20 +480,9 @@ static int launch_widened(const void* q, long long q_ld, const void* kv, const i
   if (e != cudaSuccess) return (int)e;
   const int tiles = (T + 2 * WA_BM - 1) / (2 * WA_BM) + S;   // every sequence can add a part tile
   if (tiles > 65535) return IX_ERR_SIZE;
-  const int cut = wa_cut(T, S, heads, rows_per_seq, window);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(heads << cut, tiles);
-  cfg.blockDim = dim3(WA_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = cut ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, kern, map_q, map_kv, cu_q, q_pos0, (bf16*)out, S, heads, rows_per_seq,
-                     window, scale * 1.4426950408889634f, (const bf16*)gate, gate_ld, cut, status);
+  kern<<<dim3(heads, tiles), WA_THREADS, smem, stream>>>(
+      map_q, map_kv, cu_q, q_pos0, (bf16*)out, S, heads, rows_per_seq, window,
+      scale * 1.4426950408889634f, (const bf16*)gate, gate_ld, status);
   return ix_launch_status();
 }
 

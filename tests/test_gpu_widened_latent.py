@@ -304,27 +304,35 @@ def test_widened_is_no_further_from_exact_than_folded(heads, dim, rot, rank, q_r
     assert off[1] <= off[0], off
 
 
-@pytest.mark.parametrize("window", [0, 90])
-def test_a_row_does_not_depend_on_its_neighbours(window):
-    """The same query in another company, and in a portion that begins elsewhere: the same bits."""
+@pytest.mark.parametrize("n", [300, 1290])          # (few tiles; walks longer than an SM's share)
+@pytest.mark.parametrize("window", [0, 90, 700])
+def test_a_row_does_not_depend_on_its_neighbours(window, n):
+    """The same query in another company, in a portion that begins elsewhere, beside another
+    sequence and with more rows a sequence: the same bits."""
     g = torch.Generator().manual_seed(window)
-    H, dk, dv, n, rows = 2, 128, 128, 300, 320
+    H, dk, dv = 2, 128, 128
+    rows = -(-n // 64) * 64
     q = torch.randn(n, H * dk, generator=g).to(BF)
     kv = torch.randn(rows, H * (dk + dv), generator=g).to(BF)
 
-    def run(q, start):
-        st = _step([q.shape[0]], [start])
+    def run(q, start, beside=(), more=0):
+        st = _step([q.shape[0], *beside], [start] + [0] * len(beside))
         base = max(0, start - window + 1) // 64 * 64 if window else 0
-        own = torch.zeros_like(kv)
+        own = torch.zeros((1 + len(beside)) * (rows + more), kv.shape[1], dtype=BF)
         own[:rows - base] = kv[base:]
-        out = _ops().widened_attention(q.cuda().view(-1), H * dk, own.cuda(), st.cu_q.cuda(),
-                                       st.q_pos0.cuda(), q.shape[0], H, dk, dv, rows, window, 0.3)
+        both = torch.cat([q, q.new_ones(sum(beside), q.shape[1])])
+        out = _ops().widened_attention(both.cuda().view(-1), H * dk, own.cuda(), st.cu_q.cuda(),
+                                       st.q_pos0.cuda(), both.shape[0], H, dk, dv, rows + more,
+                                       window, 0.3)
         _ops().check_async_errors()
-        return out.cpu()
+        return out.cpu()[:q.shape[0]]
 
     whole = run(q, 0)
     loud = q.clone()
     loud[::2] *= 30.0                            # every other row's maxima grow all along its keys
     assert torch.equal(run(loud, 0)[1::2], whole[1::2])
-    for cut in (1, 64, 129, 200):
+    for cut in (1, 64, 129, 200, n - 30):
         assert torch.equal(run(q[cut:].contiguous(), cut), whole[cut:])
+    assert torch.equal(run(q, 0, beside=(40,)), whole)
+    assert torch.equal(run(q[n - 30:].contiguous(), n - 30, beside=(n - 200, 7), more=128),
+                       whole[n - 30:])
