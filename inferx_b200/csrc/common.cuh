@@ -112,8 +112,11 @@ __device__ __forceinline__ float ix_cap_raw_score(float s, float c1, float cap_o
 // in the stream is still draining (its blocks sit at the wait until the predecessor
 // has completed and its writes are visible), which hides launch latency, block
 // scheduling and the kernel's own prologue.  IX_PDL_WAIT() must come before the
-// first access to global memory; a kernel launched the ordinary way passes through
-// it at once.  INFERX_PDL=0 in the environment turns the attribute off.
+// first access to global memory that a kernel of a step writes, whichever kernel it is:
+// activations, tables, per-request state.  Ahead of it only what no step writes may be
+// read (weights), and what was closed before the step (earlier pages of the cache; the
+// offsets where the caller says that they are settled).  A kernel launched the ordinary way
+// passes through it at once.  INFERX_PDL=0 in the environment turns the attribute off.
 // ---------------------------------------------------------------------------
 #define IX_PDL_WAIT()                                             \
   do {                                                            \
@@ -153,7 +156,7 @@ static inline cudaError_t ix_launch_impl(void (*kern)(P...), dim3 grid, dim3 blo
   return cudaLaunchKernelExC(&cfg, (const void*)kern, ptrs);
 }
 
-// Launch a kernel whose first statement is IX_PDL_WAIT().
+// Launch a kernel that keeps to IX_PDL_WAIT()'s rule.
 template <typename... P, typename... A>
 static inline void ix_launch(void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
                              cudaStream_t stream, A... a) {

@@ -728,8 +728,9 @@ delta_recurrence_kernel(const TA* __restrict__ q, long long ldq, const TA* __res
 // ---------------------------------------------------------------------------
 // Both recurrences for sequences of one token (a batch that decodes): nothing but the state, once
 // in and once out.  A block has a whole (sequence, head); a thread KPT entries of four neighbouring
-// columns, all of them on their way before anything else is read (16 bytes an access, the block's
-// 32 KB at once), and no chunk is staged.  Slices, roundings and orders of sums are the walks', so
+// columns, all of them on their way before any other operand is read (16 bytes an access, the block's
+// 32 KB at once), and no chunk is staged.  The state is the preceding kernel's to write, where that is
+// this one on the same state, so nothing is read ahead of the wait.  Slices, roundings and orders of sums are the walks', so
 // the bits are too.  48 sequences: 32 heads of 128 x 64 (state space) 20.3 us against 42.4 walked,
 // 5.0 TB/s; 16 heads of 64 x 128 (delta rule) 16.2 against 23.5; 8 sequences 4.2 against 7.8 and 4.4
 // against 5.5.
@@ -771,11 +772,10 @@ ssd_single_kernel(const TA* __restrict__ xbc, long long ld, const TA* __restrict
   const int h = blockIdx.x, s = blockIdx.y;
   const int cols = V >> 2, KS = K / KPT;
   const int c4 = threadIdx.x % cols, ks = threadIdx.x / cols, kk0 = ks * KPT;
-  // the state is not the preceding kernel's to write
+  IX_PDL_WAIT();
   float* st = state + ((size_t)state_slot[s] * H + h) * K * V;
   float4 S[KPT];
   rs_load<KPT>(st, kk0, V, c4, S);
-  IX_PDL_WAIT();
   const int t = cu_q[s], g = h / (H / G);
   if (cu_q[s + 1] <= t) return;
   const TA* row = xbc + (size_t)t * ld;
@@ -834,11 +834,10 @@ delta_single_kernel(const TA* __restrict__ q, long long ldq, const TA* __restric
   const int h = blockIdx.x, s = blockIdx.y, j = h / (H / HK);
   const int cols = V >> 2, KS = K / KPT;
   const int c4 = threadIdx.x % cols, ks = threadIdx.x / cols, kk0 = ks * KPT;
-  // the state is not the preceding kernel's to write
+  IX_PDL_WAIT();
   float* st = state + ((size_t)state_slot[s] * H + h) * K * V;
   float4 S[KPT];
   rs_load<KPT>(st, kk0, V, c4, S);
-  IX_PDL_WAIT();
   const size_t t = cu_q[s];
   if (cu_q[s + 1] <= (int)t) return;
   float4 vv;

@@ -700,3 +700,69 @@ def test_single_tokens_give_the_walk_s_bits(dtype, K, V):
     for walk, single in zip(*got):
         assert torch.equal(walk, single)
     assert torch.equal(got[1][1][3], state[3]) and not torch.equal(got[1][1][6], state[6])
+
+
+@pytest.mark.parametrize("S,H", [(3, 4), (16, 32)])
+def test_single_tokens_back_to_back(S, H):
+    """Calls right behind one another on one state, launched so that the next may come onto the
+    device while the one before still computes: every call finds what the one before left."""
+    ops, K, V, G = _ops(), 64, 128, 2
+    g = torch.Generator().manual_seed(S)
+
+    def rand(*shape):
+        return torch.randn(shape, generator=g)
+    calls = 8
+    xbc, dt = rand(calls, S, H * V + 2 * G * K).bfloat16().cuda(), rand(calls, S, H).bfloat16().cuda()
+    per_head = [rand(H).cuda() for _ in range(3)]
+    q, k, v = (rand(calls, S, H * n).bfloat16().cuda() for n in (K, K, V))
+    beta = rand(calls, S, H).bfloat16().cuda()
+    decay = (torch.rand(calls, S, H * K, generator=g) * 0.1 + 0.9).cuda()
+    state = rand(S + 1, H, K, V).cuda()
+    step = _cuda(_step([1] * S, [9] * S, slots=list(range(S))[::-1]))
+
+    def run(singles, dependent):
+        step.num_decode_seqs = singles
+        a, b = state.clone(), state.clone()
+        torch.cuda.synchronize()
+        ops.set_dependent_launch(dependent)
+        try:
+            outs = [ops.ssd_recurrence(xbc[i], dt[i], *per_head, a, step, H, V, K, G)
+                    for i in range(calls)]
+            outs += [ops.delta_recurrence(q[i], k[i], v[i], beta[i], decay[i], b, step, H, H, K, V,
+                                          1e-6, K ** -0.5) for i in range(calls)]
+        finally:
+            ops.set_dependent_launch(False)
+        return outs + [a, b]
+
+    for one, walk in zip(run(S, True), run(0, False)):
+        assert torch.equal(one, walk)
+
+
+@pytest.mark.parametrize("graphs", [False, True])
+def test_dependent_launch_changes_no_bit(tmp_path, graphs):
+    """Decode steps of a few tokens, launched so that a kernel may come onto the device while its
+    predecessor drains, and without: the same bits, convolutions, recurrences and all."""
+    ops, cfg, new = _ops(), mk.MD, 40
+    d = mk.make_model_dir(cfg, tmp_path / "m", 9, dtype="bfloat16")
+    reqs = mk.make_requests(cfg, [new + 41, new + 20, new + 9], 9)
+    steps = [{"step": 0, "entries": [{"id": r, "tokens": t[:len(t) - new], "want": [len(t) - new - 1]}
+                                     for r, t in reqs.items()], "end": []}]
+    for i in range(new):
+        steps.append({"step": i + 1, "entries": [{"id": r, "tokens": [t[len(t) - new + i]],
+                                                   "want": [0]} for r, t in reqs.items()],
+                      "end": list(reqs) if i == new - 1 else []})
+
+    def run():
+        sess = ReplaySession(d, "bfloat16", traces.peak_tokens(steps), page_size=16, max_live=4,
+                             use_graphs=graphs)
+        return [sess.run_step(s).float().cpu() for s in steps]
+
+    limit = ops.DEPENDENT_LAUNCH_MAX_TOKENS
+    overlapped = run()
+    try:
+        ops.DEPENDENT_LAUNCH_MAX_TOKENS = 0
+        plain_launches = run()
+    finally:
+        ops.DEPENDENT_LAUNCH_MAX_TOKENS = limit
+    for a, b in zip(overlapped, plain_launches):
+        assert torch.isfinite(a).all() and torch.equal(a, b)

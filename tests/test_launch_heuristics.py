@@ -1,8 +1,11 @@
 """Host-side launch decisions of the kernel library (no GPU needed: the functions only
 compute): into how many runs of keys the attention kernels cut a step."""
+import os
+import re
+
 import pytest
 
-from inferx_b200.kernels import ops
+from inferx_b200.kernels import library, ops
 
 
 @pytest.fixture(scope="module")
@@ -56,3 +59,22 @@ def test_recurrence_is_cut_into_segments_only_for_long_portions():
                     continue
                 assert seg_len >= 64 and seg_len % 16 == 0 and 2 <= nseg <= 64
                 assert (nseg - 1) * seg_len < tokens <= nseg * seg_len    # the segments cover it
+
+
+def test_no_kernel_reads_per_request_state_ahead_of_its_wait():
+    """A kernel that may come onto the device while its predecessor still computes reads no state,
+    and no table that says whose it is, before it has waited: the predecessor may be what writes it."""
+    seen = 0
+    for path in library.sources() + library._headers():
+        with open(path) as f:
+            text = re.sub(r"//[^\n]*|__launch_bounds__\([^)]*\)", "", f.read())
+        for m in re.finditer(r"__global__[^;{]*?(\w+)\s*\(([^{}]*?)\)\s*\{", text):
+            body = text[m.end():]
+            wait = body.find("IX_PDL_WAIT();")
+            following = body.find("__global__")
+            if wait < 0 or (0 <= following < wait):
+                continue                                   # launched the ordinary way
+            seen += 1
+            ahead = re.findall(r"\b(?:state|state_slot|cu_q|st)\b\s*\[|\bstate\s*\+", body[:wait])
+            assert not ahead, f"{os.path.basename(path)}: {m.group(1)} reads {ahead}"
+    assert seen > 80
