@@ -845,10 +845,15 @@ static size_t router_choose_bytes(int T, int E, int k) {
   return ((size_t)T * E + 2 * (size_t)T * k + E + 1) * sizeof(float);
 }
 
-// Whether ix_router_dispatch takes these sizes.
+// Whether ix_router_dispatch takes these sizes: not where the tables alone are for more than one
+// block (32 tokens, 32 of 300: 88 us in one block, 41 as selection and ix_moe_dispatch), nor where
+// the picks are most of the work and an SM's schedulers take turns at them (32 tokens, 16 of 32: 22.3
+// and 20.5; 16 of 128 31.6 either way; 4 of 60 11.1 and 12.1).
 IX_API int ix_router_dispatch_applies(int T, int E, int k) {
-  return T > 0 && E > 0 && k > 0 && k <= E && k <= ROUTER_MAX_TOPK &&
-         T <= ROUTER_CHOOSE_MAX_TOKENS && router_choose_bytes(T, E, k) <= ROUTER_CHOOSE_MAX_BYTES;
+  if (T <= 0 || E <= 0 || k <= 0 || k > E || k > ROUTER_MAX_TOPK || T > ROUTER_CHOOSE_MAX_TOKENS)
+    return 0;
+  if (ix_moe_dispatch_scratch_ints(T, E, k) > 0 || (T * k > 256 && 4 * k >= E)) return 0;
+  return router_choose_bytes(T, E, k) <= ROUTER_CHOOSE_MAX_BYTES;
 }
 
 // ix_router_topk_ruled (ruled 0: ix_router_topk) and ix_moe_dispatch of its choice, for a few

@@ -936,7 +936,7 @@ def test_token_logprobs(R, V, top):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("T,E,k", [(1, 60, 4), (16, 60, 4), (32, 32, 4), (32, 33, 32), (7, 5, 5),
+@pytest.mark.parametrize("T,E,k", [(1, 60, 4), (16, 60, 4), (32, 32, 4), (32, 33, 32), (16, 129, 32), (7, 5, 5),
                                    (3, 400, 2), (1, 1, 1), (33, 60, 4)])
 @pytest.mark.parametrize("rule", ["plain", "groups", "sigmoid", "sigmoid_groups"])
 def test_router_dispatch_is_router_then_dispatch(dtype, T, E, k, rule):

@@ -78,3 +78,15 @@ def test_no_kernel_reads_per_request_state_ahead_of_its_wait():
             ahead = re.findall(r"\b(?:state|state_slot|cu_q|st)\b\s*\[|\bstate\s*\+", body[:wait])
             assert not ahead, f"{os.path.basename(path)}: {m.group(1)} reads {ahead}"
     assert seen > 80
+
+
+def test_one_block_routes_no_more_than_one_block_dispatches(lib):
+    """Selection and tables by one block only where the tables alone are one block's too."""
+    f = lib.ix_router_dispatch_applies                     # (tokens, experts, chosen)
+    assert f(1, 60, 4) and f(32, 60, 4) and f(32, 256, 8) and f(16, 300, 32) and not f(32, 32, 16)
+    assert not f(17, 300, 32) and not f(32, 64, 32) and not f(33, 60, 4) and not f(0, 60, 4)
+    for tokens in range(1, 33):
+        for experts in (8, 60, 300, 384):
+            for chosen in (1, 2, 8, 17, 32):
+                if f(tokens, experts, chosen):
+                    assert lib.ix_moe_dispatch_scratch_ints(tokens, experts, chosen) == 0
