@@ -110,16 +110,15 @@ IX_API int ix_shift_mix(const void* x, int dtype, const float* mu, float* state,
 // channel's column of the transposed matrix w2t [R][C] once for all of the block's tokens
 // (neighbouring threads read neighbouring addresses), the activations from shared memory.  A
 // token's sum runs over r in ascending order whatever else is in the block.  What bounds it
-// is the chain of weight reads: 16 inner entries are read ahead of the products that use the
-// 16 before, and with few tokens a block takes 4 instead of 16, so that four times as many
-// blocks read: 48 tokens of 1,024 channels, R 64, 5.5 us against 20.7 with reads of 4 entries and
-// 16 tokens a block; 2,048 tokens 21.5 against 23.1, where the exponentials and logarithms of
+// is the chain of weight reads: AHEAD inner entries are read ahead of the products that use the
+// AHEAD before, and with few tokens a block takes 4 instead of 16, so that four times as many
+// blocks read: 300 tokens of 1,024 channels, R 64, 5.8 us against 13.1 with reads of 4 entries and
+// 16 tokens a block; 2,048 tokens 17.1 against 18.0, where the exponentials and logarithms of
 // the decays are half of the time.
 // ---------------------------------------------------------------------------
 #define LRD_THREADS 128
-#define LRD_AHEAD 16
 
-template <typename TX, int TOK>
+template <typename TX, int TOK, int AHEAD>
 __global__ void __launch_bounds__(LRD_THREADS)
 lowrank_decay_kernel(const TX* __restrict__ x, long long ldx, const float* __restrict__ w2t,
                      const float* __restrict__ b, float* __restrict__ out, int T, int C, int R,
@@ -130,11 +129,11 @@ lowrank_decay_kernel(const TX* __restrict__ x, long long ldx, const float* __res
   const int t0 = blockIdx.x * TOK;
   const int nt = min(TOK, T - t0);
   const int c = blockIdx.y * LRD_THREADS + threadIdx.x;
-  const int body = (R & 3) == 0 ? R / LRD_AHEAD * LRD_AHEAD : 0;   // read ahead; the rest after it
-  float w[LRD_AHEAD];
+  const int body = (R & 3) == 0 ? R / AHEAD * AHEAD : 0;   // read ahead; the rest after it
+  float w[AHEAD];
   if (body && c < C) {
 #pragma unroll
-    for (int i = 0; i < LRD_AHEAD; ++i) w[i] = w2t[(size_t)i * C + c];
+    for (int i = 0; i < AHEAD; ++i) w[i] = w2t[(size_t)i * C + c];
   }
   for (int i = threadIdx.x; i < TOK * R; i += blockDim.x) {
     const int j = i / R;
@@ -146,14 +145,14 @@ lowrank_decay_kernel(const TX* __restrict__ x, long long ldx, const float* __res
   float z[TOK];
 #pragma unroll
   for (int j = 0; j < TOK; ++j) z[j] = 0.f;
-  for (int r = 0; r < body; r += LRD_AHEAD) {
-    float next[LRD_AHEAD];
-    const bool more = r + LRD_AHEAD < body;
+  for (int r = 0; r < body; r += AHEAD) {
+    float next[AHEAD];
+    const bool more = r + AHEAD < body;
 #pragma unroll
-    for (int i = 0; i < LRD_AHEAD; ++i)
-      next[i] = more ? w2t[(size_t)(r + LRD_AHEAD + i) * C + c] : 0.f;
+    for (int i = 0; i < AHEAD; ++i)
+      next[i] = more ? w2t[(size_t)(r + AHEAD + i) * C + c] : 0.f;
 #pragma unroll
-    for (int i = 0; i < LRD_AHEAD; i += 4)
+    for (int i = 0; i < AHEAD; i += 4)
 #pragma unroll
       for (int j = 0; j < TOK; ++j) {         // tokens past the last hold zeros
         const float4 a = *reinterpret_cast<const float4*>(act + j * R + r + i);
@@ -163,7 +162,7 @@ lowrank_decay_kernel(const TX* __restrict__ x, long long ldx, const float* __res
         z[j] += a.w * w[i + 3];
       }
 #pragma unroll
-    for (int i = 0; i < LRD_AHEAD; ++i) w[i] = next[i];
+    for (int i = 0; i < AHEAD; ++i) w[i] = next[i];
   }
 #pragma unroll 4
   for (int r = body; r < R; ++r) {
@@ -199,18 +198,21 @@ IX_API int ix_lowrank_decay(const void* x, int x_dtype, long long ldx, const flo
   if ((size_t)16 * R * sizeof(float) > 48 * 1024) return IX_ERR_SMEM;
   const long long cb = (C + LRD_THREADS - 1) / LRD_THREADS;
   if (cb > 65535) return IX_ERR_SIZE;
-  // 16 tokens a block once such blocks are a few for every SM
-  const bool many = ((T + 15) / 16) * cb >= 4 * 148;
-  const int tok = many ? 16 : 4;
+  // 16 tokens a block once such blocks are a few for every SM; 16 entries ahead, which leaves
+  // registers for 5 blocks an SM, where 7 with 8 entries ahead do not save a round of blocks
+  // (8 / 16 ahead, us: 1,008 blocks, R 64 17.0 / 18.8; 752, R 32 9.4 / 10.1; 608, R 64 13.2 / 12.6;
+  // 1,216, R 128 39.3 / 37.0)
+  const long long many = ((T + 15) / 16) * cb;
+  const bool wide = many >= 4 * 148;
+  const bool deep = !wide || (many + 5 * 148 - 1) / (5 * 148) <= (many + 7 * 148 - 1) / (7 * 148);
+  const int tok = wide ? 16 : 4;
   const dim3 grid((T + tok - 1) / tok, (unsigned)cb);
   const size_t smem = (size_t)tok * R * sizeof(float);
   IX_DISPATCH_DTYPE(x_dtype, TX, {
-    if (many)
-      ix_launch(lowrank_decay_kernel<TX, 16>, grid, dim3(LRD_THREADS), smem, stream,
-                (const TX*)x, ldx, w2t, b, out, T, C, R, form, 1.0f / tau, head_param, per_head);
-    else
-      ix_launch(lowrank_decay_kernel<TX, 4>, grid, dim3(LRD_THREADS), smem, stream,
-                (const TX*)x, ldx, w2t, b, out, T, C, R, form, 1.0f / tau, head_param, per_head);
+    auto kern = !wide ? lowrank_decay_kernel<TX, 4, 16>
+                : deep ? lowrank_decay_kernel<TX, 16, 16> : lowrank_decay_kernel<TX, 16, 8>;
+    ix_launch(kern, grid, dim3(LRD_THREADS), smem, stream, (const TX*)x, ldx, w2t, b, out, T, C, R,
+              form, 1.0f / tau, head_param, per_head);
   });
   return ix_launch_status();
 }
