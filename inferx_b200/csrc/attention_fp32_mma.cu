@@ -20,8 +20,13 @@
 // 600 queries of 16 heads of 128: 78 us against 200 on the CUDA cores, 2,048 queries 486 against
 // 1,421; relative error against 64 bits 2.1e-7 against 3.5e-7.
 //
-// Rows whose scores or result are not finite, or whose result is below 2^-64 and not 0 (operands
-// without a third term may have gone into it), are computed again from the operands at the end.
+// Bfloat16 has no normal third term of numbers below 2^-102: what is left out of one, 2^-126 at most,
+// shows where it meets a great partner.  Computed again from the operands at the end are rows whose
+// scores or result are not finite, whose result is below 2^-64 and not 0, whose query has entries
+// above 2^80 (over the scale, if that is above 1), or that see a key with such entries or a value
+// with entries above 2^24.  A block keeps the greatest magnitudes (summed by fours) that it split, and
+// looks for the rows only where they are above that (0.5 to 2.5 % of the time; noted key by key on the
+// way, 2 to 12).  All of it follows from what the row sees, so its bits do too.
 #include <cfloat>
 
 #include "attention_distance.cuh"
@@ -66,9 +71,14 @@ __device__ __forceinline__ void fm_split2(float a, float b, unsigned& t1, unsign
   p = __floats2bfloat162_rn(a, b);
   t3 = *reinterpret_cast<unsigned*>(&p);
 }
-// eight numbers of a row into the three term tiles, `part` bytes apart
+// the magnitudes of eight numbers' first terms, every second one's summed
+__device__ __forceinline__ __nv_bfloat162 fm_size(const unsigned* t1) {
+  auto size = [&](int i) { return __habs2(*reinterpret_cast<const __nv_bfloat162*>(t1 + i)); };
+  return __hadd2(__hadd2(size(0), size(1)), __hadd2(size(2), size(3)));
+}
+// eight numbers of a row into the three term tiles, `part` bytes apart; `most`: the greatest fm_size
 __device__ __forceinline__ void fm_split8(const float4& u, const float4& v, unsigned char* at,
-                                          int part) {
+                                          int part, __nv_bfloat162& most) {
   unsigned t1[4], t2[4], t3[4];
   fm_split2(u.x, u.y, t1[0], t2[0], t3[0]);
   fm_split2(u.z, u.w, t1[1], t2[1], t3[1]);
@@ -77,6 +87,17 @@ __device__ __forceinline__ void fm_split8(const float4& u, const float4& v, unsi
   *reinterpret_cast<uint4*>(at) = make_uint4(t1[0], t1[1], t1[2], t1[3]);
   *reinterpret_cast<uint4*>(at + part) = make_uint4(t2[0], t2[1], t2[2], t2[3]);
   *reinterpret_cast<uint4*>(at + 2 * part) = make_uint4(t3[0], t3[1], t3[2], t3[3]);
+  most = __hmax2_nan(most, fm_size(t1));
+}
+// whether eight numbers in memory are above `limit` by fm_size, or not numbers
+__device__ __forceinline__ bool fm_great8(const float* p, __nv_bfloat162 limit) {
+  unsigned t[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __nv_bfloat162 two = __floats2bfloat162_rn(p[2 * i], p[2 * i + 1]);
+    t[i] = *reinterpret_cast<const unsigned*>(&two);
+  }
+  return !__hble2(fm_size(t), limit);
 }
 // (term of the left, term of the right operand), small products first
 __device__ constexpr int FM_L[6] = {1, 0, 2, 0, 1, 0}, FM_R[6] = {1, 2, 0, 1, 0, 0};
@@ -155,12 +176,16 @@ attention_fp32_mma_kernel(const FmArgs a) {
       }
     }
   };
-  auto store = [&](unsigned char* to, int pitch, int part, int pieces, int count) {
+  const __nv_bfloat162 great = __float2bfloat162_rn(1.2089258196146292e24f / fmaxf(a.scale, 1.f));
+  const __nv_bfloat162 great_v = __float2bfloat162_rn(16777216.f);
+  __nv_bfloat162 most = __float2bfloat162_rn(0.f), most_v = most;     // queries and keys; values
+  auto store = [&](unsigned char* to, int pitch, int part, int pieces, int count,
+                   __nv_bfloat162& most) {
 #pragma unroll
     for (int i = 0; i < MN; ++i) {
       if (i >= count) break;
       const int idx = tid + i * FM_THREADS, r = idx / pieces, c = idx - r * pieces;
-      fm_split8(buf[i][0], buf[i][1], to + r * pitch + c * 16, part);
+      fm_split8(buf[i][0], buf[i][1], to + r * pitch + c * 16, part, most);
     }
   };
 
@@ -174,7 +199,7 @@ attention_fp32_mma_kernel(const FmArgs a) {
       u = *reinterpret_cast<const float4*>(p);
       v = *reinterpret_cast<const float4*>(p + 4);
     }
-    fm_split8(u, v, Qs + r * QP + c * 16, Q_PART);
+    fm_split8(u, v, Qs + r * QP + c * 16, Q_PART, most);
   }
   if (tid < FM_BQ) again[tid] = 0;
 
@@ -194,7 +219,7 @@ attention_fp32_mma_kernel(const FmArgs a) {
   bool odd[2] = {false, false};
 
   for (; kv0 < kv_hi; kv0 = next(kv0)) {
-    store(Ks, QP, K_PART, KC, KN);
+    store(Ks, QP, K_PART, KC, KN, most);
     fetch(a.vc, VD, VC, VN, kv0);
     __syncthreads();
     const int k_first = kv0 + half * 32;
@@ -271,7 +296,7 @@ attention_fp32_mma_kernel(const FmArgs a) {
           fm_split2(pv[2], pv[3], pt[g][0][2 * u + 1], pt[g][1][2 * u + 1], pt[g][2][2 * u + 1]);
         }
     }
-    store(Vs, VP, V_PART, VC, VN);
+    store(Vs, VP, V_PART, VC, VN, most_v);
     if (next(kv0) < kv_hi) fetch(a.kc, HD, KC, KN, next(kv0));
     __syncthreads();
     if (used) {
@@ -352,13 +377,30 @@ attention_fp32_mma_kernel(const FmArgs a) {
       if (bad) again[r] = 1;
     }
   }
-  __syncthreads();
+  const bool some_great =
+      __syncthreads_or(!__hble2(most, great) || !__hble2(most_v, great_v));
 
   // rows that have to be, again: a warp a row, 32 keys at a time, from the operands
   for (int r = warp; r < rows_valid; r += FM_THREADS / 32) {
-    if (!again[r]) continue;
+    if (!again[r] && !some_great) continue;
     const int qp = pos0 + r;
     const float* qr = a.q + (size_t)(tok0 + r) * a.rows.q_ld + (size_t)h * HD;
+    auto page_of = [&](int kp) {                 // -1: not seen, or no page
+      const bool seen = kp <= qp && (kp >= ix_first_key(qp, a.window, 0) || kp < a.keep_first);
+      return seen ? bt[kp / a.page_size] : -1;
+    };
+    if (!again[r]) {                             // great numbers in the block: among this row's?
+      bool mine = lane < KC && fm_great8(qr + 8 * lane, great);
+      for (int k0 = kept > 0 ? 0 : kv_lo_tile; k0 <= qp; k0 = next(k0))
+        for (int kp = k0 + lane; kp < k0 + FM_BK; kp += 32) {
+          const int page = page_of(kp);
+          if (page < 0) continue;
+          const size_t row = ((size_t)page * a.kvh + kh) * a.page_size + kp % a.page_size;
+          for (int c = 0; c < KC; ++c) mine |= fm_great8(a.kc + row * HD + 8 * c, great);
+          for (int c = 0; c < VC; ++c) mine |= fm_great8(a.vc + row * VD + 8 * c, great_v);
+        }
+      if (!__any_sync(0xffffffffu, mine)) continue;
+    }
     float m = -INFINITY, l = 0.f, acc[VD / 32];
 #pragma unroll
     for (int j = 0; j < VD / 32; ++j) acc[j] = 0.f;

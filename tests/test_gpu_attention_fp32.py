@@ -114,3 +114,49 @@ def test_infinities_nan_and_numbers_without_a_third_term():
     got = ops.paged_attention_tiled(c["q"], c["k"], c["v"], c["bt"], c["cu"], c["pos0"], *args)
     plain = ops.paged_attention_generic(c["q"], c["k"], c["v"], c["bt"], c["seq"], c["pos"], *args)
     assert float((got - plain).double().norm()) <= 1e-5 * float(plain.double().norm())
+
+
+@pytest.mark.parametrize("hd,vd", [(64, 64), (128, 128)])
+@pytest.mark.parametrize("what", ["queries", "keys", "weights"])
+def test_operands_without_three_terms_that_meet_great_ones(what, hd, vd):
+    """Queries or keys below 2^-102 against great partners, weights of e^-87 on great values: scores
+    and results of ordinary size keep fp32's precision, what a chain of hd multiply-adds has (a
+    weight's relative error is that of its score of 87)."""
+    ops = _ops()
+    c = _case([150], [20], 2, 1, hd, vd, 16, hd)
+    bound = hd ** 0.5 * 2.0 ** -24
+    if what == "weights":             # the first key's score is 87, the others' nearly 0
+        first = int(c["bt"][0, 0])
+        u = c["q"][0, 0].clone()
+        c["q"] = u.expand_as(c["q"]).contiguous()
+        c["k"] *= 1e-3
+        c["k"][first, :, 0] = 87.0 * u / u.square().sum() * hd ** 0.5
+        c["v"] *= 2.0 ** 118
+        c["v"][first, :, 0] = 0.0
+        bound *= 87.0
+    else:
+        small, great = ("q", "k") if what == "queries" else ("k", "q")
+        c[small] *= 2.0 ** -122
+        c[great] *= 2.0 ** 122
+    args = (0, hd ** -0.5, 0.0, 0, None)
+    got = ops.paged_attention_tiled(c["q"], c["k"], c["v"], c["bt"], c["cu"], c["pos0"], *args)
+    assert _off(got, _exact(c, *args)) <= bound
+
+
+def test_a_row_is_made_again_by_what_it_sees():
+    """Great entries change no bit of a row that does not see them."""
+    ops = _ops()
+    c = _case([200], [0], 2, 2, 64, 128, 16, 4)
+    call = lambda: ops.paged_attention_tiled(c["q"], c["k"], c["v"], c["bt"], c["cu"], c["pos0"],
+                                             40, 0.125)
+    before = call()
+    c["k"][int(c["bt"][0, 90 // 16]), 0, 90 % 16, 5] = 2.0 ** 90
+    c["v"][int(c["bt"][0, 120 // 16]), 1, 120 % 16, 7] = 2.0 ** 40
+    c["q"][170, 1, 3] = 2.0 ** 90
+    after = call()
+    seen = torch.zeros(200, 2, dtype=torch.bool)
+    seen[90:130, 0] = seen[120:160, 1] = seen[170, 1] = True
+    assert torch.equal(after.cpu()[~seen], before.cpu()[~seen])
+    assert not torch.equal(after.cpu()[seen], before.cpu()[seen])
+    plain = ops.paged_attention_generic(c["q"], c["k"], c["v"], c["bt"], c["seq"], c["pos"], 40, 0.125)
+    torch.testing.assert_close(after, plain, rtol=1e-4, atol=1e-5)
