@@ -30,6 +30,7 @@
 #include <cfloat>
 
 #include "attention_distance.cuh"
+#include "bf16_terms.cuh"
 
 #define FM_BQ 64
 #define FM_BK 64
@@ -57,20 +58,6 @@ __device__ __forceinline__ void fm_mma(float* c, const unsigned* a, const unsign
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
-// The three terms of two numbers, packed.
-__device__ __forceinline__ void fm_split2(float a, float b, unsigned& t1, unsigned& t2,
-                                          unsigned& t3) {
-  __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
-  t1 = *reinterpret_cast<unsigned*>(&p);
-  a -= __uint_as_float(t1 << 16);
-  b -= __uint_as_float(t1 & 0xffff0000u);
-  p = __floats2bfloat162_rn(a, b);
-  t2 = *reinterpret_cast<unsigned*>(&p);
-  a -= __uint_as_float(t2 << 16);
-  b -= __uint_as_float(t2 & 0xffff0000u);
-  p = __floats2bfloat162_rn(a, b);
-  t3 = *reinterpret_cast<unsigned*>(&p);
-}
 // the magnitudes of eight numbers' first terms, every second one's summed
 __device__ __forceinline__ __nv_bfloat162 fm_size(const unsigned* t1) {
   auto size = [&](int i) { return __habs2(*reinterpret_cast<const __nv_bfloat162*>(t1 + i)); };
@@ -80,10 +67,10 @@ __device__ __forceinline__ __nv_bfloat162 fm_size(const unsigned* t1) {
 __device__ __forceinline__ void fm_split8(const float4& u, const float4& v, unsigned char* at,
                                           int part, __nv_bfloat162& most) {
   unsigned t1[4], t2[4], t3[4];
-  fm_split2(u.x, u.y, t1[0], t2[0], t3[0]);
-  fm_split2(u.z, u.w, t1[1], t2[1], t3[1]);
-  fm_split2(v.x, v.y, t1[2], t2[2], t3[2]);
-  fm_split2(v.z, v.w, t1[3], t2[3], t3[3]);
+  bf16_terms2(u.x, u.y, t1[0], t2[0], t3[0]);
+  bf16_terms2(u.z, u.w, t1[1], t2[1], t3[1]);
+  bf16_terms2(v.x, v.y, t1[2], t2[2], t3[2]);
+  bf16_terms2(v.z, v.w, t1[3], t2[3], t3[3]);
   *reinterpret_cast<uint4*>(at) = make_uint4(t1[0], t1[1], t1[2], t1[3]);
   *reinterpret_cast<uint4*>(at + part) = make_uint4(t2[0], t2[1], t2[2], t2[3]);
   *reinterpret_cast<uint4*>(at + 2 * part) = make_uint4(t3[0], t3[1], t3[2], t3[3]);
@@ -292,8 +279,8 @@ attention_fp32_mma_kernel(const FmArgs a) {
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           const float* pv = hi[2 * g + u];
-          fm_split2(pv[0], pv[1], pt[g][0][2 * u], pt[g][1][2 * u], pt[g][2][2 * u]);
-          fm_split2(pv[2], pv[3], pt[g][0][2 * u + 1], pt[g][1][2 * u + 1], pt[g][2][2 * u + 1]);
+          bf16_terms2(pv[0], pv[1], pt[g][0][2 * u], pt[g][1][2 * u], pt[g][2][2 * u]);
+          bf16_terms2(pv[2], pv[3], pt[g][0][2 * u + 1], pt[g][1][2 * u + 1], pt[g][2][2 * u + 1]);
         }
     }
     store(Vs, VP, V_PART, VC, VN, most_v);

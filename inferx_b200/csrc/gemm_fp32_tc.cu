@@ -40,6 +40,7 @@
 // 8 and bases on 32-byte marks.
 #include <cfloat>
 
+#include "bf16_terms.cuh"
 #include "common.cuh"
 #include "tma_common.cuh"
 #include "tcgen05_common.cuh"
@@ -79,26 +80,12 @@ __device__ __forceinline__ void f3_ld8(unsigned taddr, float* v) {
 #pragma unroll
   for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
-// The three terms of two numbers, packed.
-__device__ __forceinline__ void f3_split2(float a, float b, unsigned& t1, unsigned& t2,
-                                          unsigned& t3) {
-  __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
-  t1 = *reinterpret_cast<unsigned*>(&p);
-  a -= __uint_as_float(t1 << 16);
-  b -= __uint_as_float(t1 & 0xffff0000u);
-  p = __floats2bfloat162_rn(a, b);
-  t2 = *reinterpret_cast<unsigned*>(&p);
-  a -= __uint_as_float(t2 << 16);
-  b -= __uint_as_float(t2 & 0xffff0000u);
-  p = __floats2bfloat162_rn(a, b);
-  t3 = *reinterpret_cast<unsigned*>(&p);
-}
 // Of eight numbers, 16 bytes each, into the same place of three tiles PART bytes apart.
 template <int PART>
 __device__ __forceinline__ void f3_split8(const float* v, unsigned char* at) {
   unsigned t1[4], t2[4], t3[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) f3_split2(v[2 * i], v[2 * i + 1], t1[i], t2[i], t3[i]);
+  for (int i = 0; i < 4; ++i) bf16_terms2(v[2 * i], v[2 * i + 1], t1[i], t2[i], t3[i]);
   *reinterpret_cast<uint4*>(at) = make_uint4(t1[0], t1[1], t1[2], t1[3]);
   *reinterpret_cast<uint4*>(at + PART) = make_uint4(t2[0], t2[1], t2[2], t2[3]);
   *reinterpret_cast<uint4*>(at + 2 * PART) = make_uint4(t3[0], t3[1], t3[2], t3[3]);

@@ -30,6 +30,7 @@
 // infinite in the walk is infinite here.
 //
 // Requires K and V multiples of 8, K at most 256, rows on 16-byte marks.
+#include "bf16_terms.cuh"
 #include "common.cuh"
 
 #define SC_L 64               // tokens a chunk
@@ -54,16 +55,6 @@ __device__ __forceinline__ void sc_mma(float* c, const unsigned* a, unsigned b0,
       "{%8,%9}, {%0,%1,%2,%3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// the three terms of two numbers, packed
-__device__ __forceinline__ void sc_split(float a, float b, unsigned* t) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
-    t[i] = *reinterpret_cast<const unsigned*>(&p);
-    a -= __uint_as_float(t[i] << 16);
-    b -= __uint_as_float(t[i] & 0xffff0000u);
-  }
 }
 __device__ __forceinline__ void sc_async16(void* dst, const void* src, int bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sc_smem(dst)), "l"(src),
@@ -184,7 +175,7 @@ ssd_chunk_own_kernel(ScIn in, float* __restrict__ scr_s, float* __restrict__ scr
     const float w = expf((float)(g_end - G[t])) * dt[t];
     const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162*>(x_s + t * pv + c);
     unsigned terms[3];
-    sc_split(__low2float(x) * w, __high2float(x) * w, terms);
+    bf16_terms2(__low2float(x) * w, __high2float(x) * w, terms[0], terms[1], terms[2]);
 #pragma unroll
     for (int u = 0; u < 3; ++u)
       *reinterpret_cast<unsigned*>(x_s + (u * SC_L + t) * pv + c) = terms[u];
@@ -309,8 +300,8 @@ ssd_chunk_out_kernel(ScIn in, const float* __restrict__ scr_s, float* __restrict
     float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
     if (r < K && v0 + c < V) f = *reinterpret_cast<const float4*>(start + (size_t)r * V + v0 + c);
     unsigned t01[3], t23[3];
-    sc_split(f.x, f.y, t01);
-    sc_split(f.z, f.w, t23);
+    bf16_terms2(f.x, f.y, t01[0], t01[1], t01[2]);
+    bf16_terms2(f.z, f.w, t23[0], t23[1], t23[2]);
 #pragma unroll
     for (int u = 0; u < 3; ++u)
       *reinterpret_cast<uint2*>(s_s + ((size_t)u * Kp + r) * pv + c) = make_uint2(t01[u], t23[u]);
@@ -411,7 +402,7 @@ ssd_chunk_out_kernel(ScIn in, const float* __restrict__ scr_s, float* __restrict
       for (int e = 0; e < 4; ++e) {          // (row half, column half) of the fragment
         unsigned t[3];
         const float* f = p[2 * kk + (e >> 1)] + (e & 1) * 2;
-        sc_split(f[0], f[1], t);
+        bf16_terms2(f[0], f[1], t[0], t[1], t[2]);
         a[0][e] = t[0]; a[1][e] = t[1]; a[2][e] = t[2];
       }
       const int brow = kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
