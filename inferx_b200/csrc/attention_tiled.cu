@@ -2,7 +2,8 @@
 // against tiles of 64 keys held in shared memory, fp32 arithmetic throughout with the
 // accurate expf.  The prompt-sized counterpart of attention_generic.cu (one block per
 // (token, head), which re-reads every key for every query): the attention of the
-// 32-bit path for prompt portions, and of the bfloat16 path for head sizes the
+// 32-bit path for prompt portions whose heads attention_fp32_mma.cu does not take or
+// whose scores have distances, and of the bfloat16 path for head sizes the
 // tensor-core kernels do not take.  Reference behaviour as in attention_generic.cu
 // (src/backends/cuda/ops/layers.cu:256-318, 329-407): a query at position p sees keys
 // max(0, p - window + 1) .. p, score = (q . k) * scale, softmax with max subtraction,

@@ -266,8 +266,9 @@ delta_segment_kernel(DsIn in, const TA* __restrict__ v, long long ldv, float* __
 // of 16-byte parts apart, so that the eight rows of a quarter-warp's read meet no bank twice.  All four
 // passes, one column a thread with transitions one segment ahead against this, us: 16 heads of
 // 64 x 128, 2,048 tokens 216 and 210; 12 heads of 96 x 64, 1,000 tokens 170 and 142; 16 heads of
-// 128 x 128, 3,000 tokens 597 and 582.  (Quarters of the key summed side by side by all eight warps
-// take 205, 149 and 582 us, but theirs is another sum: last bits of every prompt's states follow.)
+// 128 x 128, 3,000 tokens 597 and 582; the join itself in a step of the first 38.5 and 31.1.  (Quarters
+// of the key summed side by side by all eight warps take 26.8, but theirs is another sum, and last bits
+// of every prompt's states follow.  Reads a step ahead of the sums, by hand or unrolled, are no faster.)
 //
 // STAGES 0: a thread owns a column and every sixteenth row, four at a time; transitions from L2.
 // ---------------------------------------------------------------------------

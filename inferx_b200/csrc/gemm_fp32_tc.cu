@@ -17,14 +17,16 @@
 // into registers (a step ahead), split them into the three terms and write those as swizzled tiles
 // in shared memory (two stages), and add up the accumulators of the step before the last; the first
 // block's last warp issues the 24 MMAs of a step for both.  A row of w is split for 160 rows of x and
-// a row of x for 256 of w, where a block on its own split either for 128.  What bounds a step of
-// 160 rows (1.8 us in the loop): its MMAs, 106 cycles each for 80 of arithmetic, and beside them the
-// splitting warps, about as long (990 cycles w, 750 x, 160 the sums, 1,070 until their writes are
-// there).  Against a block on its own: 600 rows of 11264 x 2048 176 us, was 186; of 2048 x 5632 98, was
-// 127; 800 rows of 22016 x 4096 788, was 1,019; 40 rows of 11264 x 2048 49, was 74.  Operands brought
-// as they are into shared memory by TMA, a step ahead, were slower (194 us for the first): what the
-// MMAs read there is what there is.  The terms are made in the kernel, and not by a pass of their own:
-// the weights' terms would be 1.5 times the weights, written and read again.
+// a row of x for 256 of w, where a block on its own split either for 128.  What bounds a step is the
+// splitting warps' chain of loads, splits, writes and sums: 1.5 us up to 96 rows, 1.65 at 128, 1.9 at
+// 160 (all pairs busy, K 4,096 to 16,384), with the tensor pipe 44 % busy and 1.4 instructions a cycle
+// of 4 at 600 rows of 11264 x 2048.  Against a block on its own: 600 rows of 11264 x 2048 176 us, was
+// 186; of 2048 x 5632 98, was 127; 800 rows of 22016 x 4096 788, was 1,019; 40 rows of 11264 x 2048 49,
+// was 74.  It is slower where one wave of blocks of 128 x 128 filled the device: 800 rows of 2048 x
+// 5632 140 us, was 125, 1,000 rows 146 and 134, 2,048 rows of 1024 x 2816 84 and 78.  Operands brought
+// as they are into shared memory by TMA, a step ahead, were slower too (194 us for the first).  The
+// terms are made in the kernel, and not by a pass of their own: the weights' terms would be 1.5 times
+// the weights, written and read again.
 //
 // With fewer tiles than SMs, or a last wave that is nearly empty, k is cut into `splits` runs whose
 // partial sums a second kernel adds in ascending order.
@@ -313,8 +315,10 @@ __global__ void gemm_fp32_tc_sum_kernel(const float* __restrict__ part, float* _
 }
 
 // Microseconds of a call in `splits` runs of k with tiles of `rows` rows: waves of pairs of blocks, a
-// step of which takes 0.75 us and 8.1 ns a row (1.3 us at 64 rows, 1.8 at 128, 2.05 at 160), and what
-// partial sums cost to write and read, 0.35 us a MB both ways and 3 us for their kernel's launch.
+// step of which counts 0.75 us and 8.1 ns a row (1.3 us at 64 rows, 1.8 at 128, 2.05 at 160, a steeper
+// line than the steps' own times above), and what partial sums cost to write and read, 0.35 us a MB both
+// ways and 3 us for their kernel's launch.  Of 32 products of 400 to 3,000 rows, each timed in 1 to 6
+// runs, the number that this chooses was the fastest or within 6 % of it.
 static double f3_cost(int M, int N, int K, int rows, int splits) {
   const int steps = (K + F3_BK - 1) / F3_BK, per = (steps + splits - 1) / splits;
   const long long tiles = ((M + rows - 1) / rows) * (long long)((N + 2 * F3_BF - 1) / (2 * F3_BF));

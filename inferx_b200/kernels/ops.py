@@ -542,8 +542,9 @@ def paged_attention_tiled(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch
                           block_table: torch.Tensor, cu_q: torch.Tensor, q_pos0: torch.Tensor,
                           window: int, scale: float, softcap: float = 0.0, keep_first: int = 0,
                           sink=None, gate=None):
-    """CUDA-core attention for a ragged batch, tiled (32 queries of a sequence against 64
-    keys at a time in shared memory, fp32 math): sequence s brings the queries
+    """Attention for a ragged batch in 32-bit arithmetic, tiled: fp32 heads of 64 and 128 on the
+    tensor cores in three bfloat16 terms a number, the others on the CUDA cores (32 queries of a
+    sequence against 64 keys at a time in shared memory).  Sequence s brings the queries
     q[cu_q[s]:cu_q[s+1]] at positions q_pos0[s], q_pos0[s]+1, ...  Any element type, head
     sizes that are a multiple of 4 up to 256; the value pages may have a head size of
     their own (the output then has it)."""
