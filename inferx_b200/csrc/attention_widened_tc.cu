@@ -25,7 +25,8 @@
 // (WT 2) in two, the second in the columns of the score buffer that the first leaves free.
 //
 // The attention kernel: a block owns two tiles of 128 queries of one sequence and head (a query
-// is a lane of tensor memory) and walks their keys in tiles of 64.  Warps 0 and 2 bring K and V
+// is a lane of tensor memory), or one where that leaves fewer SMs idle
+// (ix_widened_attention_tiles), and walks their keys in tiles of 64.  Warps 0 and 2 bring K and V
 // tiles with TMA into rings of two stages that both query tiles read (one warp for both would have
 // the next K wait for the V ahead of it, whose stage is freed a softmax later); one thread of warp
 // 1 issues the MMAs, S = Q K^T of tile j + 1 for both query tiles ahead of O += P V of tile j;
@@ -106,7 +107,7 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
                          const int* __restrict__ cu_q, const int* __restrict__ q_pos0,
                          bf16* __restrict__ out, int S, int heads, int rows_per_seq, int window,
                          float scale_log2e, const bf16* __restrict__ gate, long long gate_ld,
-                         int* __restrict__ status) {
+                         int own, int* __restrict__ status) {
   constexpr int KP = DK / 64, VP = DV / 64;         // 64-column panels
   constexpr int Q_PANEL = WA_BM * 128, Q_BYTES = KP * Q_PANEL;
   constexpr int PANEL = WA_BN * 128, V_TILE = VP * PANEL;
@@ -125,13 +126,13 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
   unsigned char* Vs = Ks + WA_STAGES * K_TILE;
   WaBars* bars = reinterpret_cast<WaBars*>(Vs + WA_STAGES * V_TILE);
 
-  // which sequence and which 256 queries of it; those with the longest walks first
+  // which sequence and which `own` tiles of its queries; those with the longest walks first
   int s = 0, tile = gridDim.y - 1 - blockIdx.y;
   {
     bool found = false;
     for (int ss = 0; ss < S; ++ss) {
       const int n = cu_q[ss + 1] - cu_q[ss];
-      const int tiles = (n + 2 * WA_BM - 1) / (2 * WA_BM);
+      const int tiles = (n + own * WA_BM - 1) / (own * WA_BM);
       if (tile < tiles) { s = ss; found = true; break; }
       tile -= tiles;
     }
@@ -140,8 +141,8 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
   const int h = blockIdx.x;
   const int tok0 = cu_q[s];
   const int nq = cu_q[s + 1] - tok0;
-  const int q0 = tile * 2 * WA_BM;
-  const int rows_valid = min(2 * WA_BM, nq - q0);
+  const int q0 = tile * own * WA_BM;
+  const int rows_valid = min(own * WA_BM, nq - q0);
   const int halves = rows_valid > WA_BM ? 2 : 1;
   const int base = wa_base(q_pos0[s], window);
   const int pos0 = q_pos0[s] + q0;
@@ -460,6 +461,34 @@ widened_attention_kernel(const __grid_constant__ CUtensorMap map_q,
   }
 }
 
+// Query tiles a block owns: two, whose chains hide each other (2.1 us a key tile for both), or where
+// the device has room for twice the blocks one (1.3 us a key tile, 5 us a block beside its walk).
+// By the longest block, or an SM's share of all and half of a shortest one that ends alone
+// (sequences taken as equally long).  Two / one tile a block, us: 2,048 queries of 16 heads 72.2 /
+// 46.5, 300 behind 2,000 78.6 / 48.1, 1,000 of 32 heads 38.2 / 30.8, but 1,500 of 32 54.8 / 59.0, four
+// times 300 behind 200 of 16 22.3 / 28.3.  A row's arithmetic is its own either way.
+IX_API int ix_widened_attention_tiles(int T, int S, int heads, int rows_per_seq, int window) {
+  const long long each = (T + S - 1LL) / S, most = 8 * 148;
+  if ((each + WA_BM - 1) / WA_BM * heads * S > most) return 2;
+  double us[2];
+  for (int own = 1; own <= 2; ++own) {
+    const double step = own == 2 ? 2.1 : 1.3, rest = 5.0;
+    const long long blocks = (each + own * WA_BM - 1) / (own * WA_BM);
+    long long longest = rows_per_seq / WA_BN, least = 0, all = 0;
+    if (window > 0 && longest > (window + own * WA_BM) / WA_BN + 1)
+      longest = (window + own * WA_BM) / WA_BN + 1;
+    for (long long i = 0; i < blocks; ++i) {
+      const long long n = rows_per_seq / WA_BN - i * (own * WA_BM / WA_BN);
+      least = n < 1 ? 1 : n < longest ? n : longest;
+      all += least;
+    }
+    const double share = (all * step + blocks * rest) * heads * S / 148.0;
+    const double alone = longest * step + rest, tail = 0.5 * (least * step + rest);
+    us[own - 1] = blocks * heads * S <= 148 || alone > share + tail ? alone : share + tail;
+  }
+  return us[0] < 0.97 * us[1] ? 1 : 2;
+}
+
 template <int DK, int DV, int LP, int WT>
 static int launch_widened(const void* q, long long q_ld, const void* kv, const int* cu_q,
                           const int* q_pos0, void* out, int T, int S, int heads, int rows_per_seq,
@@ -478,11 +507,12 @@ static int launch_widened(const void* q, long long q_ld, const void* kv, const i
   auto kern = widened_attention_kernel<DK, DV, LP, WT>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return (int)e;
-  const int tiles = (T + 2 * WA_BM - 1) / (2 * WA_BM) + S;   // every sequence can add a part tile
+  const int own = ix_widened_attention_tiles(T, S, heads, rows_per_seq, window);
+  const int tiles = (T + own * WA_BM - 1) / (own * WA_BM) + S;   // every sequence can add a part tile
   if (tiles > 65535) return IX_ERR_SIZE;
   kern<<<dim3(heads, tiles), WA_THREADS, smem, stream>>>(
       map_q, map_kv, cu_q, q_pos0, (bf16*)out, S, heads, rows_per_seq, window,
-      scale * 1.4426950408889634f, (const bf16*)gate, gate_ld, status);
+      scale * 1.4426950408889634f, (const bf16*)gate, gate_ld, own, status);
   return ix_launch_status();
 }
 

@@ -9,6 +9,8 @@ import torch
 import host_ops
 from test_gpu_dominex import _cuda, _step
 
+from inferx_b200.kernels import library  # noqa: E402
+
 pytestmark = pytest.mark.gpu
 BF = torch.bfloat16
 
@@ -334,5 +336,10 @@ def test_a_row_does_not_depend_on_its_neighbours(window, n):
     for cut in (1, 64, 129, 200, n - 30):
         assert torch.equal(run(q[cut:].contiguous(), cut), whole[cut:])
     assert torch.equal(run(q, 0, beside=(40,)), whole)
+    # as many others as make a block own two query tiles instead of one
+    lib, many = library.load(), (3,) * 31 + (1500,) * 64
+    assert lib.ix_widened_attention_tiles(n, 1, H, rows, window) == 1
+    assert lib.ix_widened_attention_tiles(n + sum(many), 1 + len(many), H, 1536, window) == 2
+    assert torch.equal(run(q, 0, beside=many, more=1536 - rows), whole)
     assert torch.equal(run(q[n - 30:].contiguous(), n - 30, beside=(n - 200, 7), more=128),
                        whole[n - 30:])

@@ -90,3 +90,15 @@ def test_one_block_routes_no_more_than_one_block_dispatches(lib):
             for chosen in (1, 2, 8, 17, 32):
                 if f(tokens, experts, chosen):
                     assert lib.ix_moe_dispatch_scratch_ints(tokens, experts, chosen) == 0
+
+
+def test_widened_attention_gives_a_block_one_query_tile_while_sms_are_free(lib):
+    f = lib.ix_widened_attention_tiles          # (tokens, sequences, heads, rows a sequence, window)
+    assert f(2048, 1, 16, 2048, 0) == 1 and f(300, 1, 16, 2304, 0) == 1 and f(3000, 1, 8, 3008, 1024) == 1
+    assert f(1500, 1, 32, 1536, 0) == 2         # one round of long walks either way
+    assert f(1200, 4, 16, 512, 0) == 2          # 192 blocks would be two rounds
+    assert f(60000, 8, 128, 8192, 0) == 2 and f(1 << 30, 1, 128, 1 << 20, 0) == 2
+    for tokens in (1, 100, 128, 129, 1000, 4096):
+        for seqs in (1, 3, 200):
+            for window in (0, 1, 512):
+                assert f(max(tokens, seqs), seqs, 16, 4096, window) in (1, 2)
