@@ -7,9 +7,8 @@ import pytest
 import torch
 
 import host_ops
+from inferx_b200.kernels import library
 from test_gpu_dominex import _cuda, _step
-
-from inferx_b200.kernels import library  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 BF = torch.bfloat16
